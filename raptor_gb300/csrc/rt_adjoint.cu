@@ -15,6 +15,8 @@
 // shading, the normal, the light vector and the ray-triangle solve, and
 // scatters dL/dposition and dL/dcolour onto the triangle's vertices with
 // atomics.  Memory is O(pixels + vertices).
+#include <type_traits>
+
 #include "rt_api_internal.cuh"
 #include "rt_shade.cuh"
 
@@ -43,8 +45,8 @@ __device__ __forceinline__ void atomic_add3(float *p, float3 g)
     atomicAdd(p + 2, g.z);
 }
 
-template <bool ADJOINT>
-__global__ void __launch_bounds__(kTraceThreads) k_diff(SceneView sc, const float *__restrict__ verts,
+template <bool ADJOINT, class SC>
+__global__ void __launch_bounds__(kTraceThreads) k_diff(SC sc, const float *__restrict__ verts,
                                                         CameraView cam, LightSet lights, MaterialView mat,
                                                         float *__restrict__ fimg, int32_t *__restrict__ ids,
                                                         uint8_t *__restrict__ occl, const float *__restrict__ dldpix,
@@ -337,13 +339,15 @@ rt_status rt_render_float(rt_scene *s, const rt_camera *camera, const rt_light *
     ls.n = nlights;
     ls.fast_pow = 0;
     for (int i = 0; i < nlights; ++i) ls.l[i] = make_light_view(lights[i]);
-    static const int per_sm = blocks_per_sm(k_diff<false>);
-    const int grid = per_sm * ctx->sm_count;
     RT_CUDA_A(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), ctx->stream), "counter clear");
     RT_CUDA_A(cudaEventRecord(ctx->ev0, ctx->stream), "event record");
-    k_diff<false><<<grid, kTraceThreads, 0, ctx->stream>>>(scene_view(s), s->d_verts, make_camera_view(*camera), ls,
-                                                           make_material_view(*material), rgb_f32, hit_ids, occluded,
-                                                           nullptr, nullptr, nullptr, ctx->d_counters);
+    with_scene(scene_view(s), [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_diff<false, SC>);
+        k_diff<false, SC><<<per_sm * ctx->sm_count, kTraceThreads, 0, ctx->stream>>>(
+            view, s->d_verts, make_camera_view(*camera), ls, make_material_view(*material), rgb_f32, hit_ids, occluded,
+            nullptr, nullptr, nullptr, ctx->d_counters);
+    });
     RT_CUDA_A(cudaGetLastError(), "forward launch");
     RT_CUDA_A(cudaEventRecord(ctx->ev1, ctx->stream), "event record");
     return finish(ctx, stats);
@@ -364,16 +368,18 @@ rt_status rt_render_adjoint(rt_scene *s, const rt_camera *camera, const rt_light
     ls.n = nlights;
     ls.fast_pow = 0;
     for (int i = 0; i < nlights; ++i) ls.l[i] = make_light_view(lights[i]);
-    static const int per_sm = blocks_per_sm(k_diff<true>);
-    const int grid = per_sm * ctx->sm_count;
     const size_t gbytes = (size_t)(s->nverts > 0 ? s->nverts : 1) * 3 * sizeof(float);
     RT_CUDA_A(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), ctx->stream), "counter clear");
     RT_CUDA_A(cudaEventRecord(ctx->ev0, ctx->stream), "event record");
     RT_CUDA_A(cudaMemsetAsync(dL_dpos, 0, gbytes, ctx->stream), "gradient clear");
     RT_CUDA_A(cudaMemsetAsync(dL_dattr, 0, gbytes, ctx->stream), "gradient clear");
-    k_diff<true><<<grid, kTraceThreads, 0, ctx->stream>>>(scene_view(s), s->d_verts, make_camera_view(*camera), ls,
-                                                          make_material_view(*material), nullptr, nullptr, nullptr,
-                                                          dL_dpix, dL_dpos, dL_dattr, ctx->d_counters);
+    with_scene(scene_view(s), [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_diff<true, SC>);
+        k_diff<true, SC><<<per_sm * ctx->sm_count, kTraceThreads, 0, ctx->stream>>>(
+            view, s->d_verts, make_camera_view(*camera), ls, make_material_view(*material), nullptr, nullptr, nullptr,
+            dL_dpix, dL_dpos, dL_dattr, ctx->d_counters);
+    });
     RT_CUDA_A(cudaGetLastError(), "adjoint launch");
     RT_CUDA_A(cudaEventRecord(ctx->ev1, ctx->stream), "event record");
     return finish(ctx, stats);

@@ -540,7 +540,7 @@ rt_status rt_bvh_stats_get(const rt_scene *s, rt_bvh_stats *out)
             else if ((n.imask >> k) & 1u) ++out->internal_slots;
             else {
                 ++out->leaf_slots;
-                const int c = __builtin_popcount(m >> 5);
+                const int c = (int)(m >> 5);
                 if (c >= 1 && c <= 3) ++out->leaf_tris[c];
             }
         }

@@ -10,6 +10,7 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "rt_api_internal.cuh"
@@ -27,7 +28,7 @@ namespace {
 
 // STACK: traversal stack capacity in node groups, chosen by the autotuner
 // among the capacities that hold the batch's deepest tree.
-template <int TW, int STACK>
+template <int TW, int STACK, class SC>
 __global__ void __launch_bounds__(256, RT_RENDER_MIN_BLOCKS / 2) k_render_batched(const BatchJob *__restrict__ jobs, int32_t njobs,
                                                         int32_t total_items, int32_t chunk, Counters *ctr)
 {
@@ -45,6 +46,7 @@ __global__ void __launch_bounds__(256, RT_RENDER_MIN_BLOCKS / 2) k_render_batche
                 if (__ldg(&jobs[mid].items_begin) <= item0) lo = mid; else hi = mid - 1;
             }
             const BatchJob &J = jobs[lo];
+            const SC &sc = static_cast<const SC &>(J.sc);
             int x, y;
             tile_pixel<TW>(item0 - J.items_begin + (threadIdx.x & 31), J.tiles_x, x, y);
             const bool live = (x < J.cam.xres) && (y < J.cam.yres);
@@ -53,10 +55,10 @@ __global__ void __launch_bounds__(256, RT_RENDER_MIN_BLOCKS / 2) k_render_batche
             po.secondary = 0;
             if (live) {
                 if (J.mode == RT_JOB_AO)
-                    po = shade_pixel_ao<false, STACK>(J.sc, J.cam, J.mat, J.ao_samples, J.ao_dist, J.ao_seed, x, y,
+                    po = shade_pixel_ao<false, STACK>(sc, J.cam, J.mat, J.ao_samples, J.ao_dist, J.ao_seed, x, y,
                                                       status, nullptr);
                 else
-                    po = shade_pixel_lights<false, false, STACK>(J.sc, J.cam, J.lights, J.nlights, J.mat, x, y,
+                    po = shade_pixel_lights<false, false, STACK>(sc, J.cam, J.lights, J.nlights, J.mat, x, y,
                                                                  status, nullptr, J.fast_pow != 0);
                 const size_t pix = (size_t)x + (size_t)y * (size_t)J.cam.xres;
                 store_rgb(J.rgb, pix, po.c);
@@ -72,26 +74,26 @@ __global__ void __launch_bounds__(256, RT_RENDER_MIN_BLOCKS / 2) k_render_batche
 
 // Lane-replacement form: every lane carries a pixel of any job and refills
 // from the shared queue (rt_wave.cuh).
-template <int TW>
+template <int TW, class SC>
 __global__ void __launch_bounds__(256, RT_WAVE_MIN_BLOCKS / 2) k_render_batched_wave(const BatchJob *__restrict__ jobs, int32_t njobs,
                                                              int32_t total_items, Counters *ctr)
 {
     extern __shared__ LaneShade wave_state[];
-    wave_loop<TW, false>(nullptr, jobs, njobs, total_items, wave_state[threadIdx.x], ctr);
+    wave_loop<TW, false, SC::kWatertight>(nullptr, jobs, njobs, total_items, wave_state[threadIdx.x], ctr);
 }
 
 // Traversal stack capacities the pixel kernel is built for (the wave
 // kernel keeps kStackSize).
 constexpr int kBatchStacks[3] = {16, 24, kStackSize};
 
-template <int TW, int STACK>
+template <int TW, int STACK, class SC>
 int grid_for(int kernel, int threads, int sm_count)
 {
     int per_sm = 0;
     cudaError_t e = (kernel == RT_KERNEL_WAVE)
-                        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_render_batched_wave<TW>, threads,
+                        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (k_render_batched_wave<TW, SC>), threads,
                                                                         threads * sizeof(LaneShade))
-                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_render_batched<TW, STACK>, threads,
+                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (k_render_batched<TW, STACK, SC>), threads,
                                                                         0);
     if (e != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
@@ -165,6 +167,7 @@ void drop_graph(rt_batch *b)
 int32_t nscenes(const rt_batch *b) { return (int32_t)b->tri_off.size() - 1; }
 
 // Launch one batch frame directly (the body captured into the graph).
+template <class SC>
 void launch_batch(rt_batch *b, cudaStream_t st, int grid)
 {
     cudaMemsetAsync(b->ctx->d_counters, 0, sizeof(Counters), st);
@@ -174,13 +177,13 @@ void launch_batch(rt_batch *b, cudaStream_t st, int grid)
     const size_t smem = (size_t)threads * sizeof(LaneShade);
     if (b->cfg.kernel == RT_KERNEL_WAVE) {
         if (b->cfg.tile_w == 16)
-            k_render_batched_wave<16><<<grid, threads, smem, st>>>(b->d_jobs, nj, b->total_items, b->ctx->d_counters);
+            k_render_batched_wave<16, SC><<<grid, threads, smem, st>>>(b->d_jobs, nj, b->total_items, b->ctx->d_counters);
         else
-            k_render_batched_wave<8><<<grid, threads, smem, st>>>(b->d_jobs, nj, b->total_items, b->ctx->d_counters);
+            k_render_batched_wave<8, SC><<<grid, threads, smem, st>>>(b->d_jobs, nj, b->total_items, b->ctx->d_counters);
     } else {
         Counters *ctr = b->ctx->d_counters;
         const int stack = b->cfg.stack_entries;
-#define RT_BATCH_PIXEL(TW, S) k_render_batched<TW, S><<<grid, threads, 0, st>>>(b->d_jobs, nj, b->total_items, chunk, ctr)
+#define RT_BATCH_PIXEL(TW, S) k_render_batched<TW, S, SC><<<grid, threads, 0, st>>>(b->d_jobs, nj, b->total_items, chunk, ctr)
         if (b->cfg.tile_w == 16) {
             if (stack == kBatchStacks[0]) RT_BATCH_PIXEL(16, kBatchStacks[0]);
             else if (stack == kBatchStacks[1]) RT_BATCH_PIXEL(16, kBatchStacks[1]);
@@ -195,18 +198,19 @@ void launch_batch(rt_batch *b, cudaStream_t st, int grid)
 }
 
 // Persistent grid of the configured shape: resident blocks per SM x SMs.
+template <class SC>
 int batch_grid(const rt_batch *b)
 {
     const rt_tune_config &c = b->cfg;
     const int sms = b->ctx->sm_count;
     if (c.tile_w == 16) {
-        if (c.stack_entries == kBatchStacks[0]) return grid_for<16, kBatchStacks[0]>(c.kernel, c.block_threads, sms);
-        if (c.stack_entries == kBatchStacks[1]) return grid_for<16, kBatchStacks[1]>(c.kernel, c.block_threads, sms);
-        return grid_for<16, kBatchStacks[2]>(c.kernel, c.block_threads, sms);
+        if (c.stack_entries == kBatchStacks[0]) return grid_for<16, kBatchStacks[0], SC>(c.kernel, c.block_threads, sms);
+        if (c.stack_entries == kBatchStacks[1]) return grid_for<16, kBatchStacks[1], SC>(c.kernel, c.block_threads, sms);
+        return grid_for<16, kBatchStacks[2], SC>(c.kernel, c.block_threads, sms);
     }
-    if (c.stack_entries == kBatchStacks[0]) return grid_for<8, kBatchStacks[0]>(c.kernel, c.block_threads, sms);
-    if (c.stack_entries == kBatchStacks[1]) return grid_for<8, kBatchStacks[1]>(c.kernel, c.block_threads, sms);
-    return grid_for<8, kBatchStacks[2]>(c.kernel, c.block_threads, sms);
+    if (c.stack_entries == kBatchStacks[0]) return grid_for<8, kBatchStacks[0], SC>(c.kernel, c.block_threads, sms);
+    if (c.stack_entries == kBatchStacks[1]) return grid_for<8, kBatchStacks[1], SC>(c.kernel, c.block_threads, sms);
+    return grid_for<8, kBatchStacks[2], SC>(c.kernel, c.block_threads, sms);
 }
 
 rt_status make_graph(rt_batch *b)
@@ -214,10 +218,16 @@ rt_status make_graph(rt_batch *b)
     drop_graph(b);
     cudaStream_t st = b->ctx->stream;
     cudaGraph_t g = nullptr;
-    const int grid = batch_grid(b);
-    RT_CUDA_B(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "graph capture begin");
-    launch_batch(b, st, grid);
-    cudaError_t e = cudaStreamEndCapture(st, &g);
+    cudaError_t e = cudaSuccess;
+    // every job's scene carries the intersector set when the jobs were
+    with_scene(b->h_jobs.empty() ? SceneView{} : b->h_jobs[0].sc, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        const int grid = batch_grid<SC>(b);
+        e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+        if (e == cudaSuccess) launch_batch<SC>(b, st, grid);
+    });
+    RT_CUDA_B(e, "graph capture begin");
+    e = cudaStreamEndCapture(st, &g);
     if (e != cudaSuccess) return set_cuda_error(e, "graph capture end");
     e = cudaGraphInstantiate(&b->exec, g, 0);
     cudaGraphDestroy(g);

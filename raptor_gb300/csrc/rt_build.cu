@@ -290,6 +290,7 @@ __device__ __forceinline__ int atomic_add_acq_rel(int32_t *p, int32_t v)
 
 constexpr int kRefitMaxDepth = 1 << 16;   // binary levels a refit walk may climb
 constexpr int32_t kEmptySlot = INT32_MIN;
+constexpr uint16_t kEmptyPlanes = 0x00ff;  // an empty slot's box is inverted: low plane 255, high plane 0
 
 // Bottom-up box refit from one child up: the second child to arrive at a
 // node unions both and goes on.  The climbing child's ref, box and
@@ -362,7 +363,7 @@ __global__ void k_roots(int32_t nseg, int32_t n, const int32_t *__restrict__ seg
     if (l < f) {
         WideNode W;
         memset(&W, 0, sizeof(W));
-        for (int k = 0; k < 8; ++k) { W.qlo_x[k] = W.qlo_y[k] = W.qlo_z[k] = 255; }
+        for (int k = 0; k < 8; ++k) W.qx[k] = W.qy[k] = W.qz[k] = kEmptyPlanes;
         nodes[s] = W;
         return;
     }
@@ -445,7 +446,7 @@ __global__ void k_ploc_segments(int32_t nseg, int32_t n, const int32_t *__restri
     }
     WideNode W;
     memset(&W, 0, sizeof(W));
-    for (int k = 0; k < 8; ++k) { W.qlo_x[k] = W.qlo_y[k] = W.qlo_z[k] = 255; }
+    for (int k = 0; k < 8; ++k) W.qx[k] = W.qy[k] = W.qz[k] = kEmptyPlanes;
     nodes[s] = W;
 }
 
@@ -1311,6 +1312,23 @@ __device__ __forceinline__ int sah_children(const BuildArgs &A, int32_t node, in
     return m;
 }
 
+// The quantised box bytes of a child in the node's frame.
+__device__ __forceinline__ uint32_t quant_lo(float c, float p, float inv)
+{
+    const float q = floorf(__fmul_rd(__fsub_rd(c, p), inv)) - 1.0f;
+    return (uint32_t)fminf(fmaxf(q, 0.f), 255.f);
+}
+__device__ __forceinline__ uint32_t quant_hi(float c, float p, float inv)
+{
+    const float q = ceilf(__fmul_ru(__fsub_ru(c, p), inv)) + 1.0f;
+    return (uint32_t)fminf(fmaxf(q, 0.f), 255.f);
+}
+// Both planes of a child along one axis, as a node stores them.
+__device__ __forceinline__ uint16_t quant_planes(float lo, float hi, float p, float inv)
+{
+    return (uint16_t)(quant_lo(lo, p, inv) | (quant_hi(hi, p, inv) << 8));
+}
+
 // One thread per wide node of the current level: gather up to 8 children
 // (by the surface-area decisions, or greedily by repeatedly opening the
 // largest-area internal child, those too big for a leaf first), assign slots
@@ -1427,29 +1445,21 @@ __device__ __forceinline__ void collapse_task(const BuildArgs &A, const int2 tas
         A.slot_ref[8 * (size_t)wide + s] = k < 0 ? kEmptySlot : ch[k];
         if (k < 0) {
             W.meta[s] = 0;
-            W.qlo_x[s] = W.qlo_y[s] = W.qlo_z[s] = 255;
-            W.qhi_x[s] = W.qhi_y[s] = W.qhi_z[s] = 0;
+            W.qx[s] = W.qy[s] = W.qz[s] = kEmptyPlanes;
             continue;
         }
-        const auto qlo = [](float c, float p, float inv) {
-            const float q = floorf(__fmul_rd(__fsub_rd(c, p), inv)) - 1.0f;
-            return (uint8_t)fminf(fmaxf(q, 0.f), 255.f);
-        };
-        const auto qhi = [](float c, float p, float inv) {
-            const float q = ceilf(__fmul_ru(__fsub_ru(c, p), inv)) + 1.0f;
-            return (uint8_t)fminf(fmaxf(q, 0.f), 255.f);
-        };
-        W.qlo_x[s] = qlo(clo[k].x, px, ix); W.qlo_y[s] = qlo(clo[k].y, py, iy); W.qlo_z[s] = qlo(clo[k].z, pz, iz);
-        W.qhi_x[s] = qhi(chi[k].x, px, ix); W.qhi_y[s] = qhi(chi[k].y, py, iy); W.qhi_z[s] = qhi(chi[k].z, pz, iz);
+        W.qx[s] = quant_planes(clo[k].x, chi[k].x, px, ix);
+        W.qy[s] = quant_planes(clo[k].y, chi[k].y, py, iy);
+        W.qz[s] = quant_planes(clo[k].z, chi[k].z, pz, iz);
         if (!leaf[k]) {
             W.imask |= (uint8_t)(1u << s);
-            W.meta[s] = (uint8_t)(0x20 | (24 + s));
+            W.meta[s] = 0x80;
             const int slot = atomicAdd(A.next_count, 1);
             A.tasks_out[slot] = make_int2(ch[k], child_base + int_k);
             ++int_k;
         } else {
             const int c = cnt[k];
-            W.meta[s] = (uint8_t)((((1u << c) - 1u) << 5) | (uint32_t)tri_off);
+            W.meta[s] = (uint8_t)(((uint32_t)c << 5) | (uint32_t)tri_off);
             int32_t lv[kMaxLeafTris];
             int nlv = 0;
             if (!leaf_refs(A, ch[k], lv, nlv) || nlv != c) { atomicExch(&A.counters[3], 1); return; }
@@ -1458,18 +1468,6 @@ __device__ __forceinline__ void collapse_task(const BuildArgs &A, const int2 tas
         }
     }
     A.nodes[wide] = W;
-}
-
-// The quantised box bytes of a child in the node's frame.
-__device__ __forceinline__ uint32_t quant_lo(float c, float p, float inv)
-{
-    const float q = floorf(__fmul_rd(__fsub_rd(c, p), inv)) - 1.0f;
-    return (uint32_t)fminf(fmaxf(q, 0.f), 255.f);
-}
-__device__ __forceinline__ uint32_t quant_hi(float c, float p, float inv)
-{
-    const float q = ceilf(__fmul_ru(__fsub_ru(c, p), inv)) + 1.0f;
-    return (uint32_t)fminf(fmaxf(q, 0.f), 255.f);
 }
 
 // Lane groups of 8 within a warp: ballots, reductions and shuffles confined
@@ -1496,18 +1494,6 @@ __device__ __forceinline__ uint32_t gor(uint32_t v)
     v |= __shfl_xor_sync(0xffffffffu, v, 4);
     v |= __shfl_xor_sync(0xffffffffu, v, 2);
     return v | __shfl_xor_sync(0xffffffffu, v, 1);
-}
-
-// Word h (0: slots 0-3, 1: slots 4-7) of a per-slot byte plane: every lane
-// of the group that holds a child in that half contributes its byte; empty
-// slots read `empty`.
-__device__ __forceinline__ uint32_t plane_word(bool mine, int slot, uint32_t byte, int h, uint32_t empty)
-{
-    const bool in = mine && (slot >> 2) == h;
-    const uint32_t sh = 8u * (uint32_t)(slot & 3);
-    const uint32_t occ = gor(in ? (0xffu << sh) : 0u);
-    const uint32_t val = gor(in ? (byte << sh) : 0u);
-    return (empty & ~occ) | val;
 }
 
 // One wide node per group of 8 lanes (surface-area decisions), four per
@@ -1683,11 +1669,12 @@ __device__ __forceinline__ void collapse_task_group(const BuildArgs &A, const in
     const float ix = __int_as_float((254 - ex) << 23);   // exact 1/unit
     const float iy = __int_as_float((254 - ey) << 23);
     const float iz = __int_as_float((254 - ez) << 23);
-    uint32_t meta = 0, qlx = 255, qly = 255, qlz = 255, qhx = 0, qhy = 0, qhz = 0;
+    uint32_t meta = 0, qx = 0, qy = 0, qz = 0;
     if (active) {
-        qlx = quant_lo(lo.x, px, ix); qly = quant_lo(lo.y, py, iy); qlz = quant_lo(lo.z, pz, iz);
-        qhx = quant_hi(hi.x, px, ix); qhy = quant_hi(hi.y, py, iy); qhz = quant_hi(hi.z, pz, iz);
-        meta = internal ? (0x20u | (uint32_t)(24 + myslot)) : ((((1u << cnt) - 1u) << 5) | (uint32_t)tri_off);
+        qx = quant_planes(lo.x, hi.x, px, ix);
+        qy = quant_planes(lo.y, hi.y, py, iy);
+        qz = quant_planes(lo.z, hi.z, pz, iz);
+        meta = internal ? 0x80u : (((uint32_t)cnt << 5) | (uint32_t)tri_off);
     }
     uint32_t w[20];
     w[0] = __float_as_uint(px);
@@ -1696,15 +1683,16 @@ __device__ __forceinline__ void collapse_task_group(const BuildArgs &A, const in
     w[3] = (uint32_t)ex | ((uint32_t)ey << 8) | ((uint32_t)ez << 16) | (imask << 24);
     w[4] = (uint32_t)child_base;
     w[5] = (uint32_t)tri_base;
+    w[6] = gor(active && myslot < 4 ? meta << (8 * myslot) : 0u);
+    w[7] = gor(active && myslot >= 4 ? meta << (8 * (myslot - 4)) : 0u);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        w[6 + h] = plane_word(active, myslot, meta, h, 0u);
-        w[8 + h] = plane_word(active, myslot, qlx, h, 0xffffffffu);
-        w[10 + h] = plane_word(active, myslot, qly, h, 0xffffffffu);
-        w[12 + h] = plane_word(active, myslot, qlz, h, 0xffffffffu);
-        w[14 + h] = plane_word(active, myslot, qhx, h, 0u);
-        w[16 + h] = plane_word(active, myslot, qhy, h, 0u);
-        w[18 + h] = plane_word(active, myslot, qhz, h, 0u);
+    for (int h = 0; h < 4; ++h) {
+        const bool in = active && (myslot >> 1) == h;
+        const uint32_t sh = 16u * (uint32_t)(myslot & 1);
+        const uint32_t none = kEmptyPlanes * 0x10001u & ~gor(in ? 0xffffu << sh : 0u);
+        w[8 + h] = none | gor(in ? qx << sh : 0u);
+        w[12 + h] = none | gor(in ? qy << sh : 0u);
+        w[16 + h] = none | gor(in ? qz << sh : 0u);
     }
     const uint32_t occ = gor(active ? (1u << myslot) : 0u);
     if (!writes || !fits) return;   // after the last group operation
@@ -2092,10 +2080,9 @@ __global__ void k_requant(WideNode *__restrict__ nodes, int32_t nnodes, const in
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
         if (!((occ >> s) & 1u)) continue;
-        W.qlo_x[s] = (uint8_t)quant_lo(lo[s].x, px, ix); W.qlo_y[s] = (uint8_t)quant_lo(lo[s].y, py, iy);
-        W.qlo_z[s] = (uint8_t)quant_lo(lo[s].z, pz, iz);
-        W.qhi_x[s] = (uint8_t)quant_hi(hi[s].x, px, ix); W.qhi_y[s] = (uint8_t)quant_hi(hi[s].y, py, iy);
-        W.qhi_z[s] = (uint8_t)quant_hi(hi[s].z, pz, iz);
+        W.qx[s] = quant_planes(lo[s].x, hi[s].x, px, ix);
+        W.qy[s] = quant_planes(lo[s].y, hi[s].y, py, iy);
+        W.qz[s] = quant_planes(lo[s].z, hi[s].z, pz, iz);
     }
     nodes[w] = W;
 }

@@ -59,8 +59,8 @@ struct PixelOut {
 // (ray_trace_engine::ray_trace, raytracer.cc:20-87).  TABLE: the hit
 // triangle's material from `table` (per-triangle indices in sc.mat), else
 // `mat0` for every triangle.
-template <bool COUNT, bool TABLE = false, int STACK = kStackSize>
-__device__ __forceinline__ PixelOut shade_pixel_lights(const SceneView &sc, const CameraView &cam, const LightView *lights,
+template <bool COUNT, bool TABLE = false, int STACK = kStackSize, class SC>
+__device__ __forceinline__ PixelOut shade_pixel_lights(const SC &sc, const CameraView &cam, const LightView *lights,
                                                        int nl, const MaterialView &mat0, int x, int y,
                                                        uint32_t &status, FetchCount *fc, bool fast_pow,
                                                        const MaterialTable *table = nullptr)
@@ -132,8 +132,8 @@ struct TreeFrame {
 // surface), each child's colour added to its parent's times rf, then tran
 // (combind_secondary_rays, coloured_mapper_shader.cc:117-130).  A ray that
 // misses is the background.  `frames` holds RT_MAX_BOUNCES + 1 entries.
-template <bool COUNT>
-__device__ __forceinline__ PixelOut shade_pixel_tree(const SceneView &sc, const CameraView &cam, const LightView *lights,
+template <bool COUNT, class SC>
+__device__ __forceinline__ PixelOut shade_pixel_tree(const SC &sc, const CameraView &cam, const LightView *lights,
                                                      int nl, const MaterialTable &mt, int x, int y, TreeFrame *frames,
                                                      uint32_t &status, FetchCount *fc)
 {
@@ -256,8 +256,8 @@ __device__ __forceinline__ PixelOut shade_pixel_tree(const SceneView &sc, const 
 }
 
 // Primary ray, closest hit, `samples` cosine-weighted AO rays within ao_dist.
-template <bool COUNT, int STACK = kStackSize>
-__device__ __forceinline__ PixelOut shade_pixel_ao(const SceneView &sc, const CameraView &cam, const MaterialView &mat,
+template <bool COUNT, int STACK = kStackSize, class SC>
+__device__ __forceinline__ PixelOut shade_pixel_ao(const SC &sc, const CameraView &cam, const MaterialView &mat,
                                                    int samples, float ao_dist, uint32_t seed, int x, int y,
                                                    uint32_t &status, FetchCount *fc)
 {

@@ -24,6 +24,7 @@
 #include <cstring>
 #include <new>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include <cub/cub.cuh>
@@ -302,7 +303,8 @@ struct AreaSet {
 };
 
 // Pass 1: the camera ray of every pixel; hit record and hit flag.
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_primary(SceneView sc, CameraView cam,
+template <class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_primary(SC sc, CameraView cam,
                                                                                       int4 *__restrict__ hits,
                                                                                       int32_t *__restrict__ flags,
                                                                                       Counters *ctr)
@@ -335,8 +337,9 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_pr
 
 // Pass 2: shading.  rnd holds the frame's numbers (rnd[0] = the frame's
 // first), nrnd of them; a hit pixel's first is prefix[pix] * per_hit.
+template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_shade(
-    SceneView sc, CameraView cam, LightSet lights, MaterialTable table, AreaSet areas, const int4 *__restrict__ area,
+    SC sc, CameraView cam, LightSet lights, MaterialTable table, AreaSet areas, const int4 *__restrict__ area,
     const float *__restrict__ verts, int32_t samples, int32_t per_hit, const float *__restrict__ rnd, int64_t nrnd,
     const float *__restrict__ lut, const int4 *__restrict__ hits, const int32_t *__restrict__ prefix,
     uint8_t *__restrict__ rgb, float *__restrict__ fimg, Counters *ctr)
@@ -589,7 +592,8 @@ __device__ __forceinline__ void spawn_child(const DistFrame &f, const MaterialVi
 // numbers the pixel draws in the reference's order (at each hit: the
 // lights' rays, then the reflection set, then the refraction set; then the
 // children's subtrees in order).
-__device__ __forceinline__ uint32_t dist_count_pixel(const SceneView &sc, const CameraView &cam,
+template <class SC>
+__device__ __forceinline__ uint32_t dist_count_pixel(const SC &sc, const CameraView &cam,
                                                      const LightSet &lights, const MaterialTable &table,
                                                      const DistLights &dl, const DistParams &dp,
                                                      const float *__restrict__ lut, DistStream &S, int x, int y,
@@ -883,13 +887,13 @@ __device__ __forceinline__ bool walk_advance(Walk &w, const SceneView &sc, const
 
 // Takes the result of the ray walk_advance asked for.
 template <int MODE>
-__device__ __forceinline__ void walk_consume(Walk &w, const Trav &T, bool any, const SceneView &sc,
+__device__ __forceinline__ void walk_consume(Walk &w, const HitRecord &h, bool occluded, bool any, const SceneView &sc,
                                              const CameraView &cam, const LightSet &lights, const MaterialTable &table,
                                              const DistParams &dp, DistFrame *F, uint32_t &status)
 {
     DistFrame &f = F[w.sp - 1];
     if (any) {
-        if (!T.occluded) ++w.made;
+        if (!occluded) ++w.made;
         ++w.sample;
         return;
     }
@@ -897,7 +901,7 @@ __device__ __forceinline__ void walk_consume(Walk &w, const Trav &T, bool any, c
     if (w.sp > 1 || MODE == kDistSub) ++w.nsec;
     f.nrefl = 0;
     f.nrefr = 0;
-    if (!(T.hit.t < FLT_MAX)) {
+    if (!(h.t < FLT_MAX)) {
         f.c = cam.background;
         f.stage = kDistDone;
         if (MODE == kDistRoot) {
@@ -906,7 +910,7 @@ __device__ __forceinline__ void walk_consume(Walk &w, const Trav &T, bool any, c
         }
         return;
     }
-    const int32_t id = T.hit.id - sc.tri_base;
+    const int32_t id = h.id - sc.tri_base;
     if (w.sp == 1 && MODE != kDistSub) w.hit = true;
     int32_t mi = sc.mat ? __ldg(&sc.mat[id]) : 0;
     if (mi < 0 || mi >= table.n) { status |= kStatusBadIndex; mi = 0; }
@@ -914,7 +918,7 @@ __device__ __forceinline__ void walk_consume(Walk &w, const Trav &T, bool any, c
     RayState r;
     r.o = f.o;
     r.d = f.d;
-    const SurfacePoint spt = surface_at(sc, r, T.hit);
+    const SurfacePoint spt = surface_at(sc, r, h);
     w.start = offset_start(spt.dst, spt.geo);
     w.kd = material_kd(m, spt);
     w.c = make_float3(0.f, 0.f, 0.f);
@@ -937,8 +941,8 @@ __device__ __forceinline__ void walk_consume(Walk &w, const Trav &T, bool any, c
 
 // The whole walk of one lane (its lanes' rays traced together while their
 // walks last).
-template <int MODE>
-__device__ __forceinline__ uint32_t dist_walk(const SceneView &sc, const CameraView &cam, const LightSet &lights,
+template <int MODE, class SC>
+__device__ __forceinline__ uint32_t dist_walk(const SC &sc, const CameraView &cam, const LightSet &lights,
                                               const MaterialTable &table, const DistLights &dl, const DistParams &dp,
                                               const int4 *__restrict__ area, const float *__restrict__ verts,
                                               const float *__restrict__ lut, DistStream &S, int x, int y,
@@ -947,17 +951,15 @@ __device__ __forceinline__ uint32_t dist_walk(const SceneView &sc, const CameraV
 {
     Walk w;
     walk_start<MODE>(w, cam, F, x, y);
-    uint2 stack[kStackSize];
     for (;;) {
         float3 ro, rd;
         float rt;
         bool any;
         if (!walk_advance<MODE>(w, sc, lights, table, dl, dp, area, verts, lut, S, F, ro, rd, rt, any, status)) break;
-        Trav T;
-        trav_begin(T, sc, ro, rd, rt, any);
-        while (!trav_step<false>(T, stack, sc, any, status, nullptr)) {
-        }
-        walk_consume<MODE>(w, T, any, sc, cam, lights, table, dp, F, status);
+        HitRecord h;
+        bool occluded;
+        status |= traverse_ray<false>(sc, ro, rd, rt, any, h, occluded);
+        walk_consume<MODE>(w, h, occluded, any, sc, cam, lights, table, dp, F, status);
     }
     out = w.out;
     hit = w.hit;
@@ -975,8 +977,8 @@ __device__ __forceinline__ uint32_t dist_walk(const SceneView &sc, const CameraV
 #ifndef RT_DIST_MIN_BLOCKS
 #define RT_DIST_MIN_BLOCKS 5
 #endif
-template <bool SHADE>
-__global__ void __launch_bounds__(kTraceThreads, RT_DIST_MIN_BLOCKS) k_dist(SceneView sc, CameraView cam, LightSet lights,
+template <bool SHADE, class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_DIST_MIN_BLOCKS) k_dist(SC sc, CameraView cam, LightSet lights,
                                                         MaterialTable table, DistLights dl, DistParams dp,
                                                         const int4 *__restrict__ area, const float *__restrict__ verts,
                                                         const float *__restrict__ lut, const float *__restrict__ rnd,
@@ -1066,8 +1068,9 @@ __device__ __forceinline__ DistStream pixel_streams(const DistParams &dp, uint32
     return S;
 }
 
+template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_DIST_MIN_BLOCKS) k_dist_root(
-    SceneView sc, CameraView cam, LightSet lights, MaterialTable table, DistLights dl, DistParams dp,
+    SC sc, CameraView cam, LightSet lights, MaterialTable table, DistLights dl, DistParams dp,
     const int4 *__restrict__ area, const float *__restrict__ verts, const float *__restrict__ lut,
     float4 *__restrict__ root_c, int4 *__restrict__ root_sets, DistItem *__restrict__ items, int32_t cap,
     int32_t *__restrict__ nitems, Counters *ctr)
@@ -1150,8 +1153,9 @@ __global__ void __launch_bounds__(kTraceThreads, RT_DIST_MIN_BLOCKS) k_dist_root
 #ifndef RT_DIST_SUB_MIN_BLOCKS
 #define RT_DIST_SUB_MIN_BLOCKS 6
 #endif
+template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_DIST_SUB_MIN_BLOCKS) k_dist_sub(
-    SceneView sc, CameraView cam, LightSet lights, MaterialTable table, DistLights dl, DistParams dp,
+    SC sc, CameraView cam, LightSet lights, MaterialTable table, DistLights dl, DistParams dp,
     const int4 *__restrict__ area, const float *__restrict__ verts, const float *__restrict__ lut,
     const DistItem *__restrict__ items, int32_t nr, int32_t nt, int32_t cap, float4 *__restrict__ item_c,
     Counters *ctr)
@@ -1267,11 +1271,12 @@ rt_status check_shapes(const rt_scene *s, const rt_light *lights, int32_t nlight
                        const char *who);
 rt_status stream_window(SoftState &S, int64_t offset, int64_t total, cudaStream_t st, const float **rnd);
 
+template <class SC>
 int soft_blocks_per_sm()
 {
     static const int per_sm = [] {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_soft_shade, kTraceThreads, 0) != cudaSuccess || b < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_soft_shade<SC>, kTraceThreads, 0) != cudaSuccess || b < 1) {
             cudaGetLastError();
             b = 4;
         }
@@ -1377,11 +1382,14 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
     for (int i = 0; i < nmaterials; ++i) mt.m[i] = make_material_view(materials[i]);
     const SceneView sv = scene_view(s);
     const CameraView cv = make_camera_view(*camera);
-    const int grid = soft_blocks_per_sm() * ctx->sm_count;
 
     RT_CUDA_S(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), st), "counter clear");
     RT_CUDA_S(cudaEventRecord(ctx->ev0, st), "event record");
-    k_soft_primary<<<grid, kTraceThreads, 0, st>>>(sv, cv, (int4 *)S.hits.ptr, (int32_t *)S.flags.ptr, ctx->d_counters);
+    with_scene(sv, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        k_soft_primary<SC><<<soft_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
+            view, cv, (int4 *)S.hits.ptr, (int32_t *)S.flags.ptr, ctx->d_counters);
+    });
     RT_CUDA_S(cudaGetLastError(), "primary launch");
     cub::DeviceScan::ExclusiveSum(S.scan_temp.ptr, scan_bytes, (const int32_t *)S.flags.ptr, (int32_t *)S.prefix.ptr,
                                   (int)npix, st);
@@ -1417,10 +1425,13 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
         d_f = (float *)ctx->fimg.ptr;
     }
     RT_CUDA_S(cudaMemsetAsync(&ctx->d_counters->work, 0, sizeof(int), st), "work counter clear");
-    k_soft_shade<<<grid, kTraceThreads, 0, st>>>(sv, cv, ls, mt, as, (const int4 *)S.area.ptr, s->d_verts, samples,
-                                                 per_hit, rnd, total, (const float *)S.lut.ptr,
-                                                 (const int4 *)S.hits.ptr, (const int32_t *)S.prefix.ptr, d_rgb, d_f,
-                                                 ctx->d_counters);
+    with_scene(sv, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        k_soft_shade<SC><<<soft_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
+            view, cv, ls, mt, as, (const int4 *)S.area.ptr, s->d_verts, samples, per_hit, rnd, total,
+            (const float *)S.lut.ptr, (const int4 *)S.hits.ptr, (const int32_t *)S.prefix.ptr, d_rgb, d_f,
+            ctx->d_counters);
+    });
     RT_CUDA_S(cudaGetLastError(), "shade launch");
     RT_CUDA_S(cudaEventRecord(ctx->ev1, st), "event record");
     if (rgb_host) RT_CUDA_S(cudaMemcpyAsync(rgb_out, d_rgb, npix * 3, cudaMemcpyDeviceToHost, st), "rgb copy");
@@ -1446,11 +1457,12 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
 
 namespace {
 
+template <class SC>
 int sub_blocks_per_sm()
 {
     static const int per_sm = [] {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_dist_sub, kTraceThreads, 0) != cudaSuccess || b < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_dist_sub<SC>, kTraceThreads, 0) != cudaSuccess || b < 1) {
             cudaGetLastError();
             b = 2;
         }
@@ -1459,11 +1471,12 @@ int sub_blocks_per_sm()
     return per_sm;
 }
 
+template <class SC>
 int dist_blocks_per_sm()
 {
     static const int per_sm = [] {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_dist<true>, kTraceThreads, 0) != cudaSuccess || b < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (k_dist<true, SC>), kTraceThreads, 0) != cudaSuccess || b < 1) {
             cudaGetLastError();
             b = 2;
         }
@@ -1791,7 +1804,6 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
     const SceneView sv = scene_view(s);
     const CameraView cv = make_camera_view(*camera);
     const size_t npix = (size_t)camera->xres * (size_t)camera->yres;
-    const int grid = dist_blocks_per_sm() * ctx->sm_count;
 
     RT_CUDA_S(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), st), "counter clear");
     RT_CUDA_S(cudaEventRecord(ctx->ev0, st), "event record");
@@ -1805,9 +1817,12 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
         cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (const int64_t *)S.counts.ptr, (int64_t *)S.prefix64.ptr,
                                       (int)npix, st);
         RT_CUDA_S(S.scan64_temp.reserve(scan_bytes), "scan scratch allocation");
-        k_dist<false><<<grid, kTraceThreads, 0, st>>>(sv, cv, ls, mt, dl, dp, (const int4 *)S.area.ptr, s->d_verts,
-                                                      (const float *)S.lut.ptr, nullptr, 0, nullptr,
-                                                      (int64_t *)S.counts.ptr, nullptr, nullptr, ctx->d_counters);
+        with_scene(sv, [&](const auto &view) {
+            using SC = std::decay_t<decltype(view)>;
+            k_dist<false, SC><<<dist_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
+                view, cv, ls, mt, dl, dp, (const int4 *)S.area.ptr, s->d_verts, (const float *)S.lut.ptr, nullptr, 0,
+                nullptr, (int64_t *)S.counts.ptr, nullptr, nullptr, ctx->d_counters);
+        });
         RT_CUDA_S(cudaGetLastError(), "counting launch");
         cub::DeviceScan::ExclusiveSum(S.scan64_temp.ptr, scan_bytes, (const int64_t *)S.counts.ptr,
                                       (int64_t *)S.prefix64.ptr, (int)npix, st);
@@ -1853,10 +1868,13 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
             RT_CUDA_S(S.item_c.reserve(2 * (size_t)cap * sizeof(float4)), "item colour allocation");
             RT_CUDA_S(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), st), "counter clear");
             RT_CUDA_S(cudaMemsetAsync(S.nitems.ptr, 0, 2 * sizeof(int32_t), st), "item counter clear");
-            k_dist_root<<<grid, kTraceThreads, 0, st>>>(sv, cv, ls, mt, dl, dp, (const int4 *)S.area.ptr, s->d_verts,
-                                                        (const float *)S.lut.ptr, (float4 *)S.root_c.ptr,
-                                                        (int4 *)S.root_sets.ptr, (DistItem *)S.items.ptr, (int32_t)cap,
-                                                        (int32_t *)S.nitems.ptr, ctx->d_counters);
+            with_scene(sv, [&](const auto &view) {
+                using SC = std::decay_t<decltype(view)>;
+                k_dist_root<SC><<<dist_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
+                    view, cv, ls, mt, dl, dp, (const int4 *)S.area.ptr, s->d_verts, (const float *)S.lut.ptr,
+                    (float4 *)S.root_c.ptr, (int4 *)S.root_sets.ptr, (DistItem *)S.items.ptr, (int32_t)cap,
+                    (int32_t *)S.nitems.ptr, ctx->d_counters);
+            });
             RT_CUDA_S(cudaGetLastError(), "node launch");
             RT_CUDA_S(cudaMemcpyAsync(n, S.nitems.ptr, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st),
                       "item count read");
@@ -1870,18 +1888,23 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
         S.item_cap = cap;
         RT_CUDA_S(cudaMemsetAsync(&ctx->d_counters->work, 0, sizeof(int), st), "work counter clear");
         if (n[0] + n[1] > 0)
-            k_dist_sub<<<sub_blocks_per_sm() * ctx->sm_count, kTraceThreads, 0, st>>>(
-                sv, cv, ls, mt, dl, dp, (const int4 *)S.area.ptr, s->d_verts, (const float *)S.lut.ptr,
-                (const DistItem *)S.items.ptr, n[0], n[1], (int32_t)cap, (float4 *)S.item_c.ptr, ctx->d_counters);
+            with_scene(sv, [&](const auto &view) {
+                using SC = std::decay_t<decltype(view)>;
+                k_dist_sub<SC><<<sub_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
+                    view, cv, ls, mt, dl, dp, (const int4 *)S.area.ptr, s->d_verts, (const float *)S.lut.ptr,
+                    (const DistItem *)S.items.ptr, n[0], n[1], (int32_t)cap, (float4 *)S.item_c.ptr, ctx->d_counters);
+            });
         RT_CUDA_S(cudaGetLastError(), "subtree launch");
         k_dist_combine<<<ctx->sm_count * 8, 256, 0, st>>>(cv, mt, (const float4 *)S.root_c.ptr,
                                                           (const int4 *)S.root_sets.ptr, (const float4 *)S.item_c.ptr,
                                                           n[0], n[1], (int32_t)cap, d_rgb, d_f, ctx->d_counters);
     } else {
-        k_dist<true><<<grid, kTraceThreads, 0, st>>>(sv, cv, ls, mt, dl, dp, (const int4 *)S.area.ptr, s->d_verts,
-                                                     (const float *)S.lut.ptr, rnd, total,
-                                                     (const int64_t *)S.prefix64.ptr, nullptr, d_rgb, d_f,
-                                                     ctx->d_counters);
+        with_scene(sv, [&](const auto &view) {
+            using SC = std::decay_t<decltype(view)>;
+            k_dist<true, SC><<<dist_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
+                view, cv, ls, mt, dl, dp, (const int4 *)S.area.ptr, s->d_verts, (const float *)S.lut.ptr, rnd, total,
+                (const int64_t *)S.prefix64.ptr, nullptr, d_rgb, d_f, ctx->d_counters);
+        });
     }
     RT_CUDA_S(cudaGetLastError(), "shade launch");
     RT_CUDA_S(cudaEventRecord(ctx->ev1, st), "event record");

@@ -3,13 +3,16 @@
 // Every kernel runs a fixed grid (a multiple of the SM count) whose warps
 // claim 32 work items at a time from a device counter, so uneven ray costs
 // balance across SMs without a scheduler on the host.
+#include <type_traits>
+
 #include "rt_shade.cuh"
 
 namespace rtc {
 
 namespace {
 
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_closest(SceneView sc, const rt_ray *__restrict__ rays,
+template <class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_closest(SC sc, const rt_ray *__restrict__ rays,
                                                                  int32_t n, rt_hit *__restrict__ hits,
                                                                  Counters *ctr)
 {
@@ -30,7 +33,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_c
     if (status) atomicOr(&ctr->status, status);
 }
 
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_any(SceneView sc, const rt_ray *__restrict__ rays, int32_t n,
+template <class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_any(SC sc, const rt_ray *__restrict__ rays, int32_t n,
                                                              uint8_t *__restrict__ occluded, Counters *ctr)
 {
     uint32_t status = 0;
@@ -54,8 +58,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_a
 
 namespace {
 
-template <bool COUNT>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render(SceneView sc, CameraView cam, LightSet lights,
+template <bool COUNT, class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render(SC sc, CameraView cam, LightSet lights,
                                                           MaterialView mat, uint8_t *__restrict__ rgb,
                                                           int32_t *__restrict__ ids, Counters *ctr)
 {
@@ -93,8 +97,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render(
 // frame without secondary rays, for the tone-mapping epilogue: the fused
 // primary + shadow kernel, its material per triangle from `table` (entry 0
 // when the scene has no indices).
-template <bool COUNT>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_float(SceneView sc, CameraView cam, LightSet lights,
+template <bool COUNT, class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_float(SC sc, CameraView cam, LightSet lights,
                                                           MaterialTable table, float *__restrict__ fimg,
                                                           Counters *ctr)
 {
@@ -133,8 +137,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
 // k_render with the hit triangle's material taken from a table
 // (rt_render_materials without mirror or refracted rays): a separate kernel
 // so that the single-material one keeps its code and parameter block.
-template <bool COUNT>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_table(SceneView sc, CameraView cam, LightSet lights,
+template <bool COUNT, class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_table(SC sc, CameraView cam, LightSet lights,
                                                           MaterialView mat, uint8_t *__restrict__ rgb,
                                                           int32_t *__restrict__ ids, Counters *ctr,
                                                           MaterialTable table)
@@ -176,8 +180,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
 #define RT_AO_SPREAD 1
 #endif
 
-template <bool COUNT>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_ao(SceneView sc, CameraView cam, MaterialView mat,
+template <bool COUNT, class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_ao(SC sc, CameraView cam, MaterialView mat,
                                                              int32_t samples, float ao_dist, uint32_t seed,
                                                              uint8_t *__restrict__ rgb, int32_t *__restrict__ ids,
                                                              int32_t *__restrict__ ao_count, Counters *ctr)
@@ -296,8 +300,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
 // the truncation guard of an integer is queued (redo) for k_render_aa_fix,
 // which recomputes it from samples shaded with the exact power in a compact
 // second pass, so that no warp waits on one lane's exact re-shade.
-template <bool COUNT>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa(SceneView sc, CameraView cam,
+template <bool COUNT, class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa(SC sc, CameraView cam,
                                                              LightSet lights, MaterialView mat, int32_t aa_x,
                                                              int32_t aa_y, int32_t out_x, int32_t out_y,
                                                              uint8_t *__restrict__ rgb, int32_t *__restrict__ redo,
@@ -353,8 +357,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
 // (shuffled from their lanes), so the frame is the per-pixel loop's bit for
 // bit, while the warp's lanes trace one sample each instead of looping
 // over a pixel's samples.
-template <bool COUNT>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa_lanes(SceneView sc, CameraView cam,
+template <bool COUNT, class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa_lanes(SC sc, CameraView cam,
                                                              LightSet lights, MaterialView mat, int32_t aa_x,
                                                              int32_t aa_y, int32_t out_x, int32_t out_y,
                                                              uint8_t *__restrict__ rgb, int32_t *__restrict__ redo,
@@ -417,7 +421,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
 
 // The queued pixels of k_render_aa, one per thread, every sample shaded
 // with the exact specular power.
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa_fix(SceneView sc, CameraView cam,
+template <class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa_fix(SC sc, CameraView cam,
                                                                  LightSet lights, MaterialView mat, int32_t aa_x,
                                                                  int32_t aa_y, int32_t out_x,
                                                                  uint8_t *__restrict__ rgb,
@@ -454,8 +459,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
 #define RT_TREE_MIN_BLOCKS 5
 #endif
 
-template <bool COUNT>
-__global__ void __launch_bounds__(kTraceThreads, RT_TREE_MIN_BLOCKS) k_render_tree(SceneView sc, CameraView cam, LightSet lights,
+template <bool COUNT, class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_TREE_MIN_BLOCKS) k_render_tree(SC sc, CameraView cam, LightSet lights,
                                                                MaterialTable mt, uint8_t *__restrict__ rgb,
                                                                float *__restrict__ fimg, int32_t *__restrict__ ids,
                                                                Counters *ctr)
@@ -535,62 +540,80 @@ static int blocks_per_sm(K kernel)
 void launch_trace_closest(const SceneView &sc, const rt_ray *rays, int32_t n, rt_hit *hits, Counters *ctr, int sm_count,
                           cudaStream_t st)
 {
-    static const int per_sm = blocks_per_sm(k_trace_closest);
-    const int grid = per_sm * sm_count;
-    k_trace_closest<<<grid, kTraceThreads, 0, st>>>(sc, rays, n, hits, ctr);
+    with_scene(sc, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_trace_closest<SC>);
+        const int grid = per_sm * sm_count;
+        k_trace_closest<SC><<<grid, kTraceThreads, 0, st>>>(view, rays, n, hits, ctr);
+    });
 }
 
 void launch_trace_any(const SceneView &sc, const rt_ray *rays, int32_t n, uint8_t *occ, Counters *ctr, int sm_count,
                       cudaStream_t st)
 {
-    static const int per_sm = blocks_per_sm(k_trace_any);
-    const int grid = per_sm * sm_count;
-    k_trace_any<<<grid, kTraceThreads, 0, st>>>(sc, rays, n, occ, ctr);
+    with_scene(sc, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_trace_any<SC>);
+        const int grid = per_sm * sm_count;
+        k_trace_any<SC><<<grid, kTraceThreads, 0, st>>>(view, rays, n, occ, ctr);
+    });
 }
 
 void launch_render(const SceneView &sc, const CameraView &cam, const LightSet &lights, const MaterialView &mat,
                    uint8_t *rgb, int32_t *ids, Counters *ctr, int sm_count, cudaStream_t st, bool count)
 {
-    static const int per_sm = blocks_per_sm(k_render<false>);
-    const int grid = per_sm * sm_count;
-    if (count)
-        k_render<true><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mat, rgb, ids, ctr);
-    else
-        k_render<false><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mat, rgb, ids, ctr);
+    with_scene(sc, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_render<false, SC>);
+        const int grid = per_sm * sm_count;
+        if (count)
+            k_render<true, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, rgb, ids, ctr);
+        else
+            k_render<false, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, rgb, ids, ctr);
+    });
 }
 
 void launch_render_float(const SceneView &sc, const CameraView &cam, const LightSet &lights, const MaterialTable &mt,
                          float *fimg, Counters *ctr, int sm_count, cudaStream_t st, bool count)
 {
-    static const int per_sm = blocks_per_sm(k_render_float<false>);
-    const int grid = per_sm * sm_count;
-    if (count)
-        k_render_float<true><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mt, fimg, ctr);
-    else
-        k_render_float<false><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mt, fimg, ctr);
+    with_scene(sc, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_render_float<false, SC>);
+        const int grid = per_sm * sm_count;
+        if (count)
+            k_render_float<true, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mt, fimg, ctr);
+        else
+            k_render_float<false, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mt, fimg, ctr);
+    });
 }
 
 void launch_render_table(const SceneView &sc, const CameraView &cam, const LightSet &lights, const MaterialTable &mt,
                          uint8_t *rgb, int32_t *ids, Counters *ctr, int sm_count, cudaStream_t st, bool count)
 {
-    static const int per_sm = blocks_per_sm(k_render_table<false>);
-    const int grid = per_sm * sm_count;
-    if (count)
-        k_render_table<true><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mt.m[0], rgb, ids, ctr, mt);
-    else
-        k_render_table<false><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mt.m[0], rgb, ids, ctr, mt);
+    with_scene(sc, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_render_table<false, SC>);
+        const int grid = per_sm * sm_count;
+        if (count)
+            k_render_table<true, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mt.m[0], rgb, ids, ctr, mt);
+        else
+            k_render_table<false, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mt.m[0], rgb, ids, ctr, mt);
+    });
 }
 
 void launch_render_tree(const SceneView &sc, const CameraView &cam, const LightSet &lights, const MaterialTable &mt,
                         uint8_t *rgb, float *fimg, int32_t *ids, Counters *ctr, int sm_count, cudaStream_t st,
                         bool count)
 {
-    static const int per_sm = blocks_per_sm(k_render_tree<false>);
-    const int grid = per_sm * sm_count;
-    if (count)
-        k_render_tree<true><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mt, rgb, fimg, ids, ctr);
-    else
-        k_render_tree<false><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mt, rgb, fimg, ids, ctr);
+    with_scene(sc, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_render_tree<false, SC>);
+        const int grid = per_sm * sm_count;
+        if (count)
+            k_render_tree<true, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mt, rgb, fimg, ids, ctr);
+        else
+            k_render_tree<false, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mt, rgb, fimg, ids, ctr);
+    });
 }
 
 void launch_index_range(const int32_t *v, int32_t n, int32_t *out, cudaStream_t st)
@@ -605,35 +628,41 @@ void launch_render_aa(const SceneView &sc, const CameraView &cam, const LightSet
                       int32_t aa_x, int32_t aa_y, int32_t out_x, int32_t out_y, uint8_t *rgb, int32_t *redo,
                       Counters *ctr, int sm_count, cudaStream_t st, bool count)
 {
-    static const int per_sm = blocks_per_sm(k_render_aa<false>);
-    const int grid = per_sm * sm_count;
-    if (aa_x * aa_y <= 32) {
-        if (count)
-            k_render_aa_lanes<true><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mat, aa_x, aa_y, out_x, out_y,
-                                                                     rgb, redo, ctr);
+    with_scene(sc, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_render_aa<false, SC>);
+        const int grid = per_sm * sm_count;
+        if (aa_x * aa_y <= 32) {
+            if (count)
+                k_render_aa_lanes<true, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, aa_x, aa_y, out_x, out_y,
+                                                                         rgb, redo, ctr);
+            else
+                k_render_aa_lanes<false, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, aa_x, aa_y, out_x, out_y,
+                                                                          rgb, redo, ctr);
+        } else if (count)
+            k_render_aa<true, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, aa_x, aa_y, out_x, out_y, rgb, redo,
+                                                               ctr);
         else
-            k_render_aa_lanes<false><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mat, aa_x, aa_y, out_x, out_y,
-                                                                      rgb, redo, ctr);
-    } else if (count)
-        k_render_aa<true><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mat, aa_x, aa_y, out_x, out_y, rgb, redo,
-                                                           ctr);
-    else
-        k_render_aa<false><<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mat, aa_x, aa_y, out_x, out_y, rgb, redo,
-                                                            ctr);
-    if (lights.fast_pow)
-        k_render_aa_fix<<<grid, kTraceThreads, 0, st>>>(sc, cam, lights, mat, aa_x, aa_y, out_x, rgb, redo, ctr);
+            k_render_aa<false, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, aa_x, aa_y, out_x, out_y, rgb, redo,
+                                                                ctr);
+        if (lights.fast_pow)
+            k_render_aa_fix<SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, aa_x, aa_y, out_x, rgb, redo, ctr);
+    });
 }
 
 void launch_render_ao(const SceneView &sc, const CameraView &cam, const MaterialView &mat, int32_t samples,
                       float ao_dist, uint32_t seed, uint8_t *rgb, int32_t *ids, int32_t *ao_count, Counters *ctr,
                       int sm_count, cudaStream_t st, bool count)
 {
-    static const int per_sm = blocks_per_sm(k_render_ao<false>);
-    const int grid = per_sm * sm_count;
-    if (count)
-        k_render_ao<true><<<grid, kTraceThreads, 0, st>>>(sc, cam, mat, samples, ao_dist, seed, rgb, ids, ao_count, ctr);
-    else
-        k_render_ao<false><<<grid, kTraceThreads, 0, st>>>(sc, cam, mat, samples, ao_dist, seed, rgb, ids, ao_count, ctr);
+    with_scene(sc, [&](const auto &view) {
+        using SC = std::decay_t<decltype(view)>;
+        static const int per_sm = blocks_per_sm(k_render_ao<false, SC>);
+        const int grid = per_sm * sm_count;
+        if (count)
+            k_render_ao<true, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, mat, samples, ao_dist, seed, rgb, ids, ao_count, ctr);
+        else
+            k_render_ao<false, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, mat, samples, ao_dist, seed, rgb, ids, ao_count, ctr);
+    });
 }
 
 }  // namespace rtc

@@ -3,8 +3,8 @@
 // every kernel of the core.
 //
 // Traversal keeps node groups (child base + hit bits) on a per-ray stack:
-// internal-child hits live in bits 24..31 at position (slot ^ octant) so the
-// lowest set bit is the child nearest the ray's origin side, the node's
+// internal-child hits live in bits 24..31 at position slot ^ octant ^ 7 so the
+// highest set bit is the child nearest the ray's origin side, the node's
 // internal-child mask rides in bits 0..7, and leaf triangles of a node are
 // tested as soon as the node is intersected (after Ylitie et al., HPG 2017).
 #pragma once
@@ -109,89 +109,56 @@ __device__ __forceinline__ float wt_intersect(const float4 w0, const float4 w1, 
     return t;
 }
 
-// Out-of-line entry to the watertight test (shear set up per call), so the
-// default reference-exact path keeps its registers.
-static __device__ __noinline__ float wt_intersect_ray(const float4 w0, const float4 w1, const float4 w2, const float3 o,
-                                               const float3 d, float *u_out, float *v_out)
-{
-    const Shear sh = make_shear(d);
-    float u = 0.f, v = 0.f;
-    const float t = wt_intersect(w0, w1, w2, o, sh, u, v);
-    *u_out = u;
-    *v_out = v;
-    return t;
-}
-
-// Child-box test of one wide node: returns internal-hit bits (24..31,
-// permuted by octant) | imask (0..7) in .y with child_base in .x, and the
-// triangle-hit bits (0..23) with tri_base in tgroup.
+// Child-box test of one wide node: internal-hit bits (24..31, in the ray's
+// order, nearest highest) | imask (0..7) in ngroup.y with child_base in
+// ngroup.x; the hit leaf slots as an 8-bit mask (slot order) with the node's
+// triangle base and meta bytes.
 struct NodeHits {
     uint2 ngroup;
-    uint2 tgroup;
+    uint32_t leaf_slots;
+    uint32_t tri_base, meta_lo, meta_hi;
 };
 
-__device__ __forceinline__ uint32_t byte_of(uint32_t lo, uint32_t hi, int s)
+// Signed byte weights -(1 << s) of slots s = 0..3 and 4..7: the dot product
+// of a byte mask (0xff = -1 per marked slot) with them is the slots' bit mask.
+constexpr uint32_t kSlotWeightsLo = 0xF8FCFEFFu, kSlotWeightsHi = 0x80C0E0F0u;
+
+// Highest set bit (one instruction; the lowest would take a bit reversal too).
+__device__ __forceinline__ uint32_t top_bit(uint32_t v) { return 31u - (uint32_t)__clz((int)v); }
+
+// prmt with its sign-replicate selectors (bit 3 of a nibble), which
+// __byte_perm does not promise.
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel)
 {
-    return ((s < 4) ? (lo >> (8 * s)) : (hi >> (8 * (s - 4)))) & 0xffu;
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
 }
 
-// Quantised byte s of a 64-bit plane as a float.  RT_NODE_PRMT: one byte
-// permute places q in mantissa bits 8..15 of 1.0f, giving exactly
-// 1 + q * 2^-15; intersect_node folds the constant 1 into the node's offset
-// (kQOne below), so a plane costs one permute and one FMA.  Otherwise q
-// itself.
-#ifndef RT_NODE_PRMT
-#define RT_NODE_PRMT 1
-#endif
-#if RT_NODE_PRMT
-constexpr float kQScale = 32768.0f;   // 2^15: one quantisation step per 2^-15
-constexpr float kQOne = 1.0f;         // the byte's value at q = 0
-#else
-constexpr float kQScale = 1.0f;
-constexpr float kQOne = 0.0f;
-#endif
-__device__ __forceinline__ float qbyte(uint32_t lo, uint32_t hi, int s)
+// Byte masks (0xff: sign bit set) of four floats.
+__device__ __forceinline__ uint32_t sign_bytes(float a, float b, float c, float d)
 {
-#if RT_NODE_PRMT
-    const uint32_t w = (s < 4) ? lo : hi;
-    return __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | ((uint32_t)(s & 3) << 4)));
-#else
-    return (float)byte_of(lo, hi, s);
-#endif
+    const uint32_t lo = prmt(__float_as_uint(a), __float_as_uint(b), 0x00FBu);
+    const uint32_t hi = prmt(__float_as_uint(c), __float_as_uint(d), 0xFB00u);
+    return prmt(lo, hi, 0x7610u);
 }
 
-// max / min of three floats (one instruction with RT_NODE_MINMAX3).
-#ifndef RT_NODE_MINMAX3
-#define RT_NODE_MINMAX3 1
-#endif
+// max / min of three floats (one instruction).
 __device__ __forceinline__ float fmax3f(float a, float b, float c)
 {
-#if RT_NODE_MINMAX3
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
-#else
-    return fmaxf(fmaxf(a, b), c);
-#endif
 }
 __device__ __forceinline__ float fmin3f(float a, float b, float c)
 {
-#if RT_NODE_MINMAX3
     float d;
     asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
-#else
-    return fminf(fminf(a, b), c);
-#endif
 }
 
-// Packed single-precision FMA (fma.rn.f32x2, sm_100 family): two plane
-// distances per instruction, each half rounded exactly as fmaf, so the
-// child-box test and the frames are the same either way (measured faster:
-// terrain frame -0.9 %, AO-instances frame -4.7 %).
-#ifndef RT_NODE_FMA2
-#define RT_NODE_FMA2 1
-#endif
+// Packed single-precision arithmetic (sm_100 family): each half rounded
+// exactly as its scalar counterpart.
 __device__ __forceinline__ uint64_t pack2f(float a, float b)
 {
     uint64_t r;
@@ -206,9 +173,60 @@ __device__ __forceinline__ float2 fma2f(float a0, float a1, uint64_t b, uint64_t
     asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(d));
     return r;
 }
+__device__ __forceinline__ float2 sub2f(float a0, float a1, float b0, float b1)
+{
+    uint64_t d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pack2f(a0, a1)), "l"(pack2f(b0, b1)));
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(d));
+    return r;
+}
 
+// One axis of a wide node for one ray.  A plane byte q becomes the float
+// 1 + q * 2^-16 (kQWeight * q added to the bits of 1.0f by one byte dot
+// product, whose weight picks the byte), so that plane distances are
+// t = (1 + q * 2^-16) * scale + offset with scale = 2^16 * step / d and
+// offset = (origin - o) / d - scale.  The offset rounds at the magnitude of
+// 2^16 steps: an error below 2^-7 of one step, far inside the one-step
+// padding of every box.
+constexpr float kQScale = 65536.0f;
+constexpr uint32_t kQWeight = 0x80u;
+struct AxisPlanes {
+    uint64_t scale, offset;   // the same value in both halves
+    uint32_t near_w;          // weights that pick an even slot's entry plane: byte 0 (d >= 0) or 1
+};
+__device__ __forceinline__ AxisPlanes axis_planes(uint32_t e, float p, float o, float inv)
+{
+    const float s = __uint_as_float(e << 23) * inv * kQScale;
+    const float off = (p - o) * inv - s;
+    AxisPlanes A;
+    A.scale = pack2f(s, s);
+    A.offset = pack2f(off, off);
+    A.near_w = kQWeight << (8 * (__float_as_uint(inv) >> 31));
+    return A;
+}
+
+// Plane distances of two neighbouring slots (w: low, high, low, high).
+__device__ __forceinline__ float2 plane_pair(uint32_t w, uint32_t weights, const AxisPlanes &A)
+{
+    const uint32_t one = 0x3F800000u;
+    const uint32_t a = __dp4a(w, weights, one), b = __dp4a(w, weights << 16, one);
+    return fma2f(__uint_as_float(a), __uint_as_float(b), A.scale, A.offset);
+}
+
+// What bounds it: the two half-rate arithmetic pipes (a node test alone runs
+// no faster beyond two warps per scheduler).  Byte dot products run on the
+// multiply pipe and byte permutes, selects, min/max and compares on the
+// other, so the plane bytes go through __dp4a -- which also picks the entry
+// or exit plane by its weights, where separate planes needed 12 selects --
+// and the hit masks are formed from sign bits by permutes and dot products
+// instead of a compare and three bit operations per slot.  Cycles per node and
+// scheduler: 246; 286 with permutes and selects, 257 with permutes alone.
+// Together with the watertight test in kernels of its own: 2M any-hit rays
+// 718 -> 631 us, 1080p terrain frame 759 -> 695 us, AO-instances frame 4.10 ->
+// 3.76 ms, glass trees 713 -> 642 us.
 __device__ __forceinline__ NodeHits intersect_node(const WideNode *__restrict__ nodes, uint32_t idx, const float3 o,
-                                                   const float3 inv, uint32_t oct, float tmax)
+                                                   const float3 inv, uint32_t w0, uint32_t w1, float tmax)
 {
     const float4 *np = reinterpret_cast<const float4 *>(nodes + idx);
     const float4 n0 = __ldg(np + 0);
@@ -217,69 +235,55 @@ __device__ __forceinline__ NodeHits intersect_node(const WideNode *__restrict__ 
     const float4 n3 = __ldg(np + 3);
     const float4 n4 = __ldg(np + 4);
     const uint32_t e_imask = __float_as_uint(n0.w);
-    const uint32_t ex = e_imask & 0xffu, ey = (e_imask >> 8) & 0xffu, ez = (e_imask >> 16) & 0xffu;
-    const uint32_t imask = e_imask >> 24;
-    // plane t = q * step + (origin - o) * inv, evaluated as
-    // qbyte * (step * kQScale) + ((origin - o) * inv - kQOne * step * kQScale):
-    // the folded offset rounds at the magnitude of 2^15 steps, an error below
-    // 2^-9 of one step, far inside the one-step padding of every box
-    const float ux = __uint_as_float(ex << 23) * inv.x;
-    const float uy = __uint_as_float(ey << 23) * inv.y;
-    const float uz = __uint_as_float(ez << 23) * inv.z;
-    const float sx = ux * kQScale, sy = uy * kQScale, sz = uz * kQScale;
-    const float ox = fmaf(-kQOne, sx, (n0.x - o.x) * inv.x);
-    const float oy = fmaf(-kQOne, sy, (n0.y - o.y) * inv.y);
-    const float oz = fmaf(-kQOne, sz, (n0.z - o.z) * inv.z);
     const uint32_t meta_lo = __float_as_uint(n1.z), meta_hi = __float_as_uint(n1.w);
-    // lo/hi byte planes; swap per axis so "near" is the entry plane
-    uint32_t nxl = __float_as_uint(n2.x), nxh = __float_as_uint(n2.y);   // qlo_x
-    uint32_t nyl = __float_as_uint(n2.z), nyh = __float_as_uint(n2.w);   // qlo_y
-    uint32_t nzl = __float_as_uint(n3.x), nzh = __float_as_uint(n3.y);   // qlo_z
-    uint32_t fxl = __float_as_uint(n3.z), fxh = __float_as_uint(n3.w);   // qhi_x
-    uint32_t fyl = __float_as_uint(n4.x), fyh = __float_as_uint(n4.y);   // qhi_y
-    uint32_t fzl = __float_as_uint(n4.z), fzh = __float_as_uint(n4.w);   // qhi_z
-    if (inv.x < 0.f) { uint32_t t = nxl; nxl = fxl; fxl = t; t = nxh; nxh = fxh; fxh = t; }
-    if (inv.y < 0.f) { uint32_t t = nyl; nyl = fyl; fyl = t; t = nyh; nyh = fyh; fyh = t; }
-    if (inv.z < 0.f) { uint32_t t = nzl; nzl = fzl; fzl = t; t = nzh; nzh = fzh; fzh = t; }
-    uint32_t hits_int = 0, hits_tri = 0;
-    // slot s with its six plane distances: internal children set bit
-    // 24 + (s ^ oct), leaf slots their triangle bits.  An empty slot needs
-    // no test of its meta byte: its box is inverted (low planes 255, high
-    // planes 0), and should rounding let it "hit", its clear internal bit
-    // and meta byte 0 add nothing.
-    auto slot = [&](int s, float tnx, float tny, float tnz, float tfx, float tfy, float tfz) {
-        const uint32_t meta = byte_of(meta_lo, meta_hi, s);
-        const float tn = fmax3f(tnx, tny, fmaxf(tnz, 0.0f));
-        const float tf = fmin3f(tfx, tfy, fminf(tfz, tmax));
-        if (tn <= tf) {
-            if ((imask >> s) & 1u) hits_int |= 1u << (24 + (s ^ oct));
-            else hits_tri |= (meta >> 5) << (meta & 31u);
-        }
-    };
-#if RT_NODE_FMA2
-    const uint64_t SX = pack2f(sx, sx), SY = pack2f(sy, sy), SZ = pack2f(sz, sz);
-    const uint64_t OX = pack2f(ox, ox), OY = pack2f(oy, oy), OZ = pack2f(oz, oz);
+    const AxisPlanes X = axis_planes(e_imask & 0xffu, n0.x, o.x, inv.x);
+    const AxisPlanes Y = axis_planes((e_imask >> 8) & 0xffu, n0.y, o.y, inv.y);
+    const AxisPlanes Z = axis_planes((e_imask >> 16) & 0xffu, n0.z, o.z, inv.z);
+    const uint32_t far_w = kQWeight | (kQWeight << 8);   // near_w ^ far_w: the exit plane's weights
+    const uint32_t wx[4] = {__float_as_uint(n2.x), __float_as_uint(n2.y), __float_as_uint(n2.z), __float_as_uint(n2.w)};
+    const uint32_t wy[4] = {__float_as_uint(n3.x), __float_as_uint(n3.y), __float_as_uint(n3.z), __float_as_uint(n3.w)};
+    const uint32_t wz[4] = {__float_as_uint(n4.x), __float_as_uint(n4.y), __float_as_uint(n4.z), __float_as_uint(n4.w)};
+    float m[8];
 #pragma unroll
-    for (int s = 0; s < 8; s += 2) {
-        const float2 tnx = fma2f(qbyte(nxl, nxh, s), qbyte(nxl, nxh, s + 1), SX, OX);
-        const float2 tny = fma2f(qbyte(nyl, nyh, s), qbyte(nyl, nyh, s + 1), SY, OY);
-        const float2 tnz = fma2f(qbyte(nzl, nzh, s), qbyte(nzl, nzh, s + 1), SZ, OZ);
-        const float2 tfx = fma2f(qbyte(fxl, fxh, s), qbyte(fxl, fxh, s + 1), SX, OX);
-        const float2 tfy = fma2f(qbyte(fyl, fyh, s), qbyte(fyl, fyh, s + 1), SY, OY);
-        const float2 tfz = fma2f(qbyte(fzl, fzh, s), qbyte(fzl, fzh, s + 1), SZ, OZ);
-        slot(s, tnx.x, tny.x, tnz.x, tfx.x, tfy.x, tfz.x);
-        slot(s + 1, tnx.y, tny.y, tnz.y, tfx.y, tfy.y, tfz.y);
+    for (int p = 0; p < 4; ++p) {
+        const float2 nx = plane_pair(wx[p], X.near_w, X), fx = plane_pair(wx[p], X.near_w ^ far_w, X);
+        const float2 ny = plane_pair(wy[p], Y.near_w, Y), fy = plane_pair(wy[p], Y.near_w ^ far_w, Y);
+        const float2 nz = plane_pair(wz[p], Z.near_w, Z), fz = plane_pair(wz[p], Z.near_w ^ far_w, Z);
+        // the box is hit when max(near, 0) <= min(far, tmax): no sign bit in
+        // the difference (a NaN, from an overflowing scale, counts as a hit)
+        const float2 d = sub2f(fmin3f(fx.x, fy.x, fminf(fz.x, tmax)), fmin3f(fx.y, fy.y, fminf(fz.y, tmax)),
+                               fmax3f(nx.x, ny.x, fmaxf(nz.x, 0.0f)), fmax3f(nx.y, ny.y, fmaxf(nz.y, 0.0f)));
+        m[2 * p] = d.x;
+        m[2 * p + 1] = d.y;
     }
-#else
-#pragma unroll
-    for (int s = 0; s < 8; ++s)
-        slot(s, fmaf(qbyte(nxl, nxh, s), sx, ox), fmaf(qbyte(nyl, nyh, s), sy, oy), fmaf(qbyte(nzl, nzh, s), sz, oz),
-             fmaf(qbyte(fxl, fxh, s), sx, ox), fmaf(qbyte(fyl, fyh, s), sy, oy), fmaf(qbyte(fzl, fzh, s), sz, oz));
-#endif
+    // an empty slot needs no test of its own: its box is inverted, and should
+    // rounding let it "hit", it has no internal bit and no triangles
+    const uint32_t miss_lo = sign_bytes(m[0], m[1], m[2], m[3]), miss_hi = sign_bytes(m[4], m[5], m[6], m[7]);
+    const uint32_t int_lo = prmt(meta_lo, 0u, 0xBA98u), int_hi = prmt(meta_hi, 0u, 0xBA98u);   // sign bits of the meta bytes
+    const int hits_int = __dp4a((int)(~miss_lo & int_lo), (int)w0, __dp4a((int)(~miss_hi & int_hi), (int)w1, 0));
+    const int hits_leaf = __dp4a((int)~(miss_lo | int_lo), (int)kSlotWeightsLo,
+                                 __dp4a((int)~(miss_hi | int_hi), (int)kSlotWeightsHi, 0));
     NodeHits h;
-    h.ngroup = make_uint2(__float_as_uint(n1.x), hits_int | imask);
-    h.tgroup = make_uint2(__float_as_uint(n1.y), hits_tri);
+    // byte 3: the internal hits, byte 0: imask (bits 8..23 are not looked at)
+    h.ngroup = make_uint2(__float_as_uint(n1.x), prmt((uint32_t)hits_int, e_imask, 0x0447u));
+    h.leaf_slots = (uint32_t)hits_leaf;
+    h.tri_base = __float_as_uint(n1.y);
+    h.meta_lo = meta_lo;
+    h.meta_hi = meta_hi;
     return h;
+}
+
+// The triangles of a node's hit leaf slots as bits from its triangle base.
+__device__ __forceinline__ uint32_t leaf_triangles(const NodeHits &h)
+{
+    uint32_t bits = 0u;
+    for (uint32_t ls = h.leaf_slots; ls != 0u;) {
+        const uint32_t s = __ffs(ls) - 1u;
+        ls &= ls - 1u;
+        const uint32_t m = prmt(h.meta_lo, h.meta_hi, s) & 0xffu;
+        bits |= ((1u << (m >> 5)) - 1u) << (m & 31u);
+    }
+    return bits;
 }
 
 __device__ __forceinline__ float3 safe_inv(float3 d)
@@ -296,6 +300,15 @@ __device__ __forceinline__ uint32_t octant_of(float3 d)
     return (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
 }
 
+// kSlotWeights with the slots permuted by `order`: bit s ^ order for slot s.
+__device__ __forceinline__ void order_weights(uint32_t order, uint32_t &w0, uint32_t &w1)
+{
+    const uint32_t sel = 0x3210u ^ (0x1111u * (order & 3u));
+    const uint32_t lo = prmt(kSlotWeightsLo, 0u, sel), hi = prmt(kSlotWeightsHi, 0u, sel);
+    w0 = (order & 4u) ? hi : lo;
+    w1 = (order & 4u) ? lo : hi;
+}
+
 struct HitRecord {
     int32_t id;
     float t, u, v;
@@ -310,7 +323,8 @@ struct FetchCount {
 // that node's leaf triangles.  The stack lives with the caller.
 struct Trav {
     float3 o, d, inv;
-    uint32_t oct;
+    uint32_t order;    // octant ^ 7: slot s has bit 24 + (s ^ order), nearest highest
+    uint32_t w0, w1;   // order_weights
     float tmax;        // any-hit limit
     float box_tmax;    // boxes beyond this are culled (closest: best t so far)
     uint2 ngroup;
@@ -326,11 +340,12 @@ __device__ __forceinline__ void trav_begin(Trav &T, const SceneView &sc, const f
     T.o = o;
     T.d = d;
     T.inv = safe_inv(d);
-    T.oct = octant_of(d);
+    T.order = octant_of(d) ^ 7u;
+    order_weights(T.order, T.w0, T.w1);
     T.tmax = tmax;
     T.box_tmax = any ? tmax : FLT_MAX;
     // a group holding only the root (as slot 0 of a virtual parent)
-    T.ngroup = make_uint2((uint32_t)sc.root, sc.nnodes > 0 ? ((1u << (24 + T.oct)) | 1u) : 0u);
+    T.ngroup = make_uint2((uint32_t)sc.root, sc.nnodes > 0 ? ((1u << (24 + T.order)) | 1u) : 0u);
     T.sp = 0;
     T.steps = 0;
     T.hit.id = -1;
@@ -342,44 +357,45 @@ __device__ __forceinline__ void trav_begin(Trav &T, const SceneView &sc, const f
 
 // One traversal step; returns true when the ray is finished.  Closest hit
 // (any = false) or any hit inside (EPSILON, tmax) skipping light and
-// transparent triangles (any = true).  Status bits go to `status`.  STACK:
-// the stack's capacity in node groups (a ray holds at most one group per
-// tree level, so any capacity above the tree's depth suffices).
-template <bool COUNT, int STACK = kStackSize>
+// transparent triangles (any = true).  WT: the watertight triangle test.
+// Status bits go to `status`.  STACK: the stack's capacity in node groups (a
+// ray holds at most one group per tree level, so any capacity above the
+// tree's depth suffices).
+template <bool COUNT, bool WT, int STACK = kStackSize>
 __device__ __forceinline__ bool trav_step(Trav &T, uint2 *stack, const SceneView &sc, bool any, uint32_t &status,
                                           FetchCount *fc)
 {
     if (++T.steps > kMaxTraversalSteps) { status |= kStatusStepLimit; return true; }
-    uint2 tgroup = make_uint2(0u, 0u);
+    uint32_t tri_base = 0u, tri_bits = 0u;
     if (T.ngroup.y & 0xff000000u) {
-        const uint32_t bit = __ffs(T.ngroup.y >> 24) - 1u;
-        T.ngroup.y &= ~(1u << (24 + bit));
-        const uint32_t slot = bit ^ T.oct;
-        const uint32_t idx = T.ngroup.x + __popc(T.ngroup.y & ((1u << slot) - 1u) & 0xffu);
+        const uint32_t bit = top_bit(T.ngroup.y);
+        T.ngroup.y ^= 1u << bit;
+        const uint32_t slot = (bit ^ T.order) & 7u;
+        const uint32_t idx = T.ngroup.x + __popc(T.ngroup.y & ((1u << slot) - 1u));
         if (idx >= (uint32_t)sc.nnodes) { status |= kStatusBadIndex; return true; }
         if (T.ngroup.y & 0xff000000u) {
             if (T.sp >= STACK) { status |= kStatusStackOverflow; return true; }
             stack[T.sp++] = T.ngroup;
         }
-        const NodeHits nh = intersect_node(sc.nodes, idx, T.o, T.inv, T.oct, T.box_tmax);
+        const NodeHits nh = intersect_node(sc.nodes, idx, T.o, T.inv, T.w0, T.w1, T.box_tmax);
         if (COUNT) ++fc->nodes;
         T.ngroup = nh.ngroup;
-        tgroup = nh.tgroup;
+        tri_base = nh.tri_base;
+        tri_bits = leaf_triangles(nh);
     }
-    const bool watertight = sc.isect == RT_ISECT_WATERTIGHT;
-    while (tgroup.y != 0u) {
-        const uint32_t k = __ffs(tgroup.y) - 1u;
-        tgroup.y &= tgroup.y - 1u;
-        const uint32_t ti = tgroup.x + k;
+    while (tri_bits != 0u) {
+        const uint32_t k = __ffs(tri_bits) - 1u;
+        tri_bits &= tri_bits - 1u;
+        const uint32_t ti = tri_base + k;
         if (ti >= (uint32_t)sc.ntris) { status |= kStatusBadIndex; continue; }
         const PackedTri *tp = sc.tris + ti;
         if (COUNT) ++fc->tris;
         const float4 w0 = __ldg(&tp->w0);
         const float4 w1 = __ldg(&tp->w1);
         const float4 w2 = __ldg(&tp->w2);
-        float u, v;
-        const float t = watertight ? wt_intersect_ray(w0, w1, w2, T.o, T.d, &u, &v)
-                                   : mt_intersect(w0, w1, w2, T.o, T.d, u, v);
+        float u = 0.f, v = 0.f;
+        const float t = WT ? wt_intersect(w0, w1, w2, T.o, make_shear(T.d), u, v)
+                           : mt_intersect(w0, w1, w2, T.o, T.d, u, v);
         const int32_t id = __float_as_int(w2.y);
         if ((uint32_t)id >= (uint32_t)sc.ntris) { status |= kStatusBadIndex; continue; }
         if (any) {
@@ -404,20 +420,28 @@ __device__ __forceinline__ bool trav_step(Trav &T, uint2 *stack, const SceneView
     return false;
 }
 
-// Whole traversal of one ray.  Returns the device status bits.
-template <bool ANY, bool COUNT = false, int STACK = kStackSize>
-__device__ __forceinline__ uint32_t traverse(const SceneView &sc, const float3 o, const float3 d, float tmax,
-                                             HitRecord &hit, bool &occluded, FetchCount *fc = nullptr)
+// Whole traversal of one ray, closest or any hit.  Returns the device status
+// bits.
+template <bool COUNT, int STACK = kStackSize, class SC>
+__device__ __forceinline__ uint32_t traverse_ray(const SC &sc, const float3 o, const float3 d, float tmax, bool any,
+                                                 HitRecord &hit, bool &occluded, FetchCount *fc = nullptr)
 {
     uint2 stack[STACK];
     Trav T;
-    trav_begin(T, sc, o, d, tmax, ANY);
+    trav_begin(T, sc, o, d, tmax, any);
     uint32_t status = 0u;
-    while (!trav_step<COUNT, STACK>(T, stack, sc, ANY, status, fc)) {
+    while (!trav_step<COUNT, SC::kWatertight, STACK>(T, stack, sc, any, status, fc)) {
     }
     hit = T.hit;
     occluded = T.occluded;
     return status;
+}
+
+template <bool ANY, bool COUNT = false, int STACK = kStackSize, class SC>
+__device__ __forceinline__ uint32_t traverse(const SC &sc, const float3 o, const float3 d, float tmax, HitRecord &hit,
+                                             bool &occluded, FetchCount *fc = nullptr)
+{
+    return traverse_ray<COUNT, STACK>(sc, o, d, tmax, ANY, hit, occluded, fc);
 }
 
 // ------------------------------------------------------------ shading

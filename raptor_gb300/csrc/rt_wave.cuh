@@ -46,7 +46,7 @@ enum : int { kLaneIdle = 0, kLaneTraverse = 1, kLaneFinished = 2 };
 
 // Jobs: `single` (nullable) is the one job of a single-frame launch; else
 // the table `jobs` of njobs entries is searched by item.
-template <int TW, bool COUNT>
+template <int TW, bool COUNT, bool WT>
 __device__ __forceinline__ void wave_loop(const FrameJob *single, const FrameJob *__restrict__ jobs, int32_t njobs,
                                           int32_t total_items, LaneShade &S, Counters *ctr)
 {
@@ -183,7 +183,7 @@ __device__ __forceinline__ void wave_loop(const FrameJob *single, const FrameJob
         // ---- one traversal step of every traversing lane
         if (state == kLaneTraverse) {
             const FrameJob &J = single ? *single : jobs[j];
-            if (trav_step<COUNT>(T, stack, J.sc, phase > 0, status, &fc)) state = kLaneFinished;
+            if (trav_step<COUNT, WT>(T, stack, J.sc, phase > 0, status, &fc)) state = kLaneFinished;
         }
     }
     warp_add(&ctr->primary, n_primary);
