@@ -963,7 +963,7 @@ rt_status rt_sum_sequential_f32(rt_context *ctx, const float *values, int64_t n,
     const void *dv = nullptr;
     rt_status st = stage_in(ctx, ctx->stage_a, values, (size_t)n * sizeof(float), &dv);
     if (st != RT_OK) return st;
-    RT_CUDA(ctx->tone.reserve(kToneScratch + tone_scratch_bytes(n)), "scratch allocation");
+    RT_CUDA(ctx->tone.reserve(kToneScratch + sum_scratch_bytes(n)), "scratch allocation");
     ToneAcc *acc = (ToneAcc *)ctx->tone.ptr;
     uint32_t *mx = (uint32_t *)((char *)ctx->tone.ptr + kToneWord);
     launch_abs_max((const float *)dv, n, mx, ctx->sm_count, ctx->stream);

@@ -103,6 +103,8 @@ void launch_abs_max(const float *v, int64_t n, uint32_t *out, int sm_count, cuda
 void launch_check_log10(int64_t n, uint64_t seed, unsigned long long *out, int sm_count, cudaStream_t st);
 void launch_sequential_sum(const float *v, int64_t n, float max_abs, ToneAcc *acc, void *scratch, int sm_count,
                            cudaStream_t st);
+// Device scratch of launch_sequential_sum over n values.
+size_t sum_scratch_bytes(int64_t n);
 // scratch: tone_scratch_bytes(fw * fh, blocks) of device memory (blocks:
 // hist_sx * hist_sy of a histogram mode, else 0).
 size_t tone_scratch_bytes(int64_t n, int64_t blocks = 0);

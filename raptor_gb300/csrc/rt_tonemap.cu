@@ -901,30 +901,57 @@ __global__ void __launch_bounds__(kToneThreads) k_tone_range(const float *__rest
     }
 }
 
+__device__ __forceinline__ bool same_bits(float3 a, float3 b)
+{
+    return ((__float_as_uint(a.x) ^ __float_as_uint(b.x)) | (__float_as_uint(a.y) ^ __float_as_uint(b.y)) |
+            (__float_as_uint(a.z) ^ __float_as_uint(b.z))) == 0u;
+}
+
+// One sample (index s, value c) through the chain.
+template <bool EXACT>
+__device__ __forceinline__ float3 tone_sample(float3 c, int64_t s, const ToneView &t, const ToneScalars &k,
+                                              const ToneHist &hh, bool stretch, float offset, float scale,
+                                              bool *inexact = nullptr)
+{
+    if (!t.enabled) return c;
+    const Yxy p = to_yxy<EXACT>(c, t);
+    float g = t.mode == RT_TONE_GLOBAL_BILATERAL ? t.bil[s] : map_lum<EXACT>(p.Y, t, k, hh);
+    if (stretch) g = xmul(xadd(g, offset), scale);
+    return to_rgb<EXACT>(p.x, g, p.y, t.gamma, inexact);
+}
+
 // One output pixel: each of its aa_x * aa_y samples through the chain, then
-// clip_image_to_rgb's sum (a_x outer, a_y inner) and division.  inexact
-// (nullable) is set when a single-precision library call took part: every
-// mode's luminance map but the bilateral one (precomputed exactly), or a
-// gamma power inside (0, 1).
+// clip_image_to_rgb's sum (a_x outer, a_y inner) and division.  A sample
+// equal to the one before it (sky, flat colour) takes that one's result.
+// inexact (nullable) is set when a single-precision library call took part:
+// every mode's luminance map but the bilateral one (precomputed exactly), or a
+// gamma power inside (0, 1).  flat (nullable): all samples equal, their value
+// in `value`, so that the pixel's colour depends on that value alone.
 template <bool EXACT>
 __device__ __forceinline__ float3 tone_pixel(const float *__restrict__ fimg, int32_t fw, int32_t aa_x, int32_t aa_y,
                                              int32_t ox, int32_t oy, const ToneView &t, const ToneScalars &k,
                                              const ToneHist &hh, bool stretch, float offset, float scale,
-                                             float samples, bool *inexact = nullptr)
+                                             float samples, bool *inexact = nullptr, bool *flat = nullptr,
+                                             float3 *value = nullptr)
 {
-    if (inexact) *inexact = t.enabled && t.mode != RT_TONE_GLOBAL_BILATERAL;
+    const bool bilateral = t.mode == RT_TONE_GLOBAL_BILATERAL;   // its map depends on the sample's place
+    if (inexact) *inexact = t.enabled && !bilateral;
+    if (flat) *flat = !bilateral;
     float3 a = make_float3(0.0f, 0.0f, 0.0f);
+    float3 from = a, to = a;
+    bool first = true;
     for (int32_t ax = 0; ax < aa_x; ++ax)
         for (int32_t ay = 0; ay < aa_y; ++ay) {
             const int64_t s = (int64_t)(ox * aa_x + ax) + (int64_t)(oy * aa_y + ay) * fw;
-            float3 c = make_float3(fimg[3 * s], fimg[3 * s + 1], fimg[3 * s + 2]);
-            if (t.enabled) {
-                const Yxy p = to_yxy<EXACT>(c, t);
-                float g = (t.mode == RT_TONE_GLOBAL_BILATERAL) ? t.bil[s] : map_lum<EXACT>(p.Y, t, k, hh);
-                if (stretch) g = xmul(xadd(g, offset), scale);
-                c = to_rgb<EXACT>(p.x, g, p.y, t.gamma, inexact);
+            const float3 c = make_float3(fimg[3 * s], fimg[3 * s + 1], fimg[3 * s + 2]);
+            if (first || bilateral || !same_bits(c, from)) {
+                if (flat && !first) *flat = false;
+                if (value && first) *value = c;
+                first = false;
+                from = c;
+                to = tone_sample<EXACT>(c, s, t, k, hh, stretch, offset, scale, inexact);
             }
-            a = xadd3(a, c);
+            a = xadd3(a, to);
         }
     return make_float3(xdiv(a.x, samples), xdiv(a.y, samples), xdiv(a.z, samples));
 }
@@ -967,10 +994,13 @@ __device__ __forceinline__ void store_pixel(uint8_t *rgb, int64_t o, float3 v)
 // Per output pixel: tone_pixel with the single-precision library calls; a
 // pixel with a channel near a truncation boundary is queued for k_tone_fix
 // instead (warp-aggregated append), then the clamp and truncation of
-// clip_image_to_rgb.
+// clip_image_to_rgb.  A queue entry is (pixel of lane 0, lanes): pixels of a
+// warp whose samples all have one value share an entry, so a sky whose colour
+// lands near a boundary is redone once per 32 pixels, not once per pixel.
+// (1283x717 terrain, 2x2 samples, such a sky: k_tone_fix 1047 -> 108 us.)
 __global__ void __launch_bounds__(kToneThreads) k_tone_final(const float *__restrict__ fimg, int32_t fw, int32_t aa_x,
                                                              int32_t aa_y, int32_t ow, int32_t oh, ToneView t,
-                                                             ToneAcc *acc, int32_t *__restrict__ redo,
+                                                             ToneAcc *acc, int2 *__restrict__ redo,
                                                              uint8_t *__restrict__ rgb)
 {
     ToneScalars k = {};
@@ -981,42 +1011,79 @@ __global__ void __launch_bounds__(kToneThreads) k_tone_final(const float *__rest
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t start = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t steps = (npix + stride - 1) / stride;   // uniform trip count: whole warps append
+    const int lane = threadIdx.x & 31;
     for (int64_t it = 0; it < steps; ++it) {
         const int64_t o = start + it * stride;
-        bool queue = false;
+        bool queue = false, flat = false;
+        float3 value = make_float3(0.0f, 0.0f, 0.0f);
         if (o < npix) {
             const int32_t oy = (int32_t)(o / ow), ox = (int32_t)(o - (int64_t)oy * ow);
             bool inexact = false;
             const float3 v = tone_pixel<false>(fimg, fw, aa_x, aa_y, ox, oy, t, k, acc->h, sr.on, sr.offset, sr.scale,
-                                               samples, &inexact);
+                                               samples, &inexact, &flat, &value);
             queue = inexact && (near_integer(v.x) || near_integer(v.y) || near_integer(v.z));
             if (!queue) store_pixel(rgb, o, v);
         }
-        const uint32_t b = __ballot_sync(0xffffffffu, queue);
-        if (b) {
+        if (__any_sync(0xffffffffu, queue)) {
+            uint32_t lanes = 1u << lane;
+            const uint32_t fb = __ballot_sync(0xffffffffu, queue && flat);
+            if (queue && flat)
+                lanes = __match_any_sync(fb, __float_as_uint(value.x)) &
+                        __match_any_sync(fb, __float_as_uint(value.y)) & __match_any_sync(fb, __float_as_uint(value.z));
+            const bool leads = queue && __ffs(lanes) - 1 == lane;
+            const uint32_t lb = __ballot_sync(0xffffffffu, leads);
             int base = 0;
-            const int lane = threadIdx.x & 31;
-            if (lane == 0) base = atomicAdd(&acc->redo, __popc(b));
+            if (lane == 0) base = atomicAdd(&acc->redo, __popc(lb));
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (queue) redo[base + __popc(b & ((1u << lane) - 1u))] = (int32_t)o;
+            if (leads) redo[base + __popc(lb & ((1u << lane) - 1u))] = make_int2((int32_t)(o - lane), (int32_t)lanes);
         }
     }
 }
 
-// The queued pixels, with the library calls evaluated exactly.
+// The queued pixels, with the library calls evaluated exactly.  Bound by the
+// latency of the double-precision calls (a few per cent of the issue slots),
+// so up to 32 samples of a pixel are evaluated by as many lanes, and summed in
+// order by shuffles (1283x717, 2x2 samples: 108 -> 85 us).
 __global__ void __launch_bounds__(kToneThreads) k_tone_fix(const float *__restrict__ fimg, int32_t fw, int32_t aa_x,
                                                            int32_t aa_y, int32_t ow, ToneView t, const ToneAcc *acc,
-                                                           const int32_t *__restrict__ redo, uint8_t *__restrict__ rgb)
+                                                           const int2 *__restrict__ redo, uint8_t *__restrict__ rgb)
 {
     const ToneScalars k = acc->s;
     const Stretch sr = stretch_of(t, acc);
     const int n = acc->redo;
-    const float samples = (float)(aa_x * aa_y);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int64_t o = redo[i];
+    const int S = aa_x * aa_y;
+    const float samples = (float)S;
+    const int lane = threadIdx.x & 31;
+    const int per = S <= 32 ? 32 / S : 32;              // pixels a warp takes at a time
+    const int g = S <= 32 ? lane / S : lane;
+    const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), warps = (int)((gridDim.x * blockDim.x) >> 5);
+    for (int i0 = warp * per; i0 < n; i0 += warps * per) {
+        const bool live = g < per && i0 + g < n;
+        const int2 e = live ? redo[i0 + g] : make_int2(0, 1);
+        const int64_t o = e.x + (__ffs(e.y) - 1);
         const int32_t oy = (int32_t)(o / ow), ox = (int32_t)(o - (int64_t)oy * ow);
-        store_pixel(rgb, o,
-                    tone_pixel<true>(fimg, fw, aa_x, aa_y, ox, oy, t, k, acc->h, sr.on, sr.offset, sr.scale, samples));
+        float3 v = make_float3(0.0f, 0.0f, 0.0f);
+        if (S <= 32) {
+            const int smp = lane - g * S;               // x outer, y inner
+            if (live) {
+                const int64_t s = (int64_t)(ox * aa_x + smp / aa_y) + (int64_t)(oy * aa_y + smp % aa_y) * fw;
+                v = tone_sample<true>(make_float3(fimg[3 * s], fimg[3 * s + 1], fimg[3 * s + 2]), s, t, k, acc->h,
+                                      sr.on, sr.offset, sr.scale);
+            }
+            float3 a = make_float3(0.0f, 0.0f, 0.0f);
+            for (int j = 0; j < S; ++j) {
+                const int from = min(g * S + j, 31);
+                a = xadd3(a, make_float3(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from),
+                                         __shfl_sync(0xffffffffu, v.z, from)));
+            }
+            v = make_float3(xdiv(a.x, samples), xdiv(a.y, samples), xdiv(a.z, samples));
+            if (!live || smp != 0) continue;
+        } else {
+            if (!live) continue;
+            v = tone_pixel<true>(fimg, fw, aa_x, aa_y, ox, oy, t, k, acc->h, sr.on, sr.offset, sr.scale, samples);
+        }
+        for (uint32_t lanes = (uint32_t)e.y; lanes != 0u; lanes &= lanes - 1u)
+            store_pixel(rgb, e.x + (__ffs((int)lanes) - 1), v);
     }
 }
 
@@ -1322,12 +1389,17 @@ int blocks_for(int64_t n, int sm_count)
 
 }  // namespace
 
-size_t tone_scratch_bytes(int64_t n, int64_t blocks)
+size_t sum_scratch_bytes(int64_t n)
 {
     const int64_t nchunks = (n + kSumChunk - 1) / kSumChunk;
     const int64_t ncoarse = (nchunks + kCoarse - 1) / kCoarse;
-    return (size_t)nchunks * kSumChunk * sizeof(float) + (size_t)(nchunks + ncoarse) * 32 * sizeof(ChunkSum) +
-           (size_t)n * sizeof(int32_t) +   // redo queue (at most one entry per output pixel)
+    return (size_t)nchunks * kSumChunk * sizeof(float) + (size_t)(nchunks + ncoarse) * 32 * sizeof(ChunkSum);
+}
+
+size_t tone_scratch_bytes(int64_t n, int64_t blocks)
+{
+    return sum_scratch_bytes(n) +
+           (size_t)n * sizeof(int2) +      // redo queue (at most one entry per output pixel)
            (size_t)blocks * sizeof(float) +  // histogram modes: the per-degree luminance blocks
            (size_t)2 * 2 * 4096 * sizeof(float);   // and their bounds (at most 4096 per axis)
 }
@@ -1406,7 +1478,7 @@ void launch_tone_map(const float *fimg, int32_t fw, int32_t fh, int32_t aa_x, in
     float *terms = (float *)scratch;
     ChunkSum *rec = (ChunkSum *)(terms + nchunks * kSumChunk);
     ChunkSum *crec = rec + nchunks * 32;
-    int32_t *redo = (int32_t *)(crec + ncoarse * 32);
+    int2 *redo = (int2 *)(crec + ncoarse * 32);
     float *hblocks = (float *)(redo + n);
     cudaMemsetAsync(acc, 0, sizeof(ToneAcc), st);
     // the stretch range starts empty (k_tone_sum sets it too, for the other modes)
