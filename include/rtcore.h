@@ -510,7 +510,7 @@ typedef struct rt_light_shape {
  * rt_render_materials).  rgb_out (RGB8) and rgb_f32 (the camera's float
  * image) are nullable, not both, host or device memory.  Runs two passes
  * with one host round trip between them: the camera rays, then the frame's
- * slice of the random stream (generated on the host and copied over unless
+ * slice of the random stream (generated on the device unless
  * the previous frame's slice already covers it) and the shading. */
 rt_status rt_render_soft_shadows(rt_scene *scene, const rt_camera *camera, const rt_light *lights, int32_t nlights,
                                  const rt_light_shape *shapes, const rt_material *materials, int32_t nmaterials,
@@ -563,7 +563,7 @@ typedef struct rt_sampling {
  * added times rf, then tran.  Limits of rt_render_materials on the tree.
  * RT_STREAM_REFERENCE renders the reference's frame exactly (one counting
  * pass over the ray trees fixes every pixel's position in the stream; the
- * frame's slice is generated on the host), but not with diffuse rays,
+ * frame's slice is generated before it is shaded), but not with diffuse rays,
  * whose count depends on where earlier random rays of the frame landed:
  * replaying one stream through them is serial, so such frames need
  * RT_STREAM_PIXEL.  stream_end (nullable) receives, for

@@ -15,15 +15,15 @@
 // is therefore fixed by how many pixels before it hit something, so a frame
 // is rendered in two passes: the camera rays first (hit records kept, one
 // flag per pixel), an exclusive scan of the flags (each hit draws the same
-// count), the frame's slice of the stream generated on the host and copied
-// to the device, then the shading pass, every pixel reading its own slice.
+// count), the frame's slice of the stream generated on the device (k_ref_stream:
+// one block walks the generator's states in order), then the shading pass,
+// every pixel reading its own slice.
 // The cosine table the offsets go through (common/common.h:171-209) is
 // built on the host the same way and kept on the device.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
-#include <thread>
 #include <type_traits>
 #include <vector>
 
@@ -39,104 +39,95 @@ constexpr int kCosLutSize = 16384;                          // COS_LUT_SIZE, com
 
 namespace {
 
-// The reference's generator: a Mersenne twister seeded with 5489 whose
-// refill updates words 0..622 only, tempered and scaled to [0, 1] in
-// binary32.  pos counts the numbers produced since seeding.
-struct RefRandom {
-    uint32_t mt[624];
-    int idx = 624;
-    int64_t pos = 0;
+// The reference's generator: a Mersenne twister of kMtWords words seeded with
+// 5489 whose refill updates words 0..622 only, its words tempered and scaled
+// to [0, 1] in binary32.  Number p is word p % 624 of the state after refill
+// p / 624 (counted from 0), so the stream is kept as those states' words;
+// ref_number tempers one where it is read.
+constexpr int kMtWords = 624;
 
-    RefRandom() { reset(); }
-
-    void reset()
-    {
-        mt[0] = 5489u;
-        for (int i = 1; i < 624; ++i) mt[i] = 1812433253u * (mt[i - 1] ^ (mt[i - 1] >> 30)) + (uint32_t)i;
-        idx = 624;
-        pos = 0;
-    }
-
-    void refill()
-    {
-        for (int i = 0; i < 227; ++i) {
-            const uint32_t y = (0x80000000u & mt[i]) + (0x7FFFFFFFu & mt[i + 1]);
-            mt[i] = mt[i + 397] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
-        }
-        for (int i = 227; i < 623; ++i) {
-            const uint32_t y = (0x80000000u & mt[i]) + (0x7FFFFFFFu & mt[i + 1]);
-            mt[i] = mt[i - 227] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
-        }
-        idx = 0;
-    }
-
-    float next()
-    {
-        if (idx >= 624) refill();
-        uint32_t y = mt[idx++];
-        ++pos;
-        y ^= (y >> 11);
-        y ^= ((y << 7) & 0x9d2c5680u);
-        y ^= ((y << 15) & 0xefc60000u);
-        y ^= (y >> 18);
-        return (float)y * (1.0f / 4294967296.0f);
-    }
-
-    // Position the generator so that the next number is number p.
-    void seek(int64_t p)
-    {
-        if (p < pos) reset();
-        while (pos < p) {
-            if (idx >= 624 && p - pos >= 624) {   // skip whole blocks without tempering
-                refill();
-                idx = 624;
-                pos += 624;
-                continue;
-            }
-            (void)next();
-        }
-    }
-};
-
-// Numbers [offset, offset + total) of the stream into out.  The state only
-// changes at refills, so one pass walks the slice refill by refill
-// (without tempering) and keeps a copy of the generator at the start of
-// every chunk; host threads then temper their chunks in parallel.  The
-// generator is left at offset + total.
-void generate_slice(RefRandom &rng, int64_t offset, int64_t total, float *out)
+__device__ __forceinline__ float ref_number(uint32_t y)
 {
-    rng.seek(offset);
-    constexpr int64_t kChunk = 624 * 2048;
-    std::vector<RefRandom> starts;
-    std::vector<int64_t> begins;
-    for (int64_t b = 0; b < total; b += kChunk) {
-        starts.push_back(rng);
-        begins.push_back(b);
-        rng.seek(offset + std::min(total, b + kChunk));
+    y ^= (y >> 11);
+    y ^= ((y << 7) & 0x9d2c5680u);
+    y ^= ((y << 15) & 0xefc60000u);
+    y ^= (y >> 18);
+    return xmul(__uint2float_rn(y), 1.0f / 4294967296.0f);
+}
+
+__device__ __forceinline__ uint32_t mt_twist(uint32_t a, uint32_t b)
+{
+    const uint32_t y = (a & 0x80000000u) | (b & 0x7fffffffu);
+    return (y >> 1) ^ ((uint32_t)((int32_t)(b << 31) >> 31) & 0x9908b0dfu);
+}
+
+// `refills` refills of `state`, one after another; with OUT the words after
+// each go to out, else they are positions that are skipped.  A chain of
+// refills no two of which can overlap, so what counts is the latency of one.
+// A new word i needs old words i and i + 1 and word i + 397, which for
+// i >= 227 is the new word i - 227: thread t takes words t, t + 227 and
+// t + 454, so those chains stay inside a thread and a refill is one exchange
+// of the old words through shared memory (two buffers, one barrier).
+// Measured 106 ns a refill with output, 85 without (138 and 110 with
+// branches around the idle threads' work; 177 on four warps of two words per
+// third; a host core takes 350).
+constexpr int kMtThreads = 256;
+constexpr int kMtThird = kMtWords - 1 - 2 * 227;   // words 454..622
+constexpr int kMtBuffer = 1024;                    // idle threads read past the words
+template <bool OUT>
+__device__ __forceinline__ void mt_refill(uint32_t *w, int t, int t3, bool on, bool third, uint32_t &a, uint32_t &b,
+                                          uint32_t &c, uint32_t *dst)
+{
+    if (on) {
+        w[t] = a;
+        w[t + 227] = b;
     }
-    const int tasks = (int)starts.size();
-    const int nthreads = std::max(1, std::min<int>(tasks, (int)std::thread::hardware_concurrency()));
-    auto work = [&](int first) {
-        for (int t = first; t < tasks; t += nthreads) {
-            RefRandom g = starts[(size_t)t];
-            const int64_t end = std::min(total, begins[(size_t)t] + kChunk);
-            for (int64_t i = begins[(size_t)t]; i < end; ++i) out[i] = g.next();
+    if (third) w[t + 454] = c;
+    __syncthreads();
+    const uint32_t far = w[t + 397];
+    const uint32_t fa = mt_twist(a, w[t + 1]), fb = mt_twist(b, w[t + 228]), fc = mt_twist(c, w[t3 + 455]);
+    const uint32_t fbc = fb ^ fc;
+    a = far ^ fa;
+    b = far ^ fa ^ fb;
+    c = far ^ fa ^ fbc;
+    if (OUT) {
+        if (on) {
+            dst[t] = a;
+            dst[t + 227] = b;
         }
-    };
-    // worker k tempers chunks k, k + nthreads, ...; the workers whose thread
-    // could not be started run here, one after another, once the rest are done
-    std::vector<std::thread> pool;
-    int started = 1;
-    try {
-        for (int k = 1; k < nthreads; ++k) {
-            pool.emplace_back(work, k);
-            ++started;
-        }
-    } catch (...) {
+        if (third) dst[t + 454] = c;
     }
-    work(0);
-    for (std::thread &th : pool) th.join();
-    for (int k = started; k < nthreads; ++k) work(k);
+}
+
+template <bool OUT>
+__global__ void __launch_bounds__(kMtThreads) k_ref_stream(uint32_t *__restrict__ state, int32_t refills,
+                                                           uint32_t *__restrict__ out)
+{
+    extern __shared__ uint32_t mt_words[];   // two buffers (and what keeps other blocks off the SM)
+    const int t = threadIdx.x;
+    const bool on = t < 227, third = t < kMtThird;
+    const int t3 = third ? t : kMtThird - 1;
+    uint32_t a = state[on ? t : 0], b = state[on ? t + 227 : 0], c = state[t3 + 454];
+    const uint32_t last = state[kMtWords - 1];
+    for (int i = t; i < 2 * kMtBuffer; i += kMtThreads) mt_words[i] = 0u;
+    __syncthreads();
+    if (t < 2) mt_words[t * kMtBuffer + kMtWords - 1] = last;
+    uint32_t *dst = out;
+    int32_t r = 0;
+    for (; r + 1 < refills; r += 2) {
+        mt_refill<OUT>(mt_words, t, t3, on, third, a, b, c, dst);
+        if (OUT) dst += kMtWords;
+        mt_refill<OUT>(mt_words + kMtBuffer, t, t3, on, third, a, b, c, dst);
+        if (OUT) dst += kMtWords;
+    }
+    if (r < refills) mt_refill<OUT>(mt_words, t, t3, on, third, a, b, c, dst);
+    if (OUT)
+        for (int32_t i = t; i < refills; i += kMtThreads) out[(size_t)i * kMtWords + kMtWords - 1] = last;
+    if (on) {
+        state[t] = a;
+        state[t + 227] = b;
+    }
+    if (third) state[t + 454] = c;
 }
 
 // The rays light::find_rays makes for a triangle-defined light of ntris
@@ -171,7 +162,6 @@ struct SoftState {
     DevBuf hits;                 // int4 per pixel: the primary hit record
     DevBuf flags, prefix;        // int per pixel: hit flag, exclusive scan of the flags
     DevBuf scan_temp;
-    DevBuf window;               // numbers [win_base, win_base + win_len) of the stream
     DevBuf area;                 // int4 per ray of a triangle-defined light: triangle, its rays, index
     DevBuf counts, prefix64;     // int64 per pixel: numbers a distributed pixel draws, their exclusive scan
     DevBuf scan64_temp;
@@ -180,48 +170,53 @@ struct SoftState {
     // their subtrees' colours, the item count
     DevBuf root_c, root_sets, items, item_c, nitems;
     int64_t item_cap = 0;
-    int64_t win_base = -1, win_len = 0;
-    // Host side of the stream: staging holds numbers [stage_base, stage_base
-    // + stage_len) and rng stands at their end.  After each upload a thread
-    // reads ahead: it generates the numbers that follow the frame's slice
-    // (where the next frame starts, drawing about as many) while the GPU
-    // renders; the next window joins it first.
-    RefRandom rng;
-    float *staging = nullptr;    // pinned
-    size_t staging_cap = 0;
-    int64_t stage_base = -1, stage_len = 0;
-    std::thread ahead;
-    cudaEvent_t copied = nullptr;   // the last upload out of staging
+    // The stream's words on the device: two windows, one a frame reads from and
+    // one the generator reads ahead into on its own stream, while the frame
+    // renders, the words that follow the frame's slice (where the next frame of
+    // an animation starts, drawing about as many).  refills counts what the
+    // generator's state has behind it (-1: not seeded).
+    struct Window {
+        DevBuf words;
+        int64_t first = 0, count = 0;      // refills [first, first + count)
+        cudaEvent_t ready = nullptr;       // its words are written
+    } win[2];
+    int cur = 0;                           // the window the last frame read
+    DevBuf rng;                            // the generator's state, then the seeded one
+    int64_t refills = -1;
+    cudaStream_t gen = nullptr;
+    size_t gen_smem = 0;
+    cudaEvent_t used = nullptr;            // the last frame's reads of its window
     int device = 0;
 };
-
-// Waits for a read-ahead in flight.
-void join_ahead(SoftState &S)
-{
-    if (S.ahead.joinable()) S.ahead.join();
-}
 
 void soft_release(rt_context *ctx)
 {
     if (!ctx->soft) return;
-    join_ahead(*ctx->soft);
-    if (ctx->soft->copied) cudaEventDestroy(ctx->soft->copied);
-    ctx->soft->lut.release();
-    ctx->soft->hits.release();
-    ctx->soft->flags.release();
-    ctx->soft->prefix.release();
-    ctx->soft->scan_temp.release();
-    ctx->soft->window.release();
-    ctx->soft->area.release();
-    ctx->soft->counts.release();
-    ctx->soft->prefix64.release();
-    ctx->soft->scan64_temp.release();
-    ctx->soft->root_c.release();
-    ctx->soft->root_sets.release();
-    ctx->soft->items.release();
-    ctx->soft->item_c.release();
-    ctx->soft->nitems.release();
-    if (ctx->soft->staging) cudaFreeHost(ctx->soft->staging);
+    SoftState &S = *ctx->soft;
+    if (S.gen) {
+        cudaStreamSynchronize(S.gen);
+        cudaStreamDestroy(S.gen);
+    }
+    if (S.used) cudaEventDestroy(S.used);
+    for (SoftState::Window &w : S.win) {
+        if (w.ready) cudaEventDestroy(w.ready);
+        w.words.release();
+    }
+    S.rng.release();
+    S.lut.release();
+    S.hits.release();
+    S.flags.release();
+    S.prefix.release();
+    S.scan_temp.release();
+    S.area.release();
+    S.counts.release();
+    S.prefix64.release();
+    S.scan64_temp.release();
+    S.root_c.release();
+    S.root_sets.release();
+    S.items.release();
+    S.item_c.release();
+    S.nitems.release();
     delete ctx->soft;
     ctx->soft = nullptr;
 }
@@ -340,7 +335,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_pr
 template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_shade(
     SC sc, CameraView cam, LightSet lights, MaterialTable table, AreaSet areas, const int4 *__restrict__ area,
-    const float *__restrict__ verts, int32_t samples, int32_t per_hit, const float *__restrict__ rnd, int64_t nrnd,
+    const float *__restrict__ verts, int32_t samples, int32_t per_hit, const uint32_t *__restrict__ rnd, int64_t nrnd,
     const float *__restrict__ lut, const int4 *__restrict__ hits, const int32_t *__restrict__ prefix,
     uint8_t *__restrict__ rgb, float *__restrict__ fimg, Counters *ctr)
 {
@@ -392,12 +387,13 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_sh
                             float3 di;
                             float li;
                             if (tri_light) {
-                                const float *u = rnd + draw + 2 * i;
-                                area_ray(verts, sc.idx, __ldg(area + areas.first[l] + i), start, __ldg(u),
-                                         __ldg(u + 1), di, li);
+                                const uint32_t *u = rnd + draw + 2 * i;
+                                area_ray(verts, sc.idx, __ldg(area + areas.first[l] + i), start, ref_number(__ldg(u)),
+                                         ref_number(__ldg(u + 1)), di, li);
                             } else {
-                                const float *u = rnd + draw + 3 * i;
-                                soft_ray(L, lut, start, n, i, __ldg(u), __ldg(u + 1), __ldg(u + 2), di, li);
+                                const uint32_t *u = rnd + draw + 3 * i;
+                                soft_ray(L, lut, start, n, i, ref_number(__ldg(u)), ref_number(__ldg(u + 1)),
+                                         ref_number(__ldg(u + 2)), di, li);
                             }
                             if (i == 0) { ldir = di; len = li; }
                             HitRecord sh;
@@ -475,7 +471,7 @@ __device__ __forceinline__ uint64_t tree_child(uint64_t parent, int set, int ind
 // number base + k of the frame's slice of the reference's stream (k the
 // pixel's running index; node unused).
 struct DistStream {
-    const float *win;
+    const uint32_t *win;
     int64_t base, nwin;
     uint32_t pixel, key0, key1;
     bool pixel_mode;
@@ -499,7 +495,7 @@ struct DistStream {
             status |= kStatusBadIndex;
             return 0.0f;
         }
-        return __ldg(win + i);
+        return ref_number(__ldg(win + i));
     }
 };
 
@@ -981,7 +977,7 @@ template <bool SHADE, class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_DIST_MIN_BLOCKS) k_dist(SC sc, CameraView cam, LightSet lights,
                                                         MaterialTable table, DistLights dl, DistParams dp,
                                                         const int4 *__restrict__ area, const float *__restrict__ verts,
-                                                        const float *__restrict__ lut, const float *__restrict__ rnd,
+                                                        const float *__restrict__ lut, const uint32_t *__restrict__ rnd,
                                                         int64_t nrnd, const int64_t *__restrict__ prefix,
                                                         int64_t *__restrict__ counts, uint8_t *__restrict__ rgb,
                                                         float *__restrict__ fimg, Counters *ctr)
@@ -1269,7 +1265,8 @@ struct SGuard {
 
 rt_status check_shapes(const rt_scene *s, const rt_light *lights, int32_t nlights, const rt_light_shape *shapes,
                        const char *who);
-rt_status stream_window(SoftState &S, int64_t offset, int64_t total, cudaStream_t st, const float **rnd);
+rt_status stream_window(SoftState &S, int64_t offset, int64_t total, cudaStream_t st, const uint32_t **rnd);
+rt_status stream_used(SoftState &S, cudaStream_t st);
 
 template <class SC>
 int soft_blocks_per_sm()
@@ -1405,7 +1402,7 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
     const int64_t nhits = (int64_t)h[0] + h[1];
     const int64_t total = nhits * per_hit;
     // the frame's slice of the reference's stream
-    const float *rnd = nullptr;
+    const uint32_t *rnd = nullptr;
     {
         const rt_status wst = stream_window(S, stream_offset, total, st, &rnd);
         if (wst != RT_OK) return wst;
@@ -1434,6 +1431,10 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
     });
     RT_CUDA_S(cudaGetLastError(), "shade launch");
     RT_CUDA_S(cudaEventRecord(ctx->ev1, st), "event record");
+    {
+        const rt_status ust = stream_used(S, st);
+        if (ust != RT_OK) return ust;
+    }
     if (rgb_host) RT_CUDA_S(cudaMemcpyAsync(rgb_out, d_rgb, npix * 3, cudaMemcpyDeviceToHost, st), "rgb copy");
     if (f_host)
         RT_CUDA_S(cudaMemcpyAsync(rgb_f32, d_f, npix * 3 * sizeof(float), cudaMemcpyDeviceToHost, st), "image copy");
@@ -1590,84 +1591,138 @@ rt_status check_shapes(const rt_scene *s, const rt_light *lights, int32_t nlight
     return RT_OK;
 }
 
-// The frame's numbers [offset, offset + total) of the reference's stream on
-// the device (generated on the host into pinned memory, copied over), kept
-// while later frames fall inside them; *rnd points at number offset.  A
-// frame that starts where the last one ended finds its numbers already
-// generated by the read-ahead (or the read-ahead still running: it is
-// joined).
-rt_status stream_window(SoftState &S, int64_t offset, int64_t total, cudaStream_t st, const float **rnd)
+// Refills [r0, r1) into window `dst` (large enough), enqueued on the
+// generator's stream: what the other window already holds up to the
+// generator's position is copied, the rest generated; positions before the
+// generator's are reached from the seed.  Launches of at most kMtLaunch
+// refills, a few milliseconds each.
+constexpr int64_t kMtLaunch = 65536;
+
+rt_status generate_window(SoftState &S, int dst, int64_t r0, int64_t r1)
+{
+    SoftState::Window &w = S.win[dst];
+    const SoftState::Window &other = S.win[dst ^ 1];
+    uint32_t *state = (uint32_t *)S.rng.ptr, *out = (uint32_t *)w.words.ptr;
+    w.count = 0;
+    const int64_t at = S.refills;
+    S.refills = -1;   // whatever fails below, the next window starts from the seed
+    int64_t pos = at;
+    RT_CUDA_S(cudaStreamWaitEvent(S.gen, S.used, 0), "stream wait");
+    if (at >= 0 && other.count > 0 && other.first + other.count == at && r0 >= other.first && r0 < at) {
+        const int64_t n = std::min(at, r1) - r0;
+        RT_CUDA_S(cudaMemcpyAsync(out, (const uint32_t *)other.words.ptr + (r0 - other.first) * kMtWords,
+                                  (size_t)n * kMtWords * sizeof(uint32_t), cudaMemcpyDeviceToDevice, S.gen),
+                  "stream copy");
+    } else if (at < 0 || at > r0) {
+        RT_CUDA_S(cudaMemcpyAsync(state, state + kMtWords, kMtWords * sizeof(uint32_t), cudaMemcpyDeviceToDevice, S.gen),
+                  "generator reset");
+        pos = 0;
+    }
+    while (pos < r1) {
+        const int64_t stop = pos < r0 ? r0 : r1;
+        const int64_t n = std::min(stop - pos, kMtLaunch);
+        if (pos < r0)
+            k_ref_stream<false><<<1, kMtThreads, S.gen_smem, S.gen>>>(state, (int32_t)n, nullptr);
+        else
+            k_ref_stream<true><<<1, kMtThreads, S.gen_smem, S.gen>>>(state, (int32_t)n, out + (pos - r0) * kMtWords);
+        pos += n;
+    }
+    RT_CUDA_S(cudaGetLastError(), "generator launch");
+    RT_CUDA_S(cudaEventRecord(w.ready, S.gen), "event record");
+    S.refills = pos;
+    w.first = r0;
+    w.count = r1 - r0;
+    return RT_OK;
+}
+
+rt_status stream_setup(SoftState &S)
+{
+    if (S.used) return RT_OK;
+    // the seeded state (common/common.cc:35-50)
+    uint32_t mt[2 * kMtWords];
+    mt[0] = 5489u;
+    for (int i = 1; i < kMtWords; ++i) mt[i] = 1812433253u * (mt[i - 1] ^ (mt[i - 1] >> 30)) + (uint32_t)i;
+    std::memcpy(mt + kMtWords, mt, kMtWords * sizeof(uint32_t));
+    RT_CUDA_S(S.rng.reserve(sizeof(mt)), "generator allocation");
+    RT_CUDA_S(cudaMemcpy(S.rng.ptr, mt, sizeof(mt), cudaMemcpyHostToDevice), "generator seed");
+    // the generator's block takes all the shared memory a block can have, so
+    // that no render block shares its SM and lengthens its chain of refills
+    int most = 0;
+    RT_CUDA_S(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, S.device), "shared memory size");
+    for (const auto kernel : {k_ref_stream<false>, k_ref_stream<true>})
+        RT_CUDA_S(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most), "shared memory size");
+    S.gen_smem = (size_t)most;
+    if (!S.gen) RT_CUDA_S(cudaStreamCreateWithFlags(&S.gen, cudaStreamNonBlocking), "stream create");
+    for (SoftState::Window &w : S.win)
+        if (!w.ready) RT_CUDA_S(cudaEventCreateWithFlags(&w.ready, cudaEventDisableTiming), "event creation");
+    RT_CUDA_S(cudaEventCreateWithFlags(&S.used, cudaEventDisableTiming), "event creation");
+    S.refills = 0;
+    return RT_OK;
+}
+
+// Room for `refills` in a window; growing it waits for its readers and writers.
+rt_status window_reserve(SoftState &S, SoftState::Window &w, int64_t refills, cudaStream_t st)
+{
+    const size_t bytes = (size_t)refills * kMtWords * sizeof(uint32_t);
+    if (bytes > w.words.cap) {
+        RT_CUDA_S(cudaStreamSynchronize(st), "synchronize");
+        RT_CUDA_S(cudaStreamSynchronize(S.gen), "synchronize");
+        w.count = 0;
+        RT_CUDA_S(w.words.reserve(bytes), "stream allocation");
+    }
+    return RT_OK;
+}
+
+// The frame's numbers [offset, offset + total) of the reference's stream as
+// words on the device (ref_number), kept while later frames fall inside their
+// window; *rnd points at number offset, and `st` waits for them.  A frame that
+// starts where the last one ended finds its numbers read ahead.  The caller
+// calls stream_used after its last kernel that reads them.
+rt_status stream_window(SoftState &S, int64_t offset, int64_t total, cudaStream_t st, const uint32_t **rnd)
 {
     *rnd = nullptr;
     if (total <= 0) return RT_OK;
-    if (S.win_base >= 0 && offset >= S.win_base && offset + total <= S.win_base + S.win_len) {
-        *rnd = (const float *)S.window.ptr + (offset - S.win_base);
-        return RT_OK;
+    rt_status rc = stream_setup(S);
+    if (rc != RT_OK) return rc;
+    const auto covers = [&](const SoftState::Window &w, int64_t a, int64_t b) {
+        return w.count > 0 && a >= w.first && b <= w.first + w.count;
+    };
+    const int64_t r0 = offset / kMtWords, r1 = (offset + total + kMtWords - 1) / kMtWords;
+    int use = covers(S.win[S.cur], r0, r1) ? S.cur : covers(S.win[S.cur ^ 1], r0, r1) ? S.cur ^ 1 : -1;
+    if (use < 0) {
+        use = S.cur ^ 1;
+        rc = window_reserve(S, S.win[use], r1 - r0, st);
+        if (rc == RT_OK) rc = generate_window(S, use, r0, r1);
+        if (rc != RT_OK) return rc;
     }
-    join_ahead(S);
-    const int64_t want = total + total / 4;   // read-ahead length: the next frame draws about as many
-    if (!(S.stage_base >= 0 && offset >= S.stage_base && offset + total <= S.stage_base + S.stage_len)) {
-        // not read ahead: generate the slice here
-        // the last upload reads the staging buffer: it must be done first
-        RT_CUDA_S(cudaStreamSynchronize(st), "synchronize");
-        if (S.staging_cap < (size_t)want) {
-            if (S.staging) cudaFreeHost(S.staging);
-            S.staging = nullptr;
-            S.staging_cap = 0;
-            S.stage_base = -1;
-            S.stage_len = 0;
-            RT_CUDA_S(cudaMallocHost(&S.staging, (size_t)want * sizeof(float)), "pinned stream staging");
-            S.staging_cap = (size_t)want;
-        }
-        S.stage_base = -1;
-        S.stage_len = 0;
-        try {
-            generate_slice(S.rng, offset, total, S.staging);
-        } catch (...) {
-            return sfail(RT_ERR_OUT_OF_MEMORY, "random stream: host memory for the slice's generator states");
-        }
-        S.stage_base = offset;
-        S.stage_len = total;
-    }
-    RT_CUDA_S(S.window.reserve((size_t)total * sizeof(float)), "stream allocation");
-    RT_CUDA_S(cudaMemcpyAsync(S.window.ptr, S.staging + (offset - S.stage_base), (size_t)total * sizeof(float),
-                              cudaMemcpyHostToDevice, st),
-              "stream copy");
-    if (!S.copied) RT_CUDA_S(cudaEventCreateWithFlags(&S.copied, cudaEventDisableTiming), "event creation");
-    RT_CUDA_S(cudaEventRecord(S.copied, st), "event record");
-    S.win_base = offset;
-    S.win_len = total;
-    *rnd = (const float *)S.window.ptr;
-    // read ahead [offset + total, offset + total + want): the numbers already
-    // generated past the frame move to the front of staging (once the
-    // upload is done), the rest continue from rng, which stands at their end
-    if ((size_t)want <= S.staging_cap) {
-        const int64_t next = offset + total;
-        SoftState *P = &S;
-        try {
-            S.ahead = std::thread([P, next, want] {
-                cudaSetDevice(P->device);
-                if (cudaEventSynchronize(P->copied) != cudaSuccess) {
-                    P->stage_base = -1;   // nothing kept: the next window generates its own
-                    P->stage_len = 0;
-                    return;
-                }
-                const int64_t keep = P->stage_base + P->stage_len - next;
-                if (keep > 0)
-                    std::memmove(P->staging, P->staging + (next - P->stage_base), (size_t)keep * sizeof(float));
-                const int64_t kept = std::max<int64_t>(keep, 0);
-                try {
-                    if (want > kept) generate_slice(P->rng, next + kept, want - kept, P->staging + kept);
-                    P->stage_base = next;
-                    P->stage_len = std::max(kept, want);
-                } catch (...) {   // out of host memory: keep what is there
-                    P->stage_base = kept > 0 ? next : -1;
-                    P->stage_len = kept;
-                }
-            });
-        } catch (...) {   // no thread: the next window generates its own numbers
+    S.cur = use;
+    RT_CUDA_S(cudaStreamWaitEvent(st, S.win[use].ready, 0), "stream wait");
+    *rnd = (const uint32_t *)S.win[use].words.ptr + (offset - S.win[use].first * kMtWords);
+    // read ahead from the frame's end, a quarter more than it drew, unless the
+    // other window holds that already
+    const int64_t next = offset + total;
+    const int64_t n0 = next / kMtWords, n1 = (next + total + kMtWords - 1) / kMtWords;
+    SoftState::Window &ahead = S.win[use ^ 1];
+    if (!covers(ahead, n0, n1)) {
+        const int64_t n2 = (next + total + total / 4 + kMtWords - 1) / kMtWords;
+        const size_t bytes = (size_t)(n2 - n0) * kMtWords * sizeof(uint32_t);
+        size_t free_b = 0, all_b = 0;
+        if (bytes <= ahead.words.cap || (cudaMemGetInfo(&free_b, &all_b) == cudaSuccess && 2 * bytes < free_b)) {
+            // without room to read ahead the next frame generates its own numbers
+            if (window_reserve(S, ahead, n2 - n0, st) == RT_OK) {
+                rc = generate_window(S, use ^ 1, n0, n2);
+                if (rc != RT_OK) return rc;
+            }
         }
     }
+    return RT_OK;
+}
+
+// After the last kernel on `st` that reads the frame's numbers: the window is
+// not written again before it.
+rt_status stream_used(SoftState &S, cudaStream_t st)
+{
+    if (S.used) RT_CUDA_S(cudaEventRecord(S.used, st), "event record");
     return RT_OK;
 }
 
@@ -1807,7 +1862,7 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
 
     RT_CUDA_S(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), st), "counter clear");
     RT_CUDA_S(cudaEventRecord(ctx->ev0, st), "event record");
-    const float *rnd = nullptr;
+    const uint32_t *rnd = nullptr;
     int64_t total = 0;
     if (smp.stream == RT_STREAM_REFERENCE) {
         // counting pass, scan, the frame's slice of the stream
@@ -1908,6 +1963,10 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
     }
     RT_CUDA_S(cudaGetLastError(), "shade launch");
     RT_CUDA_S(cudaEventRecord(ctx->ev1, st), "event record");
+    {
+        const rt_status ust = stream_used(S, st);
+        if (ust != RT_OK) return ust;
+    }
     if (rgb_host) RT_CUDA_S(cudaMemcpyAsync(rgb_out, d_rgb, npix * 3, cudaMemcpyDeviceToHost, st), "rgb copy");
     if (f_host)
         RT_CUDA_S(cudaMemcpyAsync(rgb_f32, d_f, npix * 3 * sizeof(float), cudaMemcpyDeviceToHost, st), "image copy");
