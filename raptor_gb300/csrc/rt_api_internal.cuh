@@ -46,6 +46,7 @@ struct rt_context {
     rtc::Counters *d_counters = nullptr;
     rtc::Counters *h_counters = nullptr;   // pinned
     int32_t *h_scratch = nullptr;          // pinned
+    void *h_rays = nullptr;                // pinned: host rays and results of small ray queries (kFewHostRays)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     rtc::DevBuf stage_a, stage_b, stage_c;
     rtc::DevBuf redo;                      // pixels queued for an exact second pass
