@@ -62,34 +62,45 @@ __global__ void __launch_bounds__(kTraceThreads) k_diff(SC sc, const float *__re
         int x, y;
         tile_pixel<8>(base + (threadIdx.x & 31), tiles_x, x, y);
         const bool live = (x < cam.xres) && (y < cam.yres);
-        bool hit = false;
-        uint32_t nsec = 0;
+        // every ray first, the warp's in step; then the lanes' shading from the
+        // hit and the lights' answers (the shading's registers are not held
+        // through the traversals)
+        const RayState r = camera_ray(cam, x, y);
+        HitRecord h;
+        bool occ;
+        status |= traverse_warp<false>(sc, live, r.o, r.d, FLT_MAX, h, occ);
+        const bool hit = h.t < FLT_MAX;
+        const uint32_t nsec = hit ? (uint32_t)lights.n : 0u;
+        uint32_t obits = 0;
+        float3 start = r.o;
+        if (hit) {
+            const SurfacePoint sp = surface_at(sc, r, h);
+            start = offset_start(sp.dst, sp.geo);
+        }
+        const int nl = __any_sync(0xffffffffu, hit) ? lights.n : 0;
+        for (int l = 0; l < nl; ++l) {
+            float3 ldir = r.d;
+            float len = 0.f;
+            if (hit) shadow_ray(lights.l[l], start, ldir, len);
+            HitRecord sh;
+            bool blocked;
+            status |= traverse_warp<true>(sc, hit, start, ldir, len, sh, blocked);
+            if (blocked) obits |= 1u << l;
+        }
         if (live) {
             const size_t pix = (size_t)x + (size_t)y * (size_t)cam.xres;
-            const RayState r = camera_ray(cam, x, y);
-            HitRecord h;
-            bool occ;
-            status |= traverse<false>(sc, r.o, r.d, FLT_MAX, h, occ);
-            hit = h.t < FLT_MAX;
             if (!ADJOINT) {
                 // float forward: the same per-pixel work as rt_render, unclipped
                 float3 c = cam.background;
-                uint32_t obits = 0;
                 if (hit) {
                     const SurfacePoint sp = surface_at(sc, r, h);
-                    const float3 start = offset_start(sp.dst, sp.geo);
                     const float3 kd = material_kd(mat, sp);
                     c = make_float3(0.f, 0.f, 0.f);
                     for (int l = 0; l < lights.n; ++l) {
                         float3 ldir;
                         float len;
                         shadow_ray(lights.l[l], start, ldir, len);
-                        HitRecord sh;
-                        bool blocked;
-                        status |= traverse<true>(sc, start, ldir, len, sh, blocked);
-                        ++nsec;
-                        if (blocked) obits |= 1u << l;
-                        phong_add(lights.l[l], mat, kd, sp.sn, r.d, ldir, len, blocked ? 0.0f : 1.0f, c);
+                        phong_add(lights.l[l], mat, kd, sp.sn, r.d, ldir, len, ((obits >> l) & 1u) ? 0.0f : 1.0f, c);
                     }
                     c = xadd3(c, mat.ka);
                 }
@@ -100,8 +111,6 @@ __global__ void __launch_bounds__(kTraceThreads) k_diff(SC sc, const float *__re
                 if (occl) occl[pix] = (uint8_t)obits;
             } else if (hit) {
                 const float3 g = f3(dldpix[3 * pix], dldpix[3 * pix + 1], dldpix[3 * pix + 2]);
-                const SurfacePoint sp = surface_at(sc, r, h);
-                const float3 start = offset_start(sp.dst, sp.geo);
                 const int3 tv = sc.idx[h.id];
                 const float3 A = f3(verts[3 * tv.x], verts[3 * tv.x + 1], verts[3 * tv.x + 2]);
                 const float3 B = f3(verts[3 * tv.y], verts[3 * tv.y + 1], verts[3 * tv.y + 2]);
@@ -132,11 +141,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_diff(SC sc, const float *__re
                     float3 ldir_f;
                     float len_f;
                     shadow_ray(L, start, ldir_f, len_f);
-                    HitRecord sh;
-                    bool blocked;
-                    status |= traverse<true>(sc, start, ldir_f, len_f, sh, blocked);
-                    ++nsec;
-                    if (blocked) continue;
+                    if ((obits >> l) & 1u) continue;
                     // analytic light vector from the unrefined hit point
                     float3 ldir;
                     float len;

@@ -53,13 +53,16 @@ __global__ void __launch_bounds__(256, RT_RENDER_MIN_BLOCKS / 2) k_render_batche
             PixelOut po;
             po.hit = false;
             po.secondary = 0;
+            // not in step: the kernel holds the AO path too, and in step it
+            // lost (24 scenes: 2.60 -> 2.77 ms)
             if (live) {
                 if (J.mode == RT_JOB_AO)
                     po = shade_pixel_ao<false, STACK>(sc, J.cam, J.mat, J.ao_samples, J.ao_dist, J.ao_seed, x, y,
                                                       status, nullptr);
                 else
-                    po = shade_pixel_lights<false, false, STACK>(sc, J.cam, J.lights, J.nlights, J.mat, x, y,
-                                                                 status, nullptr, J.fast_pow != 0);
+                    po = shade_pixel_lights<false, false, false, STACK>(sc, J.cam, J.lights, J.nlights, J.mat, x, y,
+                                                                        status, nullptr, J.fast_pow != 0, nullptr,
+                                                                        true);
                 const size_t pix = (size_t)x + (size_t)y * (size_t)J.cam.xres;
                 store_rgb(J.rgb, pix, po.c);
                 if (J.ids) J.ids[pix] = po.id;

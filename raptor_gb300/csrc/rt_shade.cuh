@@ -58,48 +58,58 @@ struct PixelOut {
 // Primary ray, closest hit, one shadow ray per light, coloured Phong
 // (ray_trace_engine::ray_trace, raytracer.cc:20-87).  TABLE: the hit
 // triangle's material from `table` (per-triangle indices in sc.mat), else
-// `mat0` for every triangle.
-template <bool COUNT, bool TABLE = false, int STACK = kStackSize, class SC>
+// `mat0` for every triangle.  live: the lane has a pixel.  STEP: the warp's
+// rays are traced in step (traverse_warp), so every lane calls it, converged.
+template <bool COUNT, bool TABLE = false, bool STEP = true, int STACK = kStackSize, class SC>
 __device__ __forceinline__ PixelOut shade_pixel_lights(const SC &sc, const CameraView &cam, const LightView *lights,
                                                        int nl, const MaterialView &mat0, int x, int y,
                                                        uint32_t &status, FetchCount *fc, bool fast_pow,
-                                                       const MaterialTable *table = nullptr)
+                                                       const MaterialTable *table, bool live)
 {
     PixelOut out;
     out.secondary = 0;
     out.ao_made = 0;
     const RayState r = camera_ray(cam, x, y);
     HitRecord h;
+    h.t = FLT_MAX;
     bool occ;
-    status |= traverse<false, COUNT, STACK>(sc, r.o, r.d, FLT_MAX, h, occ, fc);
+    if (STEP) status |= traverse_warp<false, COUNT, STACK>(sc, live, r.o, r.d, FLT_MAX, h, occ, fc);
+    else if (live) status |= traverse<false, COUNT, STACK>(sc, r.o, r.d, FLT_MAX, h, occ, fc);
     out.hit = h.t < FLT_MAX;
     out.id = out.hit ? h.id - sc.tri_base : -1;
     out.c = cam.background;
+    if (STEP ? !__any_sync(0xffffffffu, out.hit) : !out.hit) return out;
+    SurfacePoint sp;
+    float3 start = r.o, kd = r.o, c = make_float3(0.f, 0.f, 0.f);
+    int32_t mi = 0;
     if (out.hit) {
-        int32_t mi = 0;
         if (TABLE && sc.mat) {
             mi = __ldg(&sc.mat[out.id]);
             if (mi < 0 || mi >= table->n) { status |= kStatusBadIndex; mi = 0; }
         }
-        const MaterialView &mat = TABLE ? table->m[mi] : mat0;
-        const SurfacePoint sp = surface_at(sc, r, h);
-        const float3 start = offset_start(sp.dst, sp.geo);
-        const float3 kd = material_kd(mat, sp);
-        float3 c = make_float3(0.f, 0.f, 0.f);
-        uint32_t blocked_bits = 0;
-        for (int l = 0; l < nl; ++l) {
-            const LightView &L = lights[l];
-            float3 ldir;
-            float len;
-            shadow_ray(L, start, ldir, len);
-            HitRecord sh;
-            bool blocked;
-            status |= traverse<true, COUNT, STACK>(sc, start, ldir, len, sh, blocked, fc);
+        sp = surface_at(sc, r, h);
+        start = offset_start(sp.dst, sp.geo);
+        kd = material_kd(TABLE ? table->m[mi] : mat0, sp);
+    }
+    const MaterialView &mat = TABLE ? table->m[mi] : mat0;
+    uint32_t blocked_bits = 0;
+    for (int l = 0; l < nl; ++l) {
+        const LightView &L = lights[l];
+        float3 ldir = r.d;
+        float len = 0.f;
+        if (out.hit) shadow_ray(L, start, ldir, len);
+        HitRecord sh;
+        bool blocked = false;
+        if (STEP) status |= traverse_warp<true, COUNT, STACK>(sc, out.hit, start, ldir, len, sh, blocked, fc);
+        else status |= traverse<true, COUNT, STACK>(sc, start, ldir, len, sh, blocked, fc);
+        if (out.hit) {
             ++out.secondary;
             if (blocked) blocked_bits |= 1u << l;
             if (fast_pow) phong_add<false>(L, mat, kd, sp.sn, r.d, ldir, len, blocked ? 0.0f : 1.0f, c);
             else phong_add<true>(L, mat, kd, sp.sn, r.d, ldir, len, blocked ? 0.0f : 1.0f, c);
         }
+    }
+    if (out.hit) {
         out.c = xadd3(c, mat.ka);
         if (fast_pow && near_truncation(out.c))
             out.c = shade_lights_exact(lights, nl, mat, kd, sp.sn, r.d, start, blocked_bits);

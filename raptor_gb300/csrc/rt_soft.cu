@@ -314,11 +314,11 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_pr
         tile_pixel<8>(base + (threadIdx.x & 31), tiles_x, x, y);
         const bool live = (x < cam.xres) && (y < cam.yres);
         bool hit = false;
+        const RayState r = camera_ray(cam, x, y);
+        HitRecord h;
+        bool occ;
+        status |= traverse_warp<false>(sc, live, r.o, r.d, FLT_MAX, h, occ);
         if (live) {
-            const RayState r = camera_ray(cam, x, y);
-            HitRecord h;
-            bool occ;
-            status |= traverse<false>(sc, r.o, r.d, FLT_MAX, h, occ);
             hit = h.t < FLT_MAX;
             const size_t pix = (size_t)x + (size_t)y * (size_t)cam.xres;
             hits[pix] = make_int4(h.id, __float_as_int(h.t), __float_as_int(h.u), __float_as_int(h.v));
@@ -348,73 +348,86 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_sh
         int x, y;
         tile_pixel<8>(base + (threadIdx.x & 31), tiles_x, x, y);
         const bool live = (x < cam.xres) && (y < cam.yres);
+        // every lane goes through the lights and their rays, so that the warp's
+        // rays to one light are traced in step
         uint32_t nsec = 0;
+        const size_t pix = (size_t)x + (size_t)y * (size_t)cam.xres;
+        HitRecord h;
+        h.t = FLT_MAX;
         if (live) {
-            const size_t pix = (size_t)x + (size_t)y * (size_t)cam.xres;
             const int4 hr = hits[pix];
-            float3 c = cam.background;
-            if (__int_as_float(hr.y) < FLT_MAX) {
-                HitRecord h;
-                h.id = hr.x;
-                h.t = __int_as_float(hr.y);
-                h.u = __int_as_float(hr.z);
-                h.v = __int_as_float(hr.w);
-                const RayState r = camera_ray(cam, x, y);
-                int32_t mi = 0;
-                if (sc.mat) {
-                    mi = __ldg(&sc.mat[h.id - sc.tri_base]);
-                    if (mi < 0 || mi >= table.n) { status |= kStatusBadIndex; mi = 0; }
-                }
-                const MaterialView &mat = table.m[mi];
-                const SurfacePoint sp = surface_at(sc, r, h);
-                const float3 start = offset_start(sp.dst, sp.geo);
-                const float3 kd = material_kd(mat, sp);
-                int64_t draw = (int64_t)prefix[pix] * per_hit;
-                c = make_float3(0.f, 0.f, 0.f);
-                for (int l = 0; l < lights.n; ++l) {
-                    const LightView &L = lights.l[l];
-                    float3 ldir;
-                    float len;
-                    int n = 1, made = 0;
-                    if (soft_light(L, samples)) {
-                        n = samples;
-                        if (draw + (int64_t)areas.draws[l] > nrnd) {   // never expected: the host sized the slice
-                            status |= kStatusBadIndex;
-                            break;
-                        }
-                        const bool tri_light = areas.made[l] > 0;
-                        for (int i = 0; i < n; ++i) {
-                            float3 di;
-                            float li;
-                            if (tri_light) {
-                                const uint32_t *u = rnd + draw + 2 * i;
-                                area_ray(verts, sc.idx, __ldg(area + areas.first[l] + i), start, ref_number(__ldg(u)),
-                                         ref_number(__ldg(u + 1)), di, li);
-                            } else {
-                                const uint32_t *u = rnd + draw + 3 * i;
-                                soft_ray(L, lut, start, n, i, ref_number(__ldg(u)), ref_number(__ldg(u + 1)),
-                                         ref_number(__ldg(u + 2)), di, li);
-                            }
-                            if (i == 0) { ldir = di; len = li; }
-                            HitRecord sh;
-                            bool blocked;
-                            status |= traverse<true>(sc, start, di, li, sh, blocked);
-                            if (!blocked) ++made;
-                        }
-                        draw += areas.draws[l];
-                    } else {
-                        shadow_ray(L, start, ldir, len);
-                        HitRecord sh;
-                        bool blocked;
-                        status |= traverse<true>(sc, start, ldir, len, sh, blocked);
-                        made = blocked ? 0 : 1;
-                    }
-                    nsec += (uint32_t)n;
-                    // made_it / nr_pending_shadows, both floats (raytracer.cc:46-61)
-                    phong_add<true>(L, mat, kd, sp.sn, r.d, ldir, len, xdiv((float)made, (float)n), c);
-                }
-                c = xadd3(c, mat.ka);
+            h.id = hr.x;
+            h.t = __int_as_float(hr.y);
+            h.u = __int_as_float(hr.z);
+            h.v = __int_as_float(hr.w);
+        }
+        bool on = h.t < FLT_MAX;   // false from here on for a lane that leaves the lights' loop
+        const bool hit = on;
+        const RayState r = camera_ray(cam, x, y);
+        SurfacePoint sp;
+        float3 start = r.o, kd = r.o, c = make_float3(0.f, 0.f, 0.f);
+        int32_t mi = 0;
+        int64_t draw = 0;
+        if (hit) {
+            if (sc.mat) {
+                mi = __ldg(&sc.mat[h.id - sc.tri_base]);
+                if (mi < 0 || mi >= table.n) { status |= kStatusBadIndex; mi = 0; }
             }
+            sp = surface_at(sc, r, h);
+            start = offset_start(sp.dst, sp.geo);
+            kd = material_kd(table.m[mi], sp);
+            draw = (int64_t)prefix[pix] * per_hit;
+        }
+        const MaterialView &mat = table.m[mi];
+        const int nl = __any_sync(0xffffffffu, on) ? lights.n : 0;
+        for (int l = 0; l < nl; ++l) {
+            const LightView &L = lights.l[l];
+            float3 ldir = r.d;
+            float len = 0.f;
+            int n = 1, made = 0;
+            if (soft_light(L, samples)) {
+                n = samples;
+                if (on && draw + (int64_t)areas.draws[l] > nrnd) {   // never expected: the host sized the slice
+                    status |= kStatusBadIndex;
+                    on = false;
+                }
+                const bool tri_light = areas.made[l] > 0;
+                for (int i = 0; i < n; ++i) {
+                    float3 di = r.d;
+                    float li = 0.f;
+                    if (on) {
+                        if (tri_light) {
+                            const uint32_t *u = rnd + draw + 2 * i;
+                            area_ray(verts, sc.idx, __ldg(area + areas.first[l] + i), start, ref_number(__ldg(u)),
+                                     ref_number(__ldg(u + 1)), di, li);
+                        } else {
+                            const uint32_t *u = rnd + draw + 3 * i;
+                            soft_ray(L, lut, start, n, i, ref_number(__ldg(u)), ref_number(__ldg(u + 1)),
+                                     ref_number(__ldg(u + 2)), di, li);
+                        }
+                    }
+                    if (i == 0) { ldir = di; len = li; }
+                    HitRecord sh;
+                    bool blocked;
+                    status |= traverse_warp<true>(sc, on, start, di, li, sh, blocked);
+                    if (!blocked) ++made;
+                }
+                draw += areas.draws[l];
+            } else {
+                if (on) shadow_ray(L, start, ldir, len);
+                HitRecord sh;
+                bool blocked;
+                status |= traverse_warp<true>(sc, on, start, ldir, len, sh, blocked);
+                made = blocked ? 0 : 1;
+            }
+            if (on) {
+                nsec += (uint32_t)n;
+                // made_it / nr_pending_shadows, both floats (raytracer.cc:46-61)
+                phong_add<true>(L, mat, kd, sp.sn, r.d, ldir, len, xdiv((float)made, (float)n), c);
+            }
+        }
+        if (live) {
+            c = hit ? xadd3(c, mat.ka) : cam.background;
             if (rgb) store_rgb(rgb, pix, c);
             if (fimg) {
                 fimg[3 * pix] = c.x;

@@ -101,8 +101,9 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render(
         PixelOut po;
         po.hit = false;
         po.secondary = 0;
+        po = shade_pixel_lights<COUNT>(sc, cam, lights.l, lights.n, mat, x, y, status, &fc, lights.fast_pow != 0, nullptr,
+                                       live);
         if (live) {
-            po = shade_pixel_lights<COUNT>(sc, cam, lights.l, lights.n, mat, x, y, status, &fc, lights.fast_pow != 0);
             const size_t pix = (size_t)x + (size_t)y * (size_t)cam.xres;
             store_rgb(rgb, pix, po.c);
             if (ids) ids[pix] = po.id;
@@ -140,9 +141,9 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
         PixelOut po;
         po.hit = false;
         po.secondary = 0;
+        po = shade_pixel_lights<COUNT, true>(sc, cam, lights.l, lights.n, table.m[0], x, y, status, &fc, false, &table,
+                                             live);
         if (live) {
-            po = shade_pixel_lights<COUNT, true>(sc, cam, lights.l, lights.n, table.m[0], x, y, status, &fc, false,
-                                                 &table);
             const size_t pix = (size_t)x + (size_t)y * (size_t)cam.xres;
             fimg[3 * pix] = po.c.x;
             fimg[3 * pix + 1] = po.c.y;
@@ -181,9 +182,9 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
         PixelOut po;
         po.hit = false;
         po.secondary = 0;
+        po = shade_pixel_lights<COUNT, true>(sc, cam, lights.l, lights.n, mat, x, y, status, &fc, lights.fast_pow != 0,
+                                             &table, live);
         if (live) {
-            po = shade_pixel_lights<COUNT, true>(sc, cam, lights.l, lights.n, mat, x, y, status, &fc,
-                                                 lights.fast_pow != 0, &table);
             const size_t pix = (size_t)x + (size_t)y * (size_t)cam.xres;
             store_rgb(rgb, pix, po.c);
             if (ids) ids[pix] = po.id;
@@ -345,17 +346,18 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
         tile_pixel<8>(base + (threadIdx.x & 31), tiles_x, x, y);
         const bool live = (x < out_x) && (y < out_y);
         uint32_t primary = 0, hits = 0, secondary = 0;
+        float3 sum = make_float3(0.f, 0.f, 0.f);
+        for (int ax = 0; ax < aa_x; ++ax)
+            for (int ay = 0; ay < aa_y; ++ay) {
+                const PixelOut po = shade_pixel_lights<COUNT>(sc, cam, lights.l, lights.n, mat, x * aa_x + ax,
+                                                              y * aa_y + ay, status, &fc, lights.fast_pow != 0, nullptr,
+                                                              live);
+                sum = xadd3(sum, po.c);
+                primary += live ? 1u : 0u;
+                hits += po.hit ? 1u : 0u;
+                secondary += po.secondary;
+            }
         if (live) {
-            float3 sum = make_float3(0.f, 0.f, 0.f);
-            for (int ax = 0; ax < aa_x; ++ax)
-                for (int ay = 0; ay < aa_y; ++ay) {
-                    const PixelOut po = shade_pixel_lights<COUNT>(sc, cam, lights.l, lights.n, mat, x * aa_x + ax,
-                                                                  y * aa_y + ay, status, &fc, lights.fast_pow != 0);
-                    sum = xadd3(sum, po.c);
-                    ++primary;
-                    hits += po.hit ? 1u : 0u;
-                    secondary += po.secondary;
-                }
             const float3 avg = make_float3(xdiv(sum.x, nsamples), xdiv(sum.y, nsamples), xdiv(sum.z, nsamples));
             const int32_t pix = x + y * out_x;
             if (lights.fast_pow && near_truncation(avg)) {
@@ -412,9 +414,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
         po.c = make_float3(0.f, 0.f, 0.f);
         po.hit = false;
         po.secondary = 0;
-        if (live)
-            po = shade_pixel_lights<COUNT>(sc, cam, lights.l, lights.n, mat, x * aa_x + ax, y * aa_y + ay, status,
-                                           &fc, lights.fast_pow != 0);
+        po = shade_pixel_lights<COUNT>(sc, cam, lights.l, lights.n, mat, x * aa_x + ax, y * aa_y + ay, status, &fc,
+                                       lights.fast_pow != 0, nullptr, live);
         const int first = g * S;
         float3 sum = make_float3(0.f, 0.f, 0.f);
         for (int k = 0; k < S; ++k) {
@@ -456,18 +457,21 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
     const int32_t n = min(ctr->redo, out_x * (cam.yres / aa_y));
     const float nsamples = (float)(aa_x * aa_y);
     uint32_t status = 0;
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int32_t pix = redo[i];
+    const int lane = threadIdx.x & 31;
+    for (int32_t i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const bool live = i0 + lane < n;
+        const int32_t pix = live ? redo[i0 + lane] : 0;
         const int x = pix % out_x, y = pix / out_x;
         float3 sum = make_float3(0.f, 0.f, 0.f);
         for (int ax = 0; ax < aa_x; ++ax)
             for (int ay = 0; ay < aa_y; ++ay) {
                 const PixelOut po = shade_pixel_lights<false>(sc, cam, lights.l, lights.n, mat, x * aa_x + ax,
-                                                              y * aa_y + ay, status, nullptr, false);
+                                                              y * aa_y + ay, status, nullptr, false, nullptr, live);
                 sum = xadd3(sum, po.c);
             }
-        store_rgb(rgb, (size_t)pix,
-                  make_float3(xdiv(sum.x, nsamples), xdiv(sum.y, nsamples), xdiv(sum.z, nsamples)));
+        if (live)
+            store_rgb(rgb, (size_t)pix,
+                      make_float3(xdiv(sum.x, nsamples), xdiv(sum.y, nsamples), xdiv(sum.z, nsamples)));
     }
     if (status) atomicOr(&ctr->status, status);
 }
