@@ -169,6 +169,7 @@ struct SoftState {
     // (colour, material; first item, set sizes), the items (its sets' rays),
     // their subtrees' colours, the item count
     DevBuf root_c, root_sets, items, item_c, nitems;
+    DevBuf node_sets, node_hits, node_over;   // the nodes' children, hit nodes, nodes walked whole
     int64_t item_cap = 0;
     // The stream's words on the device: two windows, one a frame reads from and
     // one the generator reads ahead into on its own stream, while the frame
@@ -217,6 +218,9 @@ void soft_release(rt_context *ctx)
     S.items.release();
     S.item_c.release();
     S.nitems.release();
+    S.node_sets.release();
+    S.node_hits.release();
+    S.node_over.release();
     delete ctx->soft;
     ctx->soft = nullptr;
 }
@@ -595,6 +599,58 @@ __device__ __forceinline__ void spawn_child(const DistFrame &f, const MaterialVi
     C.stage = kDistTrace;
 }
 
+// Ray `sample` of light l's n at a hit whose numbers for the light start at kb.
+__device__ __forceinline__ void dist_light_ray(const LightSet &lights, const DistLights &dl,
+                                               const int4 *__restrict__ area, const float *__restrict__ verts,
+                                               const int3 *__restrict__ idx, const float *__restrict__ lut,
+                                               DistStream &S, uint64_t node, int l, int lvl, int n, int sample,
+                                               uint32_t kb, float3 start, float3 &di, float &li, uint32_t &status)
+{
+    const LightView &L = lights.l[l];
+    if (n == 1) {
+        shadow_ray(L, start, di, li);
+    } else if (dl.made[l][lvl] > 0) {
+        const float u0 = S.at(node, kb + 2 * sample, status);
+        const float u1 = S.at(node, kb + 2 * sample + 1, status);
+        area_ray(verts, idx, __ldg(area + dl.first[l][lvl] + sample), start, u0, u1, di, li);
+    } else {
+        const float u0 = S.at(node, kb + 3 * sample, status);
+        const float u1 = S.at(node, kb + 3 * sample + 1, status);
+        const float u2 = S.at(node, kb + 3 * sample + 2, status);
+        soft_ray(L, lut, start, n, sample, u0, u1, u2, di, li);
+    }
+}
+
+// The sets of a shaded node (f.nrefl, f.nrefr rays; 0 on entry), their
+// numbers from kb on, past the lights'.
+__device__ __forceinline__ void dist_sets(DistFrame &f, const MaterialView &m, const DistParams &dp, uint32_t &kb)
+{
+    if ((double)xmul(f.magn, m.rf) > 0.1) {
+        if (dp.diffuse > 0 && dp.rfd[f.mat] != 0.0f) {
+            f.nrefl = dist_count(dp.diffuse, f.level);
+            f.refl_at = kb;
+            kb += 2u * (uint32_t)f.nrefl;
+        } else {
+            f.nrefl = 1;
+        }
+    }
+    if ((double)xmul(f.magn, m.tran) > 0.1) {
+        float ri = m.ri;
+        const float rdn = -xdot(f.d, f.sn);
+        if (f.out_in) ri = xdiv(1.0f, ri);
+        const float cos_t2 = xsub(1.0f, xmul(xmul(ri, ri), xsub(1.0f, xmul(rdn, rdn))));
+        if (!(cos_t2 < 0.0f)) {
+            if (dp.diffuse > 0 && dp.td[f.mat] != 0.0f) {
+                f.nrefr = dist_count(dp.diffuse, f.level);
+                f.refr_at = kb;
+                kb += 2u * (uint32_t)f.nrefr;
+            } else {
+                f.nrefr = 1;
+            }
+        }
+    }
+}
+
 // The counting pass of a reference-stream frame without diffuse rays: the
 // pixel's ray tree (ray_trace_engine::ray_trace, raytracer.cc:20-87) walked
 // post-order with an explicit stack, without shadow rays, counting the
@@ -774,19 +830,8 @@ __device__ __forceinline__ bool walk_advance(Walk &w, const SceneView &sc, const
                     // ray `sample` of this light
                     float3 di;
                     float li;
-                    if (w.nl == 1) {
-                        shadow_ray(L, w.start, di, li);
-                    } else if (dl.made[w.light][w.lvl] > 0) {
-                        const float u0 = S.at(f.node, w.kb + 2 * w.sample, status);
-                        const float u1 = S.at(f.node, w.kb + 2 * w.sample + 1, status);
-                        area_ray(verts, sc.idx, __ldg(area + dl.first[w.light][w.lvl] + w.sample), w.start, u0, u1, di,
-                                 li);
-                    } else {
-                        const float u0 = S.at(f.node, w.kb + 3 * w.sample, status);
-                        const float u1 = S.at(f.node, w.kb + 3 * w.sample + 1, status);
-                        const float u2 = S.at(f.node, w.kb + 3 * w.sample + 2, status);
-                        soft_ray(L, lut, w.start, w.nl, w.sample, u0, u1, u2, di, li);
-                    }
+                    dist_light_ray(lights, dl, area, verts, sc.idx, lut, S, f.node, w.light, w.lvl, w.nl, w.sample,
+                                   w.kb, w.start, di, li, status);
                     if (w.sample == 0) {
                         w.ldir = di;
                         w.len = li;
@@ -809,30 +854,7 @@ __device__ __forceinline__ bool walk_advance(Walk &w, const SceneView &sc, const
             }
             // shaded: ka, then the sets (their numbers after the lights')
             f.c = xadd3(w.c, m.ka);
-            if ((double)xmul(f.magn, m.rf) > 0.1) {
-                if (dp.diffuse > 0 && dp.rfd[f.mat] != 0.0f) {
-                    f.nrefl = dist_count(dp.diffuse, f.level);
-                    f.refl_at = w.kb;
-                    w.kb += 2u * (uint32_t)f.nrefl;
-                } else {
-                    f.nrefl = 1;
-                }
-            }
-            if ((double)xmul(f.magn, m.tran) > 0.1) {
-                float ri = m.ri;
-                const float rdn = -xdot(f.d, f.sn);
-                if (f.out_in) ri = xdiv(1.0f, ri);
-                const float cos_t2 = xsub(1.0f, xmul(xmul(ri, ri), xsub(1.0f, xmul(rdn, rdn))));
-                if (!(cos_t2 < 0.0f)) {
-                    if (dp.diffuse > 0 && dp.td[f.mat] != 0.0f) {
-                        f.nrefr = dist_count(dp.diffuse, f.level);
-                        f.refr_at = w.kb;
-                        w.kb += 2u * (uint32_t)f.nrefr;
-                    } else {
-                        f.nrefr = 1;
-                    }
-                }
-            }
+            dist_sets(f, m, dp, w.kb);
             w.drawn += w.kb - w.k0;
             if (!dp.pixel_stream) w.k = w.kb;
             f.child = 0;
@@ -1077,6 +1099,12 @@ __device__ __forceinline__ DistStream pixel_streams(const DistParams &dp, uint32
     return S;
 }
 
+#ifndef RT_DIST_NODE_MIN_BLOCKS
+#define RT_DIST_NODE_MIN_BLOCKS 7
+#endif
+#ifndef RT_DIST_LIGHTS_MIN_BLOCKS
+#define RT_DIST_LIGHTS_MIN_BLOCKS 8
+#endif
 template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_DIST_MIN_BLOCKS) k_dist_root(
     SC sc, CameraView cam, LightSet lights, MaterialTable table, DistLights dl, DistParams dp,
@@ -1152,11 +1180,314 @@ __global__ void __launch_bounds__(kTraceThreads, RT_DIST_MIN_BLOCKS) k_dist_root
     if (status) atomicOr(&ctr->status, status);
 }
 
-// The items' subtrees, one per lane; a warp takes 32 consecutive items
-// (the rays of one or two sets) at a time.  (Lanes that take the next item
-// as soon as theirs is finished were measured slower: 61 against 41 ms on
-// the 512x512 glass frame with 16-ray diffuse sets, their rays no longer
-// neighbours.)
+// The items of a frame: nr of the reflection sets from entry 0, nt of the
+// refraction sets from entry cap, walked as [0, nr) rounded up to a warp and
+// then [0, nt).  Entries 2 cap .. 2 cap + pool hold the nodes below them.
+struct DistLists {
+    int32_t nr, nt, cap, pool;
+
+    __host__ __device__ __forceinline__ int count() const { return ((nr + 31) & ~31) + nt; }
+    __device__ __forceinline__ int slot(int v) const   // -1: none
+    {
+        const int rw = (nr + 31) & ~31;
+        return v < rw ? (v < nr ? v : -1) : (v - rw < nt ? cap + (v - rw) : -1);
+    }
+};
+
+// Counts of a piece of the items' subtrees, level by level.
+struct DistCounts {
+    int32_t hits, over;                 // nodes to shade, nodes left to k_dist_sub
+    int32_t work_lights, work_over;
+    int32_t made[kDistDepth + 1];       // nodes asked for at each level below the items' (level 0)
+    int32_t work[kDistDepth + 1];
+};
+
+// Entries [first, end) of the pool that hold level k's nodes.
+__device__ __forceinline__ void dist_level(const DistCounts *dc, int pool, int k, int &first, int &end)
+{
+    int at = 0;
+    end = 0;
+    for (int j = 1; j <= k; ++j) {
+        at = end;
+        end = (int)min((int64_t)pool, (int64_t)at + dc->made[j]);
+    }
+    first = at;
+}
+
+// A node that hit something, for its lights.
+struct DistHit {
+    float4 start_slot;   // the rays' start, the node's entry (int bits)
+    float4 kd_mat;       // diffuse colour, material (int bits)
+    float4 sn;           // shading normal
+};
+
+constexpr float kDistNoNode = -1.0f;   // the power of an entry without a node
+
+// The items' subtrees are traced a level of all of them at a time: every
+// lane of a warp traces a closest hit (k_dist_node), then every lane the
+// rays to the lights of a hit (k_dist_lights), then colours are gathered
+// from the deepest level up (k_dist_gather).  A node's numbers are keyed by
+// the node and follow the lights', whose count is known before they are
+// traced, so children are made as soon as their parent has hit.  A node
+// whose children don't fit the pool is walked whole by one lane
+// (k_dist_sub), as is everything where the lists can't be had.
+// The walk is bound by issue slots at 11.8 lanes an instruction: lanes stand at
+// nodes and rays of different kinds.  512x512 glass frame with 16-ray diffuse
+// sets and soft shadows (51.6 M rays): walked 23.9 ms, by levels 21.6, with a
+// hit's rays to a light on neighbouring lanes 19.4, with 7 and 8 blocks to an SM
+// for 6 and 6 18.65 ms.
+template <class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_DIST_NODE_MIN_BLOCKS) k_dist_node(
+    SC sc, CameraView cam, LightSet lights, MaterialTable table, DistLights dl, DistParams dp,
+    const float *__restrict__ lut, DistItem *__restrict__ items, DistLists lists, int v0, int v1, int level, int last,
+    int4 *__restrict__ sets, float4 *__restrict__ item_c, DistHit *__restrict__ hits, int32_t *__restrict__ over,
+    DistCounts *dc, Counters *ctr)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const int pool0 = 2 * lists.cap;
+    int first = v0, end = v1, next = 0;
+    if (level > 0) dist_level(dc, lists.pool, level, first, end);
+    if (level > 0) next = end;         // the next level's nodes follow
+    uint32_t status = 0;
+    uint32_t nsec = 0;
+    unsigned long long drawn = 0;
+    for (;;) {
+        const int base = first + warp_claim(&dc->work[level], 32);
+        if (base >= end) break;
+        const int v = base + (int)lane;
+        const int slot = v < end ? (level > 0 ? pool0 + v : lists.slot(v)) : -1;
+        DistFrame f;
+        f.o = f.d = make_float3(0.f, 0.f, 0.f);
+        bool on = slot >= 0;
+        uint32_t pix = 0;
+        if (on) {
+            const DistItem it = items[slot];
+            f.o = make_float3(it.o_magn.x, it.o_magn.y, it.o_magn.z);
+            f.magn = it.o_magn.w;
+            f.d = make_float3(it.d_level.x, it.d_level.y, it.d_level.z);
+            f.level = __float_as_int(it.d_level.w);
+            f.node = it.node.x;
+            pix = (uint32_t)it.node.y;
+            on = f.magn != kDistNoNode;
+        }
+        HitRecord h;
+        bool occ;
+        status |= traverse_warp<false>(sc, on, f.o, f.d, FLT_MAX, h, occ);
+        const bool hit = on && h.t < FLT_MAX;
+        float3 start, kd;
+        uint32_t kb = 0, nl = 0;
+        f.nrefl = f.nrefr = 0;
+        f.mat = 0;
+        if (hit) {
+            const int32_t id = h.id - sc.tri_base;
+            int32_t mi = sc.mat ? __ldg(&sc.mat[id]) : 0;
+            if (mi < 0 || mi >= table.n) { status |= kStatusBadIndex; mi = 0; }
+            const MaterialView &m = table.m[mi];
+            RayState r;
+            r.o = f.o;
+            r.d = f.d;
+            const SurfacePoint spt = surface_at(sc, r, h);
+            start = offset_start(spt.dst, spt.geo);
+            kd = material_kd(m, spt);
+            f.o = spt.dst;
+            f.sn = spt.sn;
+            f.geo = spt.geo;
+            f.mat = mi;
+            f.out_in = spt.out_in ? 1 : 0;
+            const int lvl = min(f.level, kDistLevels - 1);
+            for (int l = 0; l < lights.n; ++l) {
+                kb += (uint32_t)dl.draws[l][lvl];
+                nl += lights.l[l].kind == RT_LIGHT_DIRECTIONAL ? 1u : (uint32_t)dist_count(dp.soft, f.level);
+            }
+            dist_sets(f, m, dp, kb);
+        }
+        int cnt = f.nrefl + f.nrefr;
+        if (last && cnt > 0) {         // never expected: the tree's bound gives the levels
+            status |= kStatusStepLimit;
+            f.nrefl = f.nrefr = cnt = 0;
+        }
+        // the warp's children in lane order, one allocation
+        int sum = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, sum, o);
+            if ((int)lane >= o) sum += t;
+        }
+        int at = 0;
+        if (lane == 31u && sum) at = atomicAdd(&dc->made[level + 1], sum);
+        const int64_t child = (int64_t)next + __shfl_sync(0xffffffffu, at, 31) + sum - cnt;
+        const bool fits = cnt == 0 || child + cnt <= lists.pool;
+        if (cnt > 0) {
+            if (fits) {
+                const MaterialView &m = table.m[f.mat];
+                DistStream S = pixel_streams(dp, pix);
+                for (int j = 0; j < cnt; ++j) {
+                    const int set = j < f.nrefl ? 0 : 1;
+                    DistFrame C;
+                    spawn_child(f, m, dp, set, set ? j - f.nrefl : j, lut, S, status, C);
+                    DistItem it;
+                    it.o_magn = make_float4(C.o.x, C.o.y, C.o.z, C.magn);
+                    it.d_level = make_float4(C.d.x, C.d.y, C.d.z, __int_as_float(C.level));
+                    it.node = make_ulonglong2(C.node, (unsigned long long)pix);
+                    items[pool0 + (size_t)child + j] = it;
+                }
+            } else {
+                for (int64_t j = child; j < lists.pool; ++j)
+                    items[pool0 + (size_t)j].o_magn = make_float4(0.f, 0.f, 0.f, kDistNoNode);
+                over[atomicAdd(&dc->over, 1)] = slot;
+            }
+        }
+        // the hits, in lane order
+        const uint32_t hm = __ballot_sync(0xffffffffu, hit && fits);
+        int hat = 0;
+        if (lane == 0u && hm) hat = atomicAdd(&dc->hits, __popc(hm));
+        hat = __shfl_sync(0xffffffffu, hat, 0);
+        if (hit && fits) {
+            DistHit H;
+            H.start_slot = make_float4(start.x, start.y, start.z, __int_as_float(slot));
+            H.kd_mat = make_float4(kd.x, kd.y, kd.z, __int_as_float(f.mat));
+            H.sn = make_float4(f.sn.x, f.sn.y, f.sn.z, 0.f);
+            hits[hat + __popc(hm & ((1u << lane) - 1u))] = H;
+            nsec += nl;
+            drawn += kb;
+        }
+        if (slot >= 0) {
+            sets[slot] = cnt > 0 && fits ? make_int4(pool0 + (int)child, f.nrefl, f.nrefr, f.mat) : make_int4(0, 0, 0, 0);
+            if (on && !hit) item_c[slot] = make_float4(cam.background.x, cam.background.y, cam.background.z, 0.f);
+        }
+        if (on && fits) ++nsec;
+    }
+    warp_add(&ctr->secondary, nsec);
+    for (int o = 16; o > 0; o >>= 1) drawn += __shfl_xor_sync(0xffffffffu, drawn, o);
+    if (lane == 0u && drawn) atomicAdd(&ctr->drawn, drawn);
+    if (status) atomicOr(&ctr->status, status);
+}
+
+// The colour of every hit node from its lights and ka (the walk's sum).  A
+// warp has 32 hits; light by light it traces their rays 32 at a time in the
+// hits' order, so the rays of one hit, which leave one point for one light,
+// are neighbours (17.0 lanes an instruction; 11.0 with a ray of every hit at a
+// time), in step: 11.7 ms, 13.9 with a ray of every hit at a time.
+template <class SC>
+__global__ void __launch_bounds__(kTraceThreads, RT_DIST_LIGHTS_MIN_BLOCKS) k_dist_lights(
+    SC sc, LightSet lights, MaterialTable table, DistLights dl, DistParams dp, const int4 *__restrict__ area,
+    const float *__restrict__ verts, const float *__restrict__ lut, const DistItem *__restrict__ items,
+    const DistHit *__restrict__ hits, float4 *__restrict__ item_c, DistCounts *dc, Counters *ctr)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const int n = dc->hits;
+    uint32_t status = 0;
+    for (;;) {
+        const int base = warp_claim(&dc->work_lights, 32);
+        if (base >= n) break;
+        const bool on = base + (int)lane < n;
+        const DistHit H = hits[on ? base + (int)lane : base];
+        const int slot = __float_as_int(H.start_slot.w);
+        const DistItem it = items[slot];
+        const float3 start = make_float3(H.start_slot.x, H.start_slot.y, H.start_slot.z);
+        const float3 kd = make_float3(H.kd_mat.x, H.kd_mat.y, H.kd_mat.z);
+        const float3 sn = make_float3(H.sn.x, H.sn.y, H.sn.z);
+        const float3 d = make_float3(it.d_level.x, it.d_level.y, it.d_level.z);
+        const int level = __float_as_int(it.d_level.w), lvl = min(level, kDistLevels - 1);
+        const MaterialView &m = table.m[__float_as_int(H.kd_mat.w)];
+        uint32_t kb = 0;
+        float3 c = make_float3(0.f, 0.f, 0.f);
+        for (int l = 0; l < lights.n; ++l) {
+            const LightView &L = lights.l[l];
+            const int nl = L.kind == RT_LIGHT_DIRECTIONAL ? 1 : dist_count(dp.soft, level);
+            int end = on ? nl : 0;          // the hit's rays are [end - nl, end) of the warp's
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, end, o);
+                if ((int)lane >= o) end += t;
+            }
+            const int first = end - (on ? nl : 0), total = __shfl_sync(0xffffffffu, end, 31);
+            float3 ldir = d;
+            float len = 0.f;
+            int made = 0;
+            for (int at = 0; at < total; at += 32) {
+                const int r = at + (int)lane;
+                int own = 0;                // the hit of ray r: hits whose rays end at or before it
+                for (int o = 16; o > 0; o >>= 1)
+                    if (__shfl_sync(0xffffffffu, end, own + o - 1) <= r) own += o;
+                own = min(own, 31);
+                const bool ray = r < total;
+                const float3 rs = make_float3(__shfl_sync(0xffffffffu, start.x, own),
+                                              __shfl_sync(0xffffffffu, start.y, own),
+                                              __shfl_sync(0xffffffffu, start.z, own));
+                const uint64_t node = __shfl_sync(0xffffffffu, it.node.x, own);
+                const uint32_t pix = __shfl_sync(0xffffffffu, (uint32_t)it.node.y, own);
+                const int rl = __shfl_sync(0xffffffffu, lvl, own), rn = __shfl_sync(0xffffffffu, nl, own);
+                const int rfirst = __shfl_sync(0xffffffffu, first, own);
+                const uint32_t rkb = __shfl_sync(0xffffffffu, kb, own);
+                float3 di = rs;
+                float li = 0.f;
+                bool blocked;
+                if (ray) {
+                    DistStream S = pixel_streams(dp, pix);
+                    dist_light_ray(lights, dl, area, verts, sc.idx, lut, S, node, l, rl, rn, r - rfirst, rkb, rs, di,
+                                   li, status);
+                }
+                HitRecord sh;
+                status |= traverse_warp<true>(sc, ray, rs, di, li, sh, blocked);
+                const uint32_t lit = __ballot_sync(0xffffffffu, ray && !blocked);
+                const int lo = max(first - at, 0), hi = min(end - at, 32);   // the hit's lanes
+                if (lo < hi) made += __popc(lit & (0xffffffffu >> (32 - (hi - lo)) << lo));
+                const int from = (first - at) & 31;
+                const float3 d0 = make_float3(__shfl_sync(0xffffffffu, di.x, from), __shfl_sync(0xffffffffu, di.y, from),
+                                              __shfl_sync(0xffffffffu, di.z, from));
+                const float l0 = __shfl_sync(0xffffffffu, li, from);
+                if (first >= at && first < at + 32) {   // its first ray gives the direction and length
+                    ldir = d0;
+                    len = l0;
+                }
+            }
+            kb += (uint32_t)dl.draws[l][lvl];
+            if (on) phong_add<true>(L, m, kd, sn, d, ldir, len, xdiv((float)made, (float)nl), c);
+        }
+        if (on) {
+            c = xadd3(c, m.ka);
+            item_c[slot] = make_float4(c.x, c.y, c.z, 0.f);
+        }
+    }
+    if (status) atomicOr(&ctr->status, status);
+}
+
+// A set's mean colour times its weight, added to c.
+__device__ __forceinline__ float3 add_set(float3 c, const float4 *__restrict__ set, int n, float weight)
+{
+    if (!(weight > 0.0f) || n <= 0) return c;
+    float3 sum = make_float3(0.f, 0.f, 0.f);
+    for (int j = 0; j < n; ++j) {
+        const float4 q = set[j];
+        sum = xadd3(sum, make_float3(q.x, q.y, q.z));
+    }
+    return xadd3(c, xmul3(xdiv3(sum, (float)n), weight));
+}
+
+// The nodes of a level: their sets' means added times rf, then tran.
+__global__ void k_dist_gather(MaterialTable table, DistLists lists, int v0, int v1, int level,
+                              const int4 *__restrict__ sets, float4 *__restrict__ item_c, const DistCounts *dc)
+{
+    int first = v0, end = v1;
+    if (level > 0) dist_level(dc, lists.pool, level, first, end);
+    for (int v = first + blockIdx.x * blockDim.x + threadIdx.x; v < end; v += gridDim.x * blockDim.x) {
+        const int slot = level > 0 ? 2 * lists.cap + v : lists.slot(v);
+        if (slot < 0) continue;
+        const int4 s = sets[slot];
+        if (s.y + s.z == 0) continue;
+        const MaterialView &m = table.m[s.w];
+        const float4 q = item_c[slot];
+        float3 c = make_float3(q.x, q.y, q.z);
+        c = add_set(c, item_c + s.x, s.y, m.rf);
+        c = add_set(c, item_c + s.x + s.y, s.z, m.tran);
+        item_c[slot] = make_float4(c.x, c.y, c.z, 0.f);
+    }
+}
+
+// The subtrees of the items, or of the nodes of `list`, one per lane; a warp
+// takes 32 consecutive ones (the rays of one or two sets) at a time.  (Lanes
+// that take the next item as soon as theirs is finished were measured slower:
+// 61 against 41 ms on the 512x512 glass frame with 16-ray diffuse sets, their
+// rays no longer neighbours.)
 // 6 resident blocks (80 registers): 34.1 ms against 41.3 at 4 and 37.1 at 5
 // on the 512x512 glass frame with 16-ray diffuse sets; 7 and 8 no faster
 #ifndef RT_DIST_SUB_MIN_BLOCKS
@@ -1166,21 +1497,18 @@ template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_DIST_SUB_MIN_BLOCKS) k_dist_sub(
     SC sc, CameraView cam, LightSet lights, MaterialTable table, DistLights dl, DistParams dp,
     const int4 *__restrict__ area, const float *__restrict__ verts, const float *__restrict__ lut,
-    const DistItem *__restrict__ items, int32_t nr, int32_t nt, int32_t cap, float4 *__restrict__ item_c,
-    Counters *ctr)
+    const DistItem *__restrict__ items, DistLists lists, const int32_t *__restrict__ list,
+    const int32_t *__restrict__ nlist, int32_t *work, float4 *__restrict__ item_c, Counters *ctr)
 {
     DistFrame F[kDistDepth];
     const uint32_t lane = threadIdx.x & 31u;
-    // the reflection list's items, then (from a warp boundary on) the
-    // refraction list's
-    const int rw = (nr + 31) & ~31;
-    const int n = rw + nt;
+    const int n = list ? *nlist : lists.count();
     uint32_t status = 0;
     for (;;) {
-        const int base = warp_claim(&ctr->work, 32);
+        const int base = warp_claim(work, 32);
         if (base >= n) break;
         const int v = base + (int)lane;
-        const int i = v < rw ? (v < nr ? v : -1) : (v - rw < nt ? cap + (v - rw) : -1);
+        const int i = list ? (v < n ? list[v] : -1) : lists.slot(v);
         uint32_t nsec = 0, drawn = 0;
         if (i >= 0) {
             const DistItem it = items[i];
@@ -1223,18 +1551,8 @@ __global__ void k_dist_combine(CameraView cam, MaterialTable table, const float4
                 status |= kStatusBadIndex;
             } else {
                 const MaterialView &m = table.m[__float_as_int(r.w)];
-                float3 sum = make_float3(0.f, 0.f, 0.f);
-                for (int j = 0; j < sets.y; ++j) {
-                    const float4 q = item_c[sets.x + j];
-                    sum = xadd3(sum, make_float3(q.x, q.y, q.z));
-                }
-                if (m.rf > 0.0f && sets.y > 0) c = xadd3(c, xmul3(xdiv3(sum, (float)sets.y), m.rf));
-                sum = make_float3(0.f, 0.f, 0.f);
-                for (int j = 0; j < sets.w; ++j) {
-                    const float4 q = item_c[(size_t)cap + sets.z + j];
-                    sum = xadd3(sum, make_float3(q.x, q.y, q.z));
-                }
-                if (m.tran > 0.0f && sets.w > 0) c = xadd3(c, xmul3(xdiv3(sum, (float)sets.w), m.tran));
+                c = add_set(c, item_c + sets.x, sets.y, m.rf);
+                c = add_set(c, item_c + (size_t)cap + sets.z, sets.w, m.tran);
             }
         }
         if (rgb) store_rgb(rgb, (size_t)p, c);
@@ -1471,17 +1789,35 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
 
 namespace {
 
+template <class K>
+int resident_blocks(K kernel, int otherwise)
+{
+    int b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kTraceThreads, 0) != cudaSuccess || b < 1) {
+        cudaGetLastError();
+        b = otherwise;
+    }
+    return b;
+}
+
 template <class SC>
 int sub_blocks_per_sm()
 {
-    static const int per_sm = [] {
-        int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_dist_sub<SC>, kTraceThreads, 0) != cudaSuccess || b < 1) {
-            cudaGetLastError();
-            b = 2;
-        }
-        return b;
-    }();
+    static const int per_sm = resident_blocks(k_dist_sub<SC>, 2);
+    return per_sm;
+}
+
+template <class SC>
+int node_blocks_per_sm()
+{
+    static const int per_sm = resident_blocks(k_dist_node<SC>, 2);
+    return per_sm;
+}
+
+template <class SC>
+int light_blocks_per_sm()
+{
+    static const int per_sm = resident_blocks(k_dist_lights<SC>, 2);
     return per_sm;
 }
 
@@ -1739,6 +2075,57 @@ rt_status stream_used(SoftState &S, cudaStream_t st)
     return RT_OK;
 }
 
+// The subtrees of a frame's items (on the device already): a piece of at most
+// kDistPiece items at a time, level by level, the nodes below them in a pool
+// of up to kDistPoolPerItem for each.
+constexpr int32_t kDistPiece = 1 << 22;
+constexpr int32_t kDistPoolPerItem = 4;
+
+rt_status trace_items(SoftState &S, rt_scene *s, const CameraView &cv, const LightSet &ls, const MaterialTable &mt,
+                      const DistLights &dl, const DistParams &dp, const SceneView &sv, DistLists lists, int levels,
+                      rt_context *ctx, cudaStream_t st)
+{
+    const int32_t n = lists.count(), piece = std::min(n, kDistPiece);
+    DistCounts *dc = (DistCounts *)((int32_t *)S.nitems.ptr + 2);
+    DistItem *items = (DistItem *)S.items.ptr;
+    float4 *item_c = (float4 *)S.item_c.ptr;
+    const size_t entries = 2 * (size_t)lists.cap + (size_t)lists.pool;
+    const size_t nodes = (size_t)piece + (size_t)lists.pool;   // of a piece, at most
+    const int4 *area = (const int4 *)S.area.ptr;
+    const float *lut = (const float *)S.lut.ptr;
+    // without room for the lists the items are walked whole
+    const bool walk = S.node_sets.reserve(entries * sizeof(int4)) != cudaSuccess ||
+                      S.node_hits.reserve(nodes * sizeof(DistHit)) != cudaSuccess ||
+                      S.node_over.reserve(nodes * sizeof(int32_t)) != cudaSuccess;
+    if (walk) cudaGetLastError();
+    int4 *sets = (int4 *)S.node_sets.ptr;
+    DistHit *hits = (DistHit *)S.node_hits.ptr;
+    int32_t *over = (int32_t *)S.node_over.ptr;
+    for (int64_t at = 0; at < n; at += walk ? n : piece) {
+        const int32_t v0 = (int32_t)at, v1 = (int32_t)std::min<int64_t>(n, at + piece);
+        RT_CUDA_S(cudaMemsetAsync(dc, 0, sizeof(DistCounts), st), "node counter clear");
+        with_scene(sv, [&](const auto &view) {
+            using SC = std::decay_t<decltype(view)>;
+            if (!walk) {
+                for (int k = 0; k < levels; ++k)
+                    k_dist_node<SC><<<node_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
+                        view, cv, ls, mt, dl, dp, lut, items, lists, v0, v1, k, k == levels - 1, sets, item_c, hits,
+                        over, dc, ctx->d_counters);
+                k_dist_lights<SC><<<light_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
+                    view, ls, mt, dl, dp, area, s->d_verts, lut, items, hits, item_c, dc, ctx->d_counters);
+            }
+            k_dist_sub<SC><<<sub_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
+                view, cv, ls, mt, dl, dp, area, s->d_verts, lut, items, lists, walk ? nullptr : over, &dc->over,
+                &dc->work_over, item_c, ctx->d_counters);
+            if (!walk)
+                for (int k = levels - 1; k-- > 0;)
+                    k_dist_gather<<<ctx->sm_count * 8, 256, 0, st>>>(mt, lists, v0, v1, k, sets, item_c, dc);
+        });
+        RT_CUDA_S(cudaGetLastError(), "subtree launch");
+    }
+    return RT_OK;
+}
+
 }  // namespace
 
 extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera, const rt_light *lights,
@@ -1927,13 +2314,22 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
     if (split) {
         RT_CUDA_S(S.root_c.reserve(npix * sizeof(float4)), "node allocation");
         RT_CUDA_S(S.root_sets.reserve(npix * sizeof(int4)), "node allocation");
-        RT_CUDA_S(S.nitems.reserve(2 * sizeof(int32_t)), "item counter allocation");
+        RT_CUDA_S(S.nitems.reserve(2 * sizeof(int32_t) + sizeof(DistCounts)), "item counter allocation");
         // items per list (reflection sets, refraction sets)
         int64_t cap = std::min((int64_t)npix * per_pixel / 2, std::max(S.item_cap, (int64_t)npix * 2));
+        int64_t pool = 0;
         int32_t n[2] = {0, 0};
         for (int attempt = 0; attempt < 2; ++attempt) {
-            RT_CUDA_S(S.items.reserve(2 * (size_t)cap * sizeof(DistItem)), "item allocation");
-            RT_CUDA_S(S.item_c.reserve(2 * (size_t)cap * sizeof(float4)), "item colour allocation");
+            // room for the nodes below the items where it can be had
+            pool = std::min({kDistPoolPerItem * 2 * cap, (int64_t)kDistPoolPerItem * kDistPiece,
+                             ((int64_t)1 << 31) - 1 - 2 * cap});
+            if (S.items.reserve((2 * (size_t)cap + (size_t)pool) * sizeof(DistItem)) != cudaSuccess ||
+                S.item_c.reserve((2 * (size_t)cap + (size_t)pool) * sizeof(float4)) != cudaSuccess) {
+                cudaGetLastError();
+                pool = 0;
+                RT_CUDA_S(S.items.reserve(2 * (size_t)cap * sizeof(DistItem)), "item allocation");
+                RT_CUDA_S(S.item_c.reserve(2 * (size_t)cap * sizeof(float4)), "item colour allocation");
+            }
             RT_CUDA_S(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), st), "counter clear");
             RT_CUDA_S(cudaMemsetAsync(S.nitems.ptr, 0, 2 * sizeof(int32_t), st), "item counter clear");
             with_scene(sv, [&](const auto &view) {
@@ -1954,15 +2350,11 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
             cap = std::min((int64_t)npix * per_pixel / 2, need + need / 8);   // grow to fit and run again
         }
         S.item_cap = cap;
-        RT_CUDA_S(cudaMemsetAsync(&ctx->d_counters->work, 0, sizeof(int), st), "work counter clear");
-        if (n[0] + n[1] > 0)
-            with_scene(sv, [&](const auto &view) {
-                using SC = std::decay_t<decltype(view)>;
-                k_dist_sub<SC><<<sub_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
-                    view, cv, ls, mt, dl, dp, (const int4 *)S.area.ptr, s->d_verts, (const float *)S.lut.ptr,
-                    (const DistItem *)S.items.ptr, n[0], n[1], (int32_t)cap, (float4 *)S.item_c.ptr, ctx->d_counters);
-            });
-        RT_CUDA_S(cudaGetLastError(), "subtree launch");
+        if (n[0] + n[1] > 0) {
+            const rt_status wst = trace_items(S, s, cv, ls, mt, dl, dp, sv, DistLists{n[0], n[1], (int32_t)cap, (int32_t)pool},
+                                              std::max(tb.depth, 1), ctx, st);
+            if (wst != RT_OK) return wst;
+        }
         k_dist_combine<<<ctx->sm_count * 8, 256, 0, st>>>(cv, mt, (const float4 *)S.root_c.ptr,
                                                           (const int4 *)S.root_sets.ptr, (const float4 *)S.item_c.ptr,
                                                           n[0], n[1], (int32_t)cap, d_rgb, d_f, ctx->d_counters);
