@@ -161,6 +161,7 @@ SceneView scene_view(const rt_scene *s)
 {
     SceneView v;
     v.nodes = s->d_nodes;
+    v.any_nodes = s->any_ready ? (const WideNode *)s->any.ptr : s->d_nodes;
     v.tris = s->d_tris;
     v.shade = s->d_shade;
     v.idx = s->d_idx;
@@ -353,6 +354,8 @@ static void scene_free_geometry(rt_scene *s)
     cudaFree(s->d_nodes); s->d_nodes = nullptr;
     cudaFree(s->d_tris); s->d_tris = nullptr;
     s->temp.release();
+    s->any.release();
+    s->any_ready = s->passing = false;
     s->built = false;
     s->nnodes = s->tri_slots = s->depth = 0;
 }
@@ -404,12 +407,18 @@ rt_status rt_scene_upload(rt_scene *s, const float *verts, int32_t nverts, const
             RT_CUDA(cudaMemcpyAsync(s->d_vattr, vattr, (size_t)nverts * 3 * sizeof(float), cudaMemcpyDefault,
                                     ctx->stream), "attribute copy");
     }
-    if (flags && ntris > 0)
+    ctx->h_scratch[0] = 0;
+    if (flags && ntris > 0) {
         RT_CUDA(cudaMemcpyAsync(s->d_flags, flags, (size_t)ntris * sizeof(uint32_t), cudaMemcpyDefault, ctx->stream),
                 "flag copy");
-    else
+        find_passing(s->d_flags, ntris, (int32_t *)&ctx->d_counters->work, ctx->stream);
+        RT_CUDA(cudaMemcpyAsync(ctx->h_scratch, &ctx->d_counters->work, sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                ctx->stream), "flag test read");
+    } else {
         RT_CUDA(cudaMemsetAsync(s->d_flags, 0, nt * sizeof(uint32_t), ctx->stream), "flag clear");
+    }
     RT_CUDA(cudaStreamSynchronize(ctx->stream), "upload synchronize");
+    s->passing = ctx->h_scratch[0] != 0;
     return RT_OK;
 }
 
@@ -430,12 +439,28 @@ static int32_t builder_of(int b)
     return b == RT_BUILDER_LBVH ? kBuilderLbvh : b == RT_BUILDER_HPLOC ? kBuilderHploc : kBuilderPloc;
 }
 
+// The any-hit rays' nodes of a scene that has triangles they pass, after its
+// hierarchy was built (mark) or refitted; without memory for them the rays
+// take the scene's own nodes.
+static void make_any_nodes(rt_scene *s, int32_t nnodes, bool mark)
+{
+    if (!s->passing || nnodes < 1) return;
+    const size_t n = (size_t)nnodes;
+    if (mark && s->any.reserve(n * (sizeof(WideNode) + 2 * sizeof(int32_t))) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    build_any_nodes(s->d_nodes, nnodes, s->d_tris, (WideNode *)s->any.ptr,
+                    (int32_t *)((WideNode *)s->any.ptr + n), mark, s->ctx->stream);
+    s->any_ready = true;
+}
+
 rt_status rt_bvh_build(rt_scene *s, float *build_ms)
 {
     if (!s) return fail(RT_ERR_INVALID_ARG, "rt_bvh_build: NULL scene");
     rt_context *ctx = s->ctx;
     DeviceGuard g(ctx->device);
-    s->built = false;
+    s->built = s->any_ready = false;
     s->refit = RefitArrays();
     if (build_ms) *build_ms = 0.f;
     if (s->ntris == 0) {
@@ -469,6 +494,7 @@ rt_status rt_bvh_build(rt_scene *s, float *build_ms)
         if (R.status == RT_ERR_STACK_OVERFLOW) return fail(RT_ERR_STACK_OVERFLOW, "bvh build: tree deeper than the traversal stack");
         return fail(R.status, "bvh build failed");
     }
+    make_any_nodes(s, R.nodes, true);
     RT_CUDA(cudaEventRecord(ctx->ev1, ctx->stream), "event record");
     RT_CUDA(cudaEventSynchronize(ctx->ev1), "event synchronize");
     RT_CUDA(cudaGetLastError(), "bvh build kernels");
@@ -506,6 +532,7 @@ rt_status rt_scene_refit_vertices(rt_scene *s, const float *verts, int32_t nvert
         if (e != cudaSuccess) return cuda_fail(e, "refit");
         return fail(st, "rt_scene_refit_vertices: refit failed");
     }
+    if (s->any_ready) make_any_nodes(s, s->nnodes, false);
     RT_CUDA(cudaEventRecord(ctx->ev1, ctx->stream), "event record");
     RT_CUDA(cudaEventSynchronize(ctx->ev1), "event synchronize");
     if (refit_ms) cudaEventElapsedTime(refit_ms, ctx->ev0, ctx->ev1);

@@ -406,7 +406,7 @@ rt_status rt_bvh_build_batched(rt_batch *b, float *build_ms)
     // refresh scene views of already-set jobs
     for (auto &j : b->h_jobs) {
         const int s = j.sc.root;
-        j.sc.nodes = b->d_nodes; j.sc.tris = b->d_tris; j.sc.shade = b->d_shade; j.sc.idx = b->d_idx;
+        j.sc.nodes = j.sc.any_nodes = b->d_nodes; j.sc.tris = b->d_tris; j.sc.shade = b->d_shade; j.sc.idx = b->d_idx;
         j.sc.vattr = b->has_attr[s] ? b->d_vattr : nullptr; j.sc.flags = b->d_flags;
         j.sc.ntris = ntris; j.sc.nnodes = b->nnodes; j.sc.tri_base = b->tri_off[s]; j.sc.isect = b->ctx->isect;
     }
@@ -439,7 +439,7 @@ rt_status rt_batch_set_jobs(rt_batch *b, const rt_job *jobs, int32_t njobs)
         BatchJob B;
         memset(&B, 0, sizeof(B));
         const int s = J.scene;
-        B.sc.nodes = b->d_nodes; B.sc.tris = b->d_tris; B.sc.shade = b->d_shade; B.sc.idx = b->d_idx;
+        B.sc.nodes = B.sc.any_nodes = b->d_nodes; B.sc.tris = b->d_tris; B.sc.shade = b->d_shade; B.sc.idx = b->d_idx;
         B.sc.vattr = b->has_attr[s] ? b->d_vattr : nullptr;
         B.sc.flags = b->d_flags;
         B.sc.ntris = (int32_t)(b->h_idx.size() / 3);

@@ -2093,6 +2093,97 @@ __global__ void k_repack(PackedTri *__restrict__ tris, int32_t nslots, const flo
 
 }  // namespace
 
+namespace {
+
+constexpr uint32_t kPassing = RT_TRI_LIGHT | RT_TRI_TRANSPARENT;
+
+// Any-hit rays in scenes with triangles that stop none of them spend most of
+// their node tests on such triangles: a ray that leaves a glass sphere meets
+// the sphere's own nodes first.  They take a copy of the nodes in which
+// children with nothing else below are empty; it costs no instruction in the
+// traversal (another node pointer), 88 bytes a node and three short kernels a
+// build, only in scenes that have such triangles.  512x512 glass frames: ray
+// trees 649 -> 436 us, diffuse sets 18.65 -> 12.04 ms.
+
+// Do any of n triangles stop no any-hit ray?
+__global__ void k_find_passing(const uint32_t *__restrict__ flags, int32_t n, int32_t *__restrict__ out)
+{
+    uint32_t f = 0u;
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) f |= flags[i];
+    if (__any_sync(0xffffffffu, (f & kPassing) != 0u) && (threadIdx.x & 31u) == 0u) *out = 1;
+}
+
+__device__ __forceinline__ bool leaf_stops(const WideNode &N, int s, const PackedTri *__restrict__ tris)
+{
+    const PackedTri *t = tris + N.tri_base + (N.meta[s] & 31u);
+    for (int k = 0; k < (N.meta[s] >> 5); ++k)
+        if ((__float_as_uint(t[k].w2.z) & kPassing) == 0u) return true;
+    return false;
+}
+
+__global__ void k_any_parents(const WideNode *__restrict__ nodes, int32_t n, int32_t *__restrict__ parent,
+                              int32_t *__restrict__ stops)
+{
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int32_t first = (int32_t)nodes[i].child_base, kids = __popc(nodes[i].imask);
+    for (int32_t c = first; c < first + kids; ++c)
+        if (c < n) parent[c] = i;
+    if (i == 0) parent[0] = -1;
+    stops[i] = 0;
+}
+
+// A node with a triangle that stops rays marks itself and the nodes above it,
+// up to the first that is marked already.
+__global__ void k_any_marks(const WideNode *__restrict__ nodes, int32_t n, const PackedTri *__restrict__ tris,
+                            const int32_t *__restrict__ parent, int32_t *__restrict__ stops)
+{
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const WideNode N = nodes[i];
+    bool stop = false;
+    for (int s = 0; s < 8 && !stop; ++s) stop = N.meta[s] != 0 && N.meta[s] != 0x80u && leaf_stops(N, s, tris);
+    int32_t at = stop ? i : -1;
+    for (int step = 0; at >= 0 && step < kRefitMaxDepth && atomicExch(stops + at, 1) == 0; ++step) at = parent[at];
+}
+
+__global__ void k_any_nodes(const WideNode *__restrict__ nodes, int32_t n, const PackedTri *__restrict__ tris,
+                            const int32_t *__restrict__ stops, WideNode *__restrict__ out)
+{
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    WideNode N = nodes[i];
+    int32_t child = (int32_t)N.child_base;
+    for (int s = 0; s < 8; ++s) {
+        if ((N.imask >> s) & 1u) {
+            if (child >= n || !stops[child]) N.meta[s] = 0;
+            ++child;
+        } else if (N.meta[s] != 0 && !leaf_stops(N, s, tris)) {
+            N.meta[s] = 0;
+        }
+    }
+    out[i] = N;
+}
+
+}  // namespace
+
+void find_passing(const uint32_t *flags, int32_t n, int32_t *out, cudaStream_t st)
+{
+    cudaMemsetAsync(out, 0, sizeof(int32_t), st);
+    if (n > 0) k_find_passing<<<std::min((n + 255) / 256, 1024), 256, 0, st>>>(flags, n, out);
+}
+
+void build_any_nodes(const WideNode *nodes, int32_t n, const PackedTri *tris, WideNode *any_nodes, int32_t *scratch,
+                     bool mark, cudaStream_t st)
+{
+    const int g = (n + 127) / 128;
+    if (mark) {
+        k_any_parents<<<g, 128, 0, st>>>(nodes, n, scratch, scratch + n);
+        k_any_marks<<<g, 128, 0, st>>>(nodes, n, tris, scratch, scratch + n);
+    }
+    k_any_nodes<<<g, 128, 0, st>>>(nodes, n, tris, scratch + n, any_nodes);
+}
+
 int32_t refit_wide_bvh(const RefitArrays &K, const float *verts, const int3 *idx, ShadeTri *shade, WideNode *nodes,
                        PackedTri *tris, int32_t *host_scratch, cudaStream_t st)
 {

@@ -63,6 +63,15 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
 // moved vertices: shading records, boxes bottom-up, every wide node
 // re-quantised, packed triangles rewritten; topology kept.  0 or an
 // rt_status code.  Synchronises st once.
+// The any-hit rays' copy of a scene's nodes (any_nodes), for scenes with
+// triangles that stop none of them (light and transparent ones): children
+// with nothing else below are left out.  mark: n nodes' marks are made again
+// (a new hierarchy), else kept (a refit).  scratch: 2 n ints.
+void build_any_nodes(const WideNode *nodes, int32_t n, const PackedTri *tris, WideNode *any_nodes, int32_t *scratch,
+                     bool mark, cudaStream_t st);
+// Sets *out to 1 where one of n triangles' flags is a light's or transparent.
+void find_passing(const uint32_t *flags, int32_t n, int32_t *out, cudaStream_t st);
+
 int32_t refit_wide_bvh(const RefitArrays &K, const float *verts, const int3 *idx, ShadeTri *shade, WideNode *nodes,
                        PackedTri *tris, int32_t *host_scratch, cudaStream_t st);
 

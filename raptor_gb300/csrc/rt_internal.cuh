@@ -59,6 +59,7 @@ struct __align__(16) ShadeTri {
 struct SceneView {
     static constexpr bool kWatertight = false;
     const WideNode *nodes;
+    const WideNode *any_nodes;   // for any-hit rays: nodes, or a copy without the children no ray stops at
     const PackedTri *tris;
     const ShadeTri *shade;
     const int3 *idx;          // vertex indices per triangle (caller's order)

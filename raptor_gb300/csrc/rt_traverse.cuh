@@ -377,7 +377,7 @@ __device__ __forceinline__ bool trav_step(Trav &T, uint2 *stack, const SceneView
             if (T.sp >= STACK) { status |= kStatusStackOverflow; return true; }
             stack[T.sp++] = T.ngroup;
         }
-        const NodeHits nh = intersect_node(sc.nodes, idx, T.o, T.inv, T.w0, T.w1, T.box_tmax);
+        const NodeHits nh = intersect_node(any ? sc.any_nodes : sc.nodes, idx, T.o, T.inv, T.w0, T.w1, T.box_tmax);
         if (COUNT) ++fc->nodes;
         T.ngroup = nh.ngroup;
         tri_base = nh.tri_base;
@@ -532,7 +532,7 @@ __device__ __forceinline__ uint32_t traverse_warp(const SC &sc, bool live, const
                 sp = 0;
             } else {
                 if (push) stack[sp++] = group;
-                const NodeHits nh = intersect_node(sc.nodes, idx, o, inv, w0, w1, best);
+                const NodeHits nh = intersect_node(ANY ? sc.any_nodes : sc.nodes, idx, o, inv, w0, w1, best);
                 if (COUNT) ++fc->nodes;
                 group = nh.ngroup;
                 if (nh.leaf_slots) {
