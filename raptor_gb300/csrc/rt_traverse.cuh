@@ -444,6 +444,49 @@ __device__ __forceinline__ uint32_t traverse(const SC &sc, const float3 o, const
     return traverse_ray<COUNT, STACK>(sc, o, d, tmax, ANY, hit, occluded, fc);
 }
 
+// Traversal of a list of rays by a warp whose lanes take further rays once
+// kIdle of them are idle (4 and 16 were slower), every lane calling it, converged.
+// claim(want, base): up to `want` further rays, base on, the same for all lanes;
+// 0: none are left.  fetch(take, k, o, d, tmax): ray k, for the lanes with take
+// set.  done(k, trav): its result, lane by lane.
+constexpr int kIdle = 8;
+template <bool ANY, class SC, class Claim, class Fetch, class Done>
+__device__ __forceinline__ uint32_t traverse_list(const SC &sc, Claim claim, Fetch fetch, Done done)
+{
+    const uint32_t full = 0xffffffffu, below = (1u << (threadIdx.x & 31u)) - 1u;
+    uint2 stack[kStackSize];
+    Trav T;
+    int ray = -1;
+    int refill = kIdle;   // 32 once no rays are left
+    uint32_t status = 0u;
+    for (;;) {
+        const uint32_t idle = __ballot_sync(full, ray < 0);
+        if (__popc(idle) >= refill) {
+            int base = 0;
+            const int got = claim(__popc(idle), base);
+            if (got == 0) {
+                if (idle == full) break;
+                refill = 32;
+                continue;
+            }
+            const int rank = __popc(idle & below);
+            const bool take = ray < 0 && rank < got;
+            float3 o, d;
+            float tmax;
+            fetch(take, base + rank, o, d, tmax);
+            if (take) {
+                ray = base + rank;
+                trav_begin(T, sc, o, d, tmax, ANY);
+            }
+        }
+        if (ray >= 0 && trav_step<false, SC::kWatertight>(T, stack, sc, ANY, status, nullptr)) {
+            done(ray, T);
+            ray = -1;
+        }
+    }
+    return status;
+}
+
 // Traversal of a warp's rays in step, for rays that take similar paths (every
 // lane of the warp calls it, converged; live: the lane has a ray).  In
 // traverse a warp tests triangles after every node for the few lanes that met
