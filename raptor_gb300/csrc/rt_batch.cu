@@ -28,17 +28,23 @@ namespace {
 
 // STACK: traversal stack capacity in node groups, chosen by the autotuner
 // among the capacities that hold the batch's deepest tree.
-template <int TW, int STACK, class SC>
+// AO: the kind of the jobs, whose tiles are items [first, end), claimed from
+// *work.  A kernel for each kind: one for both kept both paths' registers (64,
+// 436 bytes spilled).  Side by side in the graph, as blocks of one leave those
+// of the other start.  24 scenes: 2.60 -> 2.39 ms; the AO rays of a tile spread
+// over its lanes, as k_render_ao has them, gave 0.4 % more.
+template <bool AO, int TW, int STACK, class SC>
 __global__ void __launch_bounds__(256, RT_RENDER_MIN_BLOCKS / 2) k_render_batched(const BatchJob *__restrict__ jobs, int32_t njobs,
-                                                        int32_t total_items, int32_t chunk, Counters *ctr)
+                                                        int32_t first, int32_t end, int32_t chunk, int *work,
+                                                        Counters *ctr)
 {
     uint32_t status = 0;
     for (;;) {
-        const int base = warp_claim(&ctr->work, 32 * chunk);
-        if (base >= total_items) break;
+        const int base = first + warp_claim(work, 32 * chunk);
+        if (base >= end) break;
         for (int c = 0; c < chunk; ++c) {
             const int item0 = base + 32 * c;
-            if (item0 >= total_items) break;
+            if (item0 >= end) break;
             // job owning this tile: last job with items_begin <= item0 (warp-uniform)
             int lo = 0, hi = njobs - 1;
             while (lo < hi) {
@@ -53,10 +59,9 @@ __global__ void __launch_bounds__(256, RT_RENDER_MIN_BLOCKS / 2) k_render_batche
             PixelOut po;
             po.hit = false;
             po.secondary = 0;
-            // not in step: the kernel holds the AO path too, and in step it
-            // lost (24 scenes: 2.60 -> 2.77 ms)
+            // the rays one by one: in step this kernel lost (2.39 -> 2.51 ms)
             if (live) {
-                if (J.mode == RT_JOB_AO)
+                if (AO)
                     po = shade_pixel_ao<false, STACK>(sc, J.cam, J.mat, J.ao_samples, J.ao_dist, J.ao_seed, x, y,
                                                       status, nullptr);
                 else
@@ -96,7 +101,7 @@ int grid_for(int kernel, int threads, int sm_count)
     cudaError_t e = (kernel == RT_KERNEL_WAVE)
                         ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (k_render_batched_wave<TW, SC>), threads,
                                                                         threads * sizeof(LaneShade))
-                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (k_render_batched<TW, STACK, SC>), threads,
+                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (k_render_batched<false, TW, STACK, SC>), threads,
                                                                         0);
     if (e != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
@@ -131,6 +136,7 @@ struct rt_batch {
     std::vector<BatchJob> h_jobs;
     BatchJob *d_jobs = nullptr;
     int32_t total_items = 0;
+    int32_t light_jobs = 0, light_items = 0;   // the shadow-ray jobs and their items come first
     // launch configuration and its captured graph
     rt_tune_config cfg{128, 1, 8, RT_KERNEL_PIXEL, 0.f, kStackSize};
     cudaGraphExec_t exec = nullptr;
@@ -171,7 +177,7 @@ int32_t nscenes(const rt_batch *b) { return (int32_t)b->tri_off.size() - 1; }
 
 // Launch one batch frame directly (the body captured into the graph).
 template <class SC>
-void launch_batch(rt_batch *b, cudaStream_t st, int grid)
+void launch_batch(rt_batch *b, cudaStream_t st, cudaStream_t st2, cudaEvent_t fork, cudaEvent_t join, int grid)
 {
     cudaMemsetAsync(b->ctx->d_counters, 0, sizeof(Counters), st);
     const int threads = b->cfg.block_threads;
@@ -186,7 +192,20 @@ void launch_batch(rt_batch *b, cudaStream_t st, int grid)
     } else {
         Counters *ctr = b->ctx->d_counters;
         const int stack = b->cfg.stack_entries;
-#define RT_BATCH_PIXEL(TW, S) k_render_batched<TW, S, SC><<<grid, threads, 0, st>>>(b->d_jobs, nj, b->total_items, chunk, ctr)
+        const int lj = b->light_jobs, li = b->light_items;
+        // the two kinds of jobs, side by side
+#define RT_BATCH_PIXEL(TW, S)                                                                                        \
+    do {                                                                                                             \
+        if (lj > 0)                                                                                                  \
+            k_render_batched<false, TW, S, SC><<<grid, threads, 0, st>>>(b->d_jobs, lj, 0, li, chunk, &ctr->work, ctr); \
+        if (nj > lj)                                                                                                 \
+            k_render_batched<true, TW, S, SC><<<grid, threads, 0, lj > 0 ? st2 : st>>>(                              \
+                b->d_jobs + lj, nj - lj, li, b->total_items, chunk, &ctr->redo, ctr);                                \
+    } while (0)
+        if (lj > 0 && nj > lj) {
+            cudaEventRecord(fork, st);
+            cudaStreamWaitEvent(st2, fork, 0);
+        }
         if (b->cfg.tile_w == 16) {
             if (stack == kBatchStacks[0]) RT_BATCH_PIXEL(16, kBatchStacks[0]);
             else if (stack == kBatchStacks[1]) RT_BATCH_PIXEL(16, kBatchStacks[1]);
@@ -195,6 +214,10 @@ void launch_batch(rt_batch *b, cudaStream_t st, int grid)
             if (stack == kBatchStacks[0]) RT_BATCH_PIXEL(8, kBatchStacks[0]);
             else if (stack == kBatchStacks[1]) RT_BATCH_PIXEL(8, kBatchStacks[1]);
             else RT_BATCH_PIXEL(8, kBatchStacks[2]);
+        }
+        if (lj > 0 && nj > lj) {
+            cudaEventRecord(join, st2);
+            cudaStreamWaitEvent(st, join, 0);
         }
 #undef RT_BATCH_PIXEL
     }
@@ -221,16 +244,30 @@ rt_status make_graph(rt_batch *b)
     drop_graph(b);
     cudaStream_t st = b->ctx->stream;
     cudaGraph_t g = nullptr;
-    cudaError_t e = cudaSuccess;
+    // a second branch of the graph; the stream and events are needed while it is captured
+    cudaStream_t st2 = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+    const auto drop = [&] {
+        if (join) cudaEventDestroy(join);
+        if (fork) cudaEventDestroy(fork);
+        if (st2) cudaStreamDestroy(st2);
+    };
+    if (e != cudaSuccess) {
+        drop();
+        return set_cuda_error(e, "graph capture streams");
+    }
     // every job's scene carries the intersector set when the jobs were
     with_scene(b->h_jobs.empty() ? SceneView{} : b->h_jobs[0].sc, [&](const auto &view) {
         using SC = std::decay_t<decltype(view)>;
         const int grid = batch_grid<SC>(b);
         e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) launch_batch<SC>(b, st, grid);
+        if (e == cudaSuccess) launch_batch<SC>(b, st, st2, fork, join, grid);
     });
-    RT_CUDA_B(e, "graph capture begin");
-    e = cudaStreamEndCapture(st, &g);
+    if (e == cudaSuccess) e = cudaStreamEndCapture(st, &g);
+    drop();
     if (e != cudaSuccess) return set_cuda_error(e, "graph capture end");
     e = cudaGraphInstantiate(&b->exec, g, 0);
     cudaGraphDestroy(g);
@@ -246,7 +283,11 @@ rt_status make_graph(rt_batch *b)
 rt_status layout_jobs(rt_batch *b)
 {
     int32_t items = 0;
-    for (auto &j : b->h_jobs) {
+    std::vector<BatchJob> &jobs = b->h_jobs;   // the kinds apart, else in their order
+    const auto ao = std::stable_partition(jobs.begin(), jobs.end(), [](const BatchJob &j) { return j.mode != RT_JOB_AO; });
+    b->light_jobs = (int32_t)(ao - jobs.begin());
+    b->light_items = 0;
+    for (auto &j : jobs) {
         int tx;
         const int tiles = (b->cfg.tile_w == 16) ? tiles_of<16>(j.cam.xres, j.cam.yres, tx)
                                                  : tiles_of<8>(j.cam.xres, j.cam.yres, tx);
@@ -255,6 +296,7 @@ rt_status layout_jobs(rt_batch *b)
         if ((int64_t)items + (int64_t)tiles * 32 > INT32_MAX) return bfail(RT_ERR_INVALID_ARG, "batch too large");
         items += tiles * 32;
         j.items_end = items;
+        if (j.mode != RT_JOB_AO) b->light_items = items;
     }
     b->total_items = items;
     cudaFree(b->d_jobs);
