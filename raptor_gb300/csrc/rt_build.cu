@@ -406,6 +406,23 @@ constexpr int kPlocTile = 256;
 constexpr int kPlocBlock = 1024;
 enum : int { kStCount = 0, kStBase = 2, kStForced = 4, kStTarget = 6, kStError = 7, kStWords = 8 };
 
+// A build's words: BuildArgs::counters, the tasks of every collapse level, the
+// clustering's state.
+constexpr int kLevelWord = 4, kStateWord = kLevelWord + kMaxDepth + 2, kBuildWords = kStateWord + kStWords;
+static_assert(kBuildWords <= 64, "the words are read back into BuildInputs::host_scratch");
+
+// Before a build: its words (the roots are the first nodes), empty centroid
+// bounds per segment, a single segment's triangle range.  One launch for what
+// took three clears and three copies of a few bytes from pageable memory
+// (with one copy back instead of three: 50k triangles 0.379 -> 0.367 ms).
+__global__ void k_build_init(int32_t *__restrict__ words, int *__restrict__ cbounds, int32_t *__restrict__ seg_first,
+                             int32_t n, int32_t nseg)
+{
+    for (int i = threadIdx.x; i < kBuildWords; i += blockDim.x) words[i] = i == 0 ? nseg : 0;
+    for (int i = threadIdx.x; i < 6 * nseg; i += blockDim.x) cbounds[i] = i % 6 < 3 ? 0x7fffffff : (int)0x80000000;
+    if (nseg == 1 && threadIdx.x < 2) seg_first[threadIdx.x] = threadIdx.x ? n : 0;
+}
+
 __device__ __forceinline__ float4 box_min(float4 a, float4 b)
 {
     return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), a.w);
@@ -1849,12 +1866,13 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
             cref = (int32_t *)carve(p, nn * sizeof(int32_t));
         }
         bsum = (int2 *)carve(p, (nn / kPlocBlock + 2) * sizeof(int2));
-        pstate = (int32_t *)carve(p, kStWords * sizeof(int32_t));
     }
     int2 *tq0 = (int2 *)carve(p, (nn + nseg) * sizeof(int2));
     int2 *tq1 = (int2 *)carve(p, (nn + nseg) * sizeof(int2));
-    int32_t *counters = (int32_t *)carve(p, 16 * sizeof(int32_t));
-    int32_t *level_count = (int32_t *)carve(p, (kMaxDepth + 2) * sizeof(int32_t));
+    // one block of words, read back in one copy
+    int32_t *counters = (int32_t *)carve(p, kBuildWords * sizeof(int32_t));
+    int32_t *level_count = counters + kLevelWord;
+    if (ploc) pstate = counters + kStateWord;
     int *cbounds = (int *)carve(p, 6 * (size_t)nseg * sizeof(int));
     int32_t *seg_first = (int32_t *)carve(p, ((size_t)nseg + 1) * sizeof(int32_t));
     size_t cub_bytes = 0;
@@ -1863,18 +1881,10 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
     if ((size_t)(p - (char *)temp) > temp_bytes) { R.status = -3; return R; }
 
     // segment offsets (sorted positions of each segment = its triangle range)
-    int32_t *h_cnt = in.host_scratch;   // pinned, >= 6 + kMaxDepth ints
-    std::vector<int> init_bounds(6 * (size_t)nseg);
-    for (int s = 0; s < nseg; ++s)
-        for (int k = 0; k < 3; ++k) { init_bounds[6 * s + k] = 0x7fffffff; init_bounds[6 * s + 3 + k] = (int)0x80000000; }
-    cudaMemsetAsync(counters, 0, 16 * sizeof(int32_t), st);
-    cudaMemcpyAsync(cbounds, init_bounds.data(), init_bounds.size() * sizeof(int), cudaMemcpyHostToDevice, st);
-    if (nseg > 1) {
+    int32_t *h_cnt = in.host_scratch;   // pinned
+    k_build_init<<<1, 256, 0, st>>>(counters, cbounds, seg_first, n, nseg);
+    if (nseg > 1)
         cudaMemcpyAsync(seg_first, in.seg_first, ((size_t)nseg + 1) * sizeof(int32_t), cudaMemcpyDefault, st);
-    } else {
-        const int32_t sf[2] = {0, n};
-        cudaMemcpyAsync(seg_first, sf, sizeof(sf), cudaMemcpyHostToDevice, st);
-    }
     int sb = 0;
     while ((1 << sb) < nseg) ++sb;
     // Morton bits per axis: as asked; else, from a million triangles up,
@@ -1907,9 +1917,7 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
     }
     // segment roots -> level-0 tasks (counted in level_count[0]); wide nodes
     // 0..nseg-1 are the roots
-    cudaMemsetAsync(level_count, 0, (kMaxDepth + 2) * sizeof(int32_t), st);
     if (ploc) {
-        cudaMemsetAsync(pstate, 0, kStWords * sizeof(int32_t), st);
         k_ploc_segments<<<(nseg + 127) / 128, 128, 0, st>>>(nseg, n, seg_first, pstate, in.nodes);
         if (n > 0 && (!hploc || n == 1))
             k_ploc_init<<<min((n + threads - 1) / threads, in.sm_count * 8), threads, 0, st>>>(
@@ -1956,9 +1964,6 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
         k_roots<<<(nseg + 127) / 128, 128, 0, st>>>(nseg, n, seg_first, first, last, parent, leaf_parent, tq0,
                                                     level_count, counters, in.nodes);
     }
-    const int32_t nroot_nodes = nseg;
-    cudaMemcpyAsync(&counters[0], &nroot_nodes, sizeof(int32_t), cudaMemcpyHostToDevice, st);
-
     BuildArgs A;
     A.n = n; A.left = left; A.right = right; A.count = ncount; A.dec = dec; A.slot_ref = slot_ref;
     A.ilo = ilo; A.ihi = ihi; A.llo = llo; A.lhi = lhi; A.vals = vals2;
@@ -1970,7 +1975,9 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
     // one finds no tasks), one read-back per group: most trees end within
     // the first group; a single root's first levels in one block
     const int cgrid = max(1, min((n + nseg + 63) / 64, in.sm_count * 16));
-    const int wgrid = max(1, min((n + nseg + 3) / 4, in.sm_count * 32));
+    // the blocks an SM holds: more take 3 us longer to pass through a level that
+    // finds no tasks (32 an SM: 50k triangles 0.367 ms, 10: 0.357)
+    const int wgrid = max(1, min((n + nseg + 3) / 4, in.sm_count * 10));
     int level = 0;
     if (A.dec && nseg == 1) {
         k_collapse_top<<<1, 1024, 0, st>>>(A, tq0, tq1, level_count);
@@ -1989,18 +1996,15 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
             else
                 k_collapse_level<<<cgrid, 64, 0, st>>>(A);
         }
-        cudaMemcpyAsync(h_cnt, counters, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(h_cnt + 4, level_count, (kMaxDepth + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-        // the clustering's error word (the in-block tail's iteration cap),
-        // read with the first group of levels
-        if (ploc) cudaMemcpyAsync(h_cnt + 5 + kMaxDepth, pstate + kStError, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+        // with the clustering's error word (the in-block tail's iteration cap)
+        cudaMemcpyAsync(h_cnt, counters, kBuildWords * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) { R.status = -2; return R; }
-        if (ploc && h_cnt[5 + kMaxDepth]) { R.status = -6; return R; }
-        if (level >= kMaxDepth || h_cnt[4 + level] == 0 || h_cnt[3]) break;
+        if (ploc && h_cnt[kStateWord + kStError]) { R.status = -6; return R; }
+        if (level >= kMaxDepth || h_cnt[kLevelWord + level] == 0 || h_cnt[3]) break;
     }
     if (h_cnt[3]) { R.status = -8; return R; }
-    if (h_cnt[4 + kMaxDepth] != 0) { R.status = -5; return R; }   // deeper than kMaxDepth levels
-    while (depth < kMaxDepth && h_cnt[4 + depth] > 0) ++depth;
+    if (h_cnt[kLevelWord + kMaxDepth] != 0) { R.status = -5; return R; }   // deeper than kMaxDepth levels
+    while (depth < kMaxDepth && h_cnt[kLevelWord + depth] > 0) ++depth;
     R.status = 0;
     R.nodes = h_cnt[0];
     R.tri_slots = h_cnt[1];
