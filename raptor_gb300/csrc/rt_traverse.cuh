@@ -723,11 +723,59 @@ __device__ __forceinline__ void shadow_ray(const LightView &L, float3 start, flo
     dir = xdiv3(dv, len);
 }
 
+// x^n rounded as (float)pow((double)x, (double)n) is, for x > 0.  The double
+// power keeps a warp on the SM's few FP64 units.  Whole exponents from 1 to 128
+// (specular exponents mostly are) go by squaring in pairs of floats: x = m 2^e
+// with m in [0.70, 1.41], so no product of at most 128 m's leaves 2^-65 .. 2^64.
+// With u = 2^-24 a product of pairs is off by at most 6.1 u^2 < 2^-45.3 of itself
+// (two roundings of the low parts, 2 u^2 and 3 u^2, and the dropped product of
+// the tails, u^2), a power of up to 127 products by less than 2^-38.3; 5 M powers
+// over all exponents were off by 2^-40.7 at most.  The pair's head is the rounded
+// power unless its tail, made larger by 2^-11 of itself (a tail that can matter is
+// above 2^-26 of the head), carries the head to a neighbour: those (one in 2000),
+// results outside the normal range and other exponents take the double power.
+// 512^2 glass frames: ray trees 435 -> 401 us, diffuse sets 12.04 -> 11.17 ms;
+// float terrain frames 1369 -> 1360 us, adjoint step 751 -> 738 us.
+struct FloatPair { float h, l; };
+__device__ __forceinline__ FloatPair pair_mul(FloatPair a, FloatPair b)
+{
+    const float p = __fmul_rn(a.h, b.h);
+    float e = __fmaf_rn(a.h, b.h, -p);
+    e = __fmaf_rn(a.h, b.l, e);
+    e = __fmaf_rn(a.l, b.h, e);
+    const float h = __fadd_rn(p, e);
+    return {h, __fsub_rn(e, __fsub_rn(h, p))};
+}
+__device__ __forceinline__ float specular_power(float x, float n)
+{
+    const int k = (int)n;
+    if ((float)k == n && k >= 1 && k <= 128 && x > 1.0e-30f && x < 1.0e30f) {
+        int e = (int)(__float_as_uint(x) >> 23) - 127;
+        float m = __uint_as_float((__float_as_uint(x) & 0x007fffffu) | 0x3f800000u);
+        if (m > 1.41f) {
+            m = __fmul_rn(m, 0.5f);
+            ++e;
+        }
+        FloatPair b = {m, 0.f}, r = {1.f, 0.f};
+        for (int q = k;;) {
+            if (q & 1) r = pair_mul(r, b);
+            q >>= 1;
+            if (!q) break;
+            b = pair_mul(b, b);
+        }
+        const int scale = e * k;
+        const int top = (int)((__float_as_uint(r.h) >> 23) & 0xffu) + scale;   // the result's biased exponent
+        if (top > 1 && top < 254 && __fadd_rn(r.h, __fmul_rn(r.l, 1.0f + 0x1p-11f)) == r.h)
+            return __uint_as_float(__float_as_uint(r.h) + ((uint32_t)scale << 23));
+    }
+    return (float)pow((double)x, (double)n);
+}
+
 // One light's Phong term (coloured_mapper_shader.cc:76-109,
 // light::get_light_intensity light.h:44-59) added into c.  EXACT = true
-// evaluates the specular power in double and rounds once, the reference's
-// result; EXACT = false uses single-precision powf (a few ulp), whose frames
-// are made exact by exact_if_near_boundary below.
+// takes the double power rounded once, the reference's result (specular_power);
+// EXACT = false single-precision powf (a few ulp), whose pixels near a
+// truncation are shaded again with the exact one.
 template <bool EXACT = true>
 __device__ __forceinline__ void phong_add(const LightView &L, const MaterialView &m, const float3 kd, const float3 sn,
                                           const float3 view_dir, const float3 ldir, float len, float magn, float3 &c)
@@ -738,7 +786,7 @@ __device__ __forceinline__ void phong_add(const LightView &L, const MaterialView
     const float rdr = xdot(view_dir, ref);
     float3 sc = make_float3(xmul(shade, kd.x), xmul(shade, kd.y), xmul(shade, kd.z));
     if (rdr > 0.0f) {
-        const float p = EXACT ? (float)pow((double)rdr, (double)m.ns) : powf(rdr, m.ns);
+        const float p = EXACT ? specular_power(rdr, m.ns) : powf(rdr, m.ns);
         sc = make_float3(xadd(sc.x, xmul(p, m.ks.x)), xadd(sc.y, xmul(p, m.ks.y)), xadd(sc.z, xmul(p, m.ks.z)));
     }
     const float dist = xmul(len, L.d);
