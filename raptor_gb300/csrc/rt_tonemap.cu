@@ -10,10 +10,12 @@
 //   k_tone_terms    one pass over the samples: count and maximum of the
 //                   luminances above 3.18e-7, their log10 terms (rounded
 //                   once from the exact value: float-float, double for the
-//                   few too close to a rounding boundary) and the per-chunk
-//                   increments of the exact sequential sum
+//                   few too close to a rounding boundary) and their sums
+//                   per chunk
+//   k_tone_estimate prefix sums of those: about where the running sum is
+//   k_tone_records  the chunks' increments of the exact sequential sum
 //   k_tone_coarse   the chunk increments summed over groups of chunks
-//   k_tone_sum      one warp: the reference's binary32 sum of the terms,
+//   k_tone_sum      one block: the reference's binary32 sum of the terms,
 //                   reproduced exactly, then the mode's scale factors
 //   k_hist_blocks   (histogram modes) the luminance averaged per degree of view
 //   k_hist_main     (histogram modes) histogram, trimming, cumulative map
@@ -493,11 +495,11 @@ __device__ __forceinline__ float key_float(uint32_t k)
 // sample order (camera.cc:1158).  That sum is reproduced exactly: while the
 // running sum S stays in one binade [2^e, 2^(e+1)), every addition rounds
 // to a multiple of u = 2^(e-23), so S + a_i = S + u * rne(a_i / u) as long
-// as no rne is a tie and no partial sum leaves the binade.  k_tone_terms
-// writes the terms and, per chunk of kSumChunk terms and for each of 32
-// candidate binades, the sums of the positive and of the negative rne
+// as no rne is a tie and no partial sum leaves the binade.  k_tone_records
+// writes, per chunk of kSumChunk terms and for the binades S can be in there
+// (of 32 candidates), the sums of the positive and of the negative rne
 // increments and a tie flag; k_tone_sum walks the chunks in order with one
-// warp, applying a chunk in one step when its increments provably keep S
+// block, applying a chunk in one step when its increments provably keep S
 // inside S's binade and adding its terms one by one otherwise (the first
 // chunk, binade changes, ties).  Uncounted samples contribute +0, which
 // leaves S unchanged.
@@ -515,30 +517,24 @@ struct ChunkSum {
 constexpr int32_t kSat = 1 << 30;
 __device__ __forceinline__ int32_t sat32(long long v) { return v > kSat ? kSat : (v < -kSat ? -kSat : (int32_t)v); }
 
-// values non-null: the terms are given (rt_sum_sequential_f32) instead of
-// derived from the frame.
+// The terms, and per chunk their sum (times 2^-e_hi, which keeps it in range;
+// est), an estimate of what the chunk adds.  values non-null: the terms are given
+// (rt_sum_sequential_f32) instead of derived from the frame.
 __global__ void __launch_bounds__(kSumThreads) k_tone_terms(const float *__restrict__ fimg,
-                                                            const float *__restrict__ values, int64_t n, int32_t e_lo,
-                                                            float *__restrict__ terms, ChunkSum *__restrict__ rec,
+                                                            const float *__restrict__ values, int64_t n, int32_t e_hi,
+                                                            float *__restrict__ terms, float *__restrict__ est,
                                                             ToneAcc *acc)
 {
-    __shared__ long long s_pos[32], s_neg[32];
-    __shared__ int32_t s_tie[32];
-    if (threadIdx.x < 32) {
-        s_pos[threadIdx.x] = 0;
-        s_neg[threadIdx.x] = 0;
-        s_tie[threadIdx.x] = 0;
-    }
-    __syncthreads();
+    __shared__ float s_sum[kSumThreads / 32];
     const int64_t base = (int64_t)blockIdx.x * kSumChunk;
-    float a[kSumPerThread];
+    float sum = 0.0f;
     uint32_t cnt = 0, maxb = 0;
 #pragma unroll
     for (int t = 0; t < kSumPerThread; ++t) {
         const int64_t i = base + t * kSumThreads + threadIdx.x;
-        a[t] = 0.0f;
+        float a = 0.0f;
         if (i < n && values) {
-            a[t] = values[i];
+            a = values[i];
         } else if (i < n) {
             const float r = xdiv(fimg[3 * i], 255.0f), g = xdiv(fimg[3 * i + 1], 255.0f),
                         b = xdiv(fimg[3 * i + 2], 255.0f);
@@ -546,64 +542,112 @@ __global__ void __launch_bounds__(kSumThreads) k_tone_terms(const float *__restr
             if (!(Y < 3.18e-7f)) {
                 ++cnt;
                 maxb = max(maxb, __float_as_uint(Y));   // Y > 0: bit order is value order
-                a[t] = log10_cr(Y);
+                a = log10_cr(Y);
             }
         }
-        terms[i] = a[t];   // the padding of the last chunk holds +0
+        terms[i] = a;   // the padding of the last chunk holds +0
+        sum += ldexpf(a, -e_hi);
     }
-    // Per binade ei: the warp's sums of the positive and negative rounded
-    // increments (one redux each) and its tie flags (bit ei, one redux for
-    // all 32); lane ei keeps binade ei's sums.  A lane's own sums (4 terms of
-    // |q| <= 2^26) fit in int32; each is clamped to +-2^25 before the warp
-    // sum, so that sum stays below 2^30 and is exact unless some lane was
-    // clamped, in which case it is >= 2^25 in magnitude: a record that large
-    // never applies, whatever its exact value.
     const int lane = threadIdx.x & 31;
-    int32_t my_pos = 0, my_neg = 0;
-    uint32_t ties = 0;
-    for (int ei = 0; ei < 32; ++ei) {
-        int32_t pos = 0, neg = 0;
-#pragma unroll
-        for (int t = 0; t < kSumPerThread; ++t) {
-            const float k = ldexpf(a[t], 23 - (e_lo + ei));   // exact: a power-of-two scale
-            int32_t q;
-            if (fabsf(k) < 33554432.0f) {                      // |k| < 2^25
-                q = __float2int_rn(k);                         // round to nearest, ties to even
-                if (xsub(k, floorf(k)) == 0.5f) ties |= 1u << ei;
-            } else {
-                q = (k > 0.0f) ? (1 << 26) : -(1 << 26);       // too large to apply: saturates the sums
-            }
-            if (q > 0) pos += q;
-            else neg += q;
-        }
-        const int32_t wpos = __reduce_add_sync(0xffffffffu, min(pos, 1 << 25));
-        const int32_t wneg = __reduce_add_sync(0xffffffffu, max(neg, -(1 << 25)));
-        if (lane == ei) {
-            my_pos = wpos;
-            my_neg = wneg;
-        }
-    }
-    ties = __reduce_or_sync(0xffffffffu, ties);
-    atomicAdd((unsigned long long *)&s_pos[lane], (unsigned long long)(long long)my_pos);
-    atomicAdd((unsigned long long *)&s_neg[lane], (unsigned long long)(long long)my_neg);
-    if ((ties >> lane) & 1u) atomicOr(&s_tie[lane], 1);
     for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
         cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
         maxb = max(maxb, __shfl_xor_sync(0xffffffffu, maxb, o));
     }
-    if (lane == 0 && cnt) {
-        atomicAdd(&acc->count, (unsigned long long)cnt);
-        atomicMax(&acc->max_bits, maxb);
+    if (lane == 0) {
+        s_sum[threadIdx.x >> 5] = sum;
+        if (cnt) {
+            atomicAdd(&acc->count, (unsigned long long)cnt);
+            atomicMax(&acc->max_bits, maxb);
+        }
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
-        ChunkSum c;
-        c.pos = sat32(s_pos[threadIdx.x]);
-        c.neg = sat32(s_neg[threadIdx.x]);
-        c.tie = s_tie[threadIdx.x];
-        c.pad = 0;
-        rec[(int64_t)blockIdx.x * 32 + threadIdx.x] = c;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kSumThreads / 32; ++w) sum += s_sum[w];
+        est[blockIdx.x] = sum;
     }
+}
+
+// Chunk sums to their prefix sums, est[c] the estimate before chunk c, est[n]
+// the whole (one block, a run of chunks to a thread).
+__global__ void __launch_bounds__(1024) k_tone_estimate(float *__restrict__ est, int64_t nchunks)
+{
+    __shared__ float s_warp[32];
+    const int64_t per = (nchunks + blockDim.x - 1) / blockDim.x;
+    const int64_t first = min((int64_t)threadIdx.x * per, nchunks), last = min(first + per, nchunks);
+    float own = 0.0f;
+    for (int64_t c = first; c < last; ++c) own += est[c];
+    const int lane = threadIdx.x & 31;
+    float incl = own;
+    for (int o = 1; o < 32; o <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_warp[threadIdx.x >> 5] = incl;
+    __syncthreads();
+    float at = incl - own;
+    for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) at += s_warp[w];
+    for (int64_t c = first; c < last; ++c) {
+        const float v = est[c];
+        est[c] = at;
+        at += v;
+    }
+    if (last == nchunks && first < last) est[nchunks] = at;
+}
+
+// Records of a warp's chunk for the binades the running sum can be in there:
+// from one below to one above those of the estimates at its ends, at most six.
+// The others are marked as ties, which are never applied; an estimate that is
+// off (sums that cancel) costs time, not bits: the chunk is added term by term.
+// With all 32 binades formed where the terms are, that kernel was bound by their
+// instructions: 131 us for 2.4 M samples, now 50 there, 9 for the estimates and 13
+// for these records.
+constexpr int kSumBinades = 6;
+__host__ __device__ constexpr int64_t estimate_floats(int64_t nchunks) { return (nchunks + 1 + 3) & ~(int64_t)3; }
+__global__ void __launch_bounds__(kSumThreads) k_tone_records(const float *__restrict__ terms, int64_t nchunks,
+                                                              int32_t e_lo, const float *__restrict__ est,
+                                                              ChunkSum *__restrict__ rec)
+{
+    const int64_t c = (int64_t)blockIdx.x * (kSumThreads / 32) + (threadIdx.x >> 5);
+    if (c >= nchunks) return;
+    const int lane = threadIdx.x & 31;
+    // candidate 31 is the binade of 2^e_hi, the estimates' unit
+    const float s0 = fabsf(est[c]), s1 = fabsf(est[c + 1]);
+    const int e0 = 31 + (int)(__float_as_uint(fminf(s0, s1)) >> 23) - 127;
+    const int e1 = 31 + (int)(__float_as_uint(fmaxf(s0, s1)) >> 23) - 127;
+    const int hi = min(max(e1 + 1, 0), 31), lo = max(max(e0 - 1, hi - (kSumBinades - 1)), 0);
+    float a[kSumChunk / 32];
+#pragma unroll
+    for (int q = 0; q < kSumChunk / 32; ++q) a[q] = terms[c * kSumChunk + q * 32 + lane];
+    ChunkSum mine = {0, 0, 1, 0};
+    for (int ei = lo; ei <= hi; ++ei) {
+        // the warp's sums of the positive and of the negative rounded increments
+        // and its ties.  A lane's own sums (16 terms of |q| <= 2^26) fit in
+        // int32; each is clamped to +-2^25 before the warp sum, so that sum
+        // stays within 2^30 and is exact unless some lane was clamped, in which
+        // case it is >= 2^25 in magnitude: a record that large never applies,
+        // whatever its exact value.
+        int32_t pos = 0, neg = 0;
+        bool tie = false;
+#pragma unroll
+        for (int q = 0; q < kSumChunk / 32; ++q) {
+            const float k = ldexpf(a[q], 23 - (e_lo + ei));   // exact: a power-of-two scale
+            int32_t r;
+            if (fabsf(k) < 33554432.0f) {                      // |k| < 2^25
+                r = __float2int_rn(k);                         // round to nearest, ties to even
+                tie |= xsub(k, floorf(k)) == 0.5f;
+            } else {
+                r = (k > 0.0f) ? (1 << 26) : -(1 << 26);       // too large to apply: saturates the sums
+            }
+            if (r > 0) pos += r;
+            else neg += r;
+        }
+        const int32_t wpos = __reduce_add_sync(0xffffffffu, min(pos, 1 << 25));
+        const int32_t wneg = __reduce_add_sync(0xffffffffu, max(neg, -(1 << 25)));
+        const bool wtie = __any_sync(0xffffffffu, tie);
+        if (lane == ei) mine = {wpos, wneg, wtie ? 1 : 0, 0};
+    }
+    rec[c * 32 + lane] = mine;
 }
 
 // The scale factors of camera::tone_map's mode branch (camera.cc:1203-1425)
@@ -767,100 +811,108 @@ __device__ __forceinline__ float add_slice(float S, float v)
     return S;
 }
 
-// The 512 terms of chunk j (16 slices of 32, slice q holding terms
-// q*32 .. q*32+31 in lane order) added to S in order.  For S's binade all
-// remaining slices are scanned at once (rounded increments, warp scans,
-// running bases); the slices before the first one whose prefix sums leave
-// the binade (or hold a tie) are applied in one step, that slice term by
-// term, and the rest tried again in the new binade.  Uniform across the warp.
+// The 512 terms of chunk j added to S in order by a block of a thread to each:
+// warp q holds slice q, terms q*32 .. q*32+31.  For S's binade all remaining
+// slices are scanned at once (rounded increments, warp scans, the slices' totals
+// before it); the slices before the first one whose prefix sums leave the binade
+// (or hold a tie) are applied in one step, that slice term by term, and the rest
+// tried again in the new binade.  S and the result are the same in every thread.
+constexpr int kSlices = kSumChunk / 32;
 __device__ float sum_chunk(float S, const float *__restrict__ terms, int64_t j)
 {
-    constexpr int Q = kSumChunk / 32;
-    const int lane = threadIdx.x & 31;
-    float a[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) a[q] = terms[j * kSumChunk + q * 32 + lane];
+    __shared__ int32_t s_total[kSlices], s_end[kSlices], s_fail[kSlices];
+    __shared__ float s_sum;
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+    const float a = terms[j * kSumChunk + threadIdx.x];
     int q0 = 0;
-    for (int round = 0; round <= Q && q0 < Q; ++round) {
+    for (int round = 0; round <= kSlices && q0 < kSlices; ++round) {
         int e;
         int32_t M;
         int bad = q0;   // the first slice that cannot be applied
         if (split(S, e, M) && 23 - e <= 127) {
             const float scale = __int_as_float((23 - e + 127) << 23);   // 2^(23-e)
-            int32_t P[Q];
-            uint32_t fails = 0;   // bit q: slice q fails in this lane
+            const float k = xmul(a, scale);                             // exact: a power-of-two scale
+            const bool big = !(fabsf(k) < 33554432.0f);
+            const bool tie = !big && xsub(k, floorf(k)) == 0.5f;
+            int32_t P = big ? 0 : __float2int_rn(k);
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const float k = xmul(a[q], scale);   // exact: a power-of-two scale
-                const bool big = !(fabsf(k) < 33554432.0f);
-                const bool tie = !big && xsub(k, floorf(k)) == 0.5f;
-                P[q] = big ? 0 : __float2int_rn(k);
-                if (big || tie) fails |= 1u << q;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t v = __shfl_up_sync(0xffffffffu, P, o);
+                if (lane >= o) P += v;
             }
+            if (lane == 31) s_total[q] = q >= q0 ? min(max(P, -(1 << 25)), 1 << 25) : 0;
+            __syncthreads();
+            int32_t incl = lane < kSlices ? s_total[lane] : 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1)
-#pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    const int32_t v = __shfl_up_sync(0xffffffffu, P[q], o);
-                    if (lane >= o) P[q] += v;
-                }
-            // running base over the slices from q0 on
-            int32_t base = 0;
-            int32_t base_at[Q];
-#pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                base_at[q] = base;
-                if (q >= q0) base += min(max(__shfl_sync(0xffffffffu, P[q], 31), -(1 << 25)), 1 << 25);
+            for (int o = 1; o < kSlices; o <<= 1) {
+                const int32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
             }
-#pragma unroll
-            for (int q = 0; q < Q; ++q)
-                if (q >= q0 && !inside(M, base_at[q] + P[q])) fails |= 1u << q;
-            fails = __reduce_or_sync(0xffffffffu, fails) & ~((1u << q0) - 1u);
-            bad = fails ? __ffs(fails) - 1 : Q;
-            if (bad > q0) {
-                int32_t upto = 0;
-#pragma unroll
-                for (int q = 0; q < Q; ++q)
-                    if (q == bad - 1) upto = __shfl_sync(0xffffffffu, base_at[q] + P[q], 31);
-                S = join(e, M + upto);
+            const int32_t before = __shfl_sync(0xffffffffu, incl, q > 0 ? q - 1 : 0);
+            const int32_t base = q > 0 ? before : 0;
+            const bool ok = __all_sync(0xffffffffu, !big && !tie && inside(M, base + P));
+            if (lane == 31) {
+                s_end[q] = base + P;
+                s_fail[q] = q >= q0 && !ok;
             }
+            __syncthreads();
+            const uint32_t fails = __ballot_sync(0xffffffffu, lane < kSlices && s_fail[lane < kSlices ? lane : 0] != 0);
+            bad = fails ? __ffs(fails) - 1 : kSlices;
+            if (bad > q0) S = join(e, M + s_end[bad - 1]);
         }
-        if (bad >= Q) break;
-        float v = 0.0f;
-#pragma unroll
-        for (int q = 0; q < Q; ++q)
-            if (q == bad) v = a[q];
-        S = add_slice(S, v);
+        if (bad >= kSlices) break;
+        if (q == bad) {
+            const float v = add_slice(S, a);
+            if (lane == 0) s_sum = v;
+        }
+        __syncthreads();
+        S = s_sum;
         q0 = bad + 1;
+        __syncthreads();   // read by all before the next round writes it
     }
+    __syncthreads();
     return S;
 }
 
-// One warp walks the groups of kCoarse chunks in order, 32 group records at
-// a time (apply_records); a group that cannot be applied goes chunk by
-// chunk (its records), a chunk slice by slice (sum_chunk).  Then the scale
-// factors.
-__global__ void __launch_bounds__(32) k_tone_sum(const float *__restrict__ terms, const ChunkSum *__restrict__ rec,
-                                                 const ChunkSum *__restrict__ crec, int64_t nchunks, int64_t ncoarse,
-                                                 int32_t e_lo, ToneView t, ToneAcc *acc, bool scalars)
+// Warp 0 walks the groups of kCoarse chunks in order, 32 group records at a
+// time (apply_records); a group that cannot be applied goes chunk by chunk (its
+// records), a chunk that cannot slice by slice, on the whole block (sum_chunk; on
+// one warp its 16 scans of 32 terms were most of the kernel: 138 us for 2.4 M
+// samples, now 100, latency of the records' loads).  Then the scale factors.
+__global__ void __launch_bounds__(kSumChunk) k_tone_sum(const float *__restrict__ terms, const ChunkSum *__restrict__ rec,
+                                                        const ChunkSum *__restrict__ crec, int64_t nchunks,
+                                                        int64_t ncoarse, int32_t e_lo, ToneView t, ToneAcc *acc,
+                                                        bool scalars)
 {
+    __shared__ float s_S;
+    __shared__ int64_t s_chunk;
     float S = 0.0f;
-    int64_t c = 0;
-    for (int64_t guard = 0; c < ncoarse && guard < 4 * ncoarse + 64; ++guard) {
-        const int n = apply_records(S, crec, c, ncoarse, 32, e_lo);
-        c += n;
-        if (n == 32 || c >= ncoarse) continue;
-        // group c chunk by chunk
-        const int64_t j_end = (c + 1) * kCoarse < nchunks ? (c + 1) * kCoarse : nchunks;
-        int64_t j = c * kCoarse;
-        for (int g2 = 0; j < j_end && g2 <= kCoarse; ++g2) {
-            const int m = apply_records(S, rec, j, j_end, 32, e_lo);
-            j += m;
-            if (j >= j_end) break;
-            S = sum_chunk(S, terms, j);
-            ++j;
+    int64_t c = 0, j = 0, j_end = 0;   // warp 0: the group, the next chunk of a group taken chunk by chunk
+    for (int64_t guard = 0; guard <= nchunks; ++guard) {   // a chunk each
+        if (threadIdx.x < 32) {
+            int64_t chunk = -1;
+            while (chunk < 0 && (j < j_end || c < ncoarse)) {
+                if (j < j_end) {
+                    j += apply_records(S, rec, j, j_end, 32, e_lo);
+                    if (j < j_end) chunk = j++;
+                    if (j >= j_end) ++c;
+                    continue;
+                }
+                const int n = apply_records(S, crec, c, ncoarse, 32, e_lo);
+                c += n;
+                if (n == 32 || c >= ncoarse) continue;
+                j = c * kCoarse;
+                j_end = (c + 1) * kCoarse < nchunks ? (c + 1) * kCoarse : nchunks;
+            }
+            if (threadIdx.x == 0) {
+                s_S = S;
+                s_chunk = chunk;
+            }
         }
-        ++c;
+        __syncthreads();
+        const int64_t chunk = s_chunk;
+        if (chunk < 0) break;
+        S = sum_chunk(s_S, terms, chunk);
     }
     if (threadIdx.x == 0) {
         acc->sum_f = S;
@@ -1393,7 +1445,8 @@ size_t sum_scratch_bytes(int64_t n)
 {
     const int64_t nchunks = (n + kSumChunk - 1) / kSumChunk;
     const int64_t ncoarse = (nchunks + kCoarse - 1) / kCoarse;
-    return (size_t)nchunks * kSumChunk * sizeof(float) + (size_t)(nchunks + ncoarse) * 32 * sizeof(ChunkSum);
+    return (size_t)nchunks * kSumChunk * sizeof(float) + (size_t)(nchunks + ncoarse) * 32 * sizeof(ChunkSum) +
+           (size_t)estimate_floats(nchunks) * sizeof(float);
 }
 
 size_t tone_scratch_bytes(int64_t n, int64_t blocks)
@@ -1472,13 +1525,14 @@ void launch_tone_map(const float *fimg, int32_t fw, int32_t fh, int32_t aa_x, in
     ToneView t = t_in;
     const int64_t n = (int64_t)fw * fh;
     const int32_t ow = fw / aa_x, oh = fh / aa_y;
-    // scratch: terms | chunk records | coarse records | redo queue
+    // scratch: terms | chunk records | coarse records | chunk estimates | redo queue
     const int64_t nchunks = (n + kSumChunk - 1) / kSumChunk;
     const int64_t ncoarse = (nchunks + kCoarse - 1) / kCoarse;
     float *terms = (float *)scratch;
     ChunkSum *rec = (ChunkSum *)(terms + nchunks * kSumChunk);
     ChunkSum *crec = rec + nchunks * 32;
-    int2 *redo = (int2 *)(crec + ncoarse * 32);
+    float *est = (float *)(crec + ncoarse * 32);
+    int2 *redo = (int2 *)(est + estimate_floats(nchunks));
     float *hblocks = (float *)(redo + n);
     cudaMemsetAsync(acc, 0, sizeof(ToneAcc), st);
     // the stretch range starts empty (k_tone_sum sets it too, for the other modes)
@@ -1489,9 +1543,11 @@ void launch_tone_map(const float *fimg, int32_t fw, int32_t fh, int32_t aa_x, in
         // candidate binades: |S| <= 39 n (|log10 Y| < 39 for any float Y)
         const int32_t e_hi = (int32_t)std::floor(std::log2(39.0 * (double)n)) + 1;
         const int32_t e_lo = e_hi - 31;
-        k_tone_terms<<<(unsigned)nchunks, kSumThreads, 0, st>>>(fimg, nullptr, n, e_lo, terms, rec, acc);
+        k_tone_terms<<<(unsigned)nchunks, kSumThreads, 0, st>>>(fimg, nullptr, n, e_hi, terms, est, acc);
+        k_tone_estimate<<<1, 1024, 0, st>>>(est, nchunks);
+        k_tone_records<<<(unsigned)((nchunks + 3) / 4), kSumThreads, 0, st>>>(terms, nchunks, e_lo, est, rec);
         k_tone_coarse<<<(unsigned)((ncoarse * 32 + 255) / 256), 256, 0, st>>>(rec, nchunks, ncoarse, crec);
-        k_tone_sum<<<1, 32, 0, st>>>(terms, rec, crec, nchunks, ncoarse, e_lo, t, acc, true);
+        k_tone_sum<<<1, kSumChunk, 0, st>>>(terms, rec, crec, nchunks, ncoarse, e_lo, t, acc, true);
         if (t.mode == RT_TONE_LOCAL_HISTOGRAM || t.mode == RT_TONE_LOCAL_HUMAN_HISTOGRAM) {
             const int64_t nb = (int64_t)t.hist_sx * t.hist_sy;
             float *bx = hblocks + nb, *by = bx + 2 * 4096;
@@ -1561,15 +1617,18 @@ void launch_sequential_sum(const float *v, int64_t n, float max_abs, ToneAcc *ac
     float *terms = (float *)scratch;
     ChunkSum *rec = (ChunkSum *)(terms + nchunks * kSumChunk);
     ChunkSum *crec = rec + nchunks * 32;
+    float *est = (float *)(crec + ncoarse * 32);
     // candidate binades: |S| <= max_abs * n
     int32_t e_hi = (int32_t)std::floor(std::log2((double)max_abs * (double)n)) + 1;
     if (e_hi > 128) e_hi = 128;
     const int32_t e_lo = e_hi - 31;
     cudaMemsetAsync(acc, 0, sizeof(ToneAcc), st);
     ToneView t = {};
-    k_tone_terms<<<(unsigned)nchunks, kSumThreads, 0, st>>>(nullptr, v, n, e_lo, terms, rec, acc);
+    k_tone_terms<<<(unsigned)nchunks, kSumThreads, 0, st>>>(nullptr, v, n, e_hi, terms, est, acc);
+    k_tone_estimate<<<1, 1024, 0, st>>>(est, nchunks);
+    k_tone_records<<<(unsigned)((nchunks + 3) / 4), kSumThreads, 0, st>>>(terms, nchunks, e_lo, est, rec);
     k_tone_coarse<<<(unsigned)((ncoarse * 32 + 255) / 256), 256, 0, st>>>(rec, nchunks, ncoarse, crec);
-    k_tone_sum<<<1, 32, 0, st>>>(terms, rec, crec, nchunks, ncoarse, e_lo, t, acc, false);
+    k_tone_sum<<<1, kSumChunk, 0, st>>>(terms, rec, crec, nchunks, ncoarse, e_lo, t, acc, false);
 }
 
 }  // namespace rtc
