@@ -6,10 +6,21 @@
 namespace rtc {
 
 constexpr int kTraceThreads = 128;   // 4 warps per block
-// Minimum resident blocks per SM the render/trace kernels are compiled for
-// (caps registers per thread: 1 -> 255, 6 -> 80, 8 -> 64; 8 measured fastest:
-// more resident warps hide the latency of the node loads better than the
-// registers the cap spills).
+// Minimum resident blocks per SM the kernels are compiled for (caps registers
+// per thread: 4 -> 128, 5 -> 96, 6 -> 80, 8 -> 64).  Rays one by one: 8, more
+// resident warps hide the latency of the node loads better than the registers the
+// cap spills.  Frames traced in step hold triangles and shading state through a
+// warp's traversal and gain from registers: at 8 / 7 / 6 / 5 / 4 blocks the 20k
+// sphere 512^2 takes 133 / 131 / 124 / 121 / 121 us, the terrain at 4K 2278 / 2229
+// / 2228 / 2192 / 2351 (k_render, k_render_table: 5); 2x2 samples of 1283x717
+// terrain 1132 / 1112 / 1104 / 1120 / 1168 and its float frame with tone mapping
+// 840 / 840 / 827 / 836 / 890 (6).
+#ifndef RT_FRAME_MIN_BLOCKS
+#define RT_FRAME_MIN_BLOCKS 5
+#endif
+#ifndef RT_SAMPLE_MIN_BLOCKS
+#define RT_SAMPLE_MIN_BLOCKS 6
+#endif
 #ifndef RT_WAVE_MIN_BLOCKS
 #define RT_WAVE_MIN_BLOCKS RT_RENDER_MIN_BLOCKS   // lane-replacement kernels
 #endif

@@ -303,7 +303,7 @@ struct AreaSet {
 
 // Pass 1: the camera ray of every pixel; hit record and hit flag.
 template <class SC>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_primary(SC sc, CameraView cam,
+__global__ void __launch_bounds__(kTraceThreads, 6) k_soft_primary(SC sc, CameraView cam,
                                                                                       int4 *__restrict__ hits,
                                                                                       int32_t *__restrict__ flags,
                                                                                       Counters *ctr)
@@ -387,8 +387,10 @@ __device__ __forceinline__ void trace_hit_rays(const SC &sc, const float3 start,
 
 // Pass 2: shading.  rnd holds the frame's numbers (rnd[0] = the frame's
 // first), nrnd of them; a hit pixel's first is prefix[pix] * per_hit.
+// 6 blocks an SM for the camera rays and 7 here: a 900p frame's kernels 2.33 -> 2.27 ms
+// (8 and 8; 5 and 5: 2.34).
 template <class SC>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_soft_shade(
+__global__ void __launch_bounds__(kTraceThreads, 7) k_soft_shade(
     SC sc, CameraView cam, LightSet lights, MaterialTable table, AreaSet areas, const int4 *__restrict__ area,
     const float *__restrict__ verts, int32_t samples, int32_t per_hit, const uint32_t *__restrict__ rnd, int64_t nrnd,
     const float *__restrict__ lut, const int4 *__restrict__ hits, const int32_t *__restrict__ prefix,

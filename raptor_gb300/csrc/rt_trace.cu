@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(32, 32) k_trace_few(SC sc, const rt_ray *__res
 namespace {
 
 template <bool COUNT, class SC>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render(SC sc, CameraView cam, LightSet lights,
+__global__ void __launch_bounds__(kTraceThreads, RT_FRAME_MIN_BLOCKS) k_render(SC sc, CameraView cam, LightSet lights,
                                                           MaterialView mat, uint8_t *__restrict__ rgb,
                                                           int32_t *__restrict__ ids, Counters *ctr)
 {
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render(
 // primary + shadow kernel, its material per triangle from `table` (entry 0
 // when the scene has no indices).
 template <bool COUNT, class SC>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_float(SC sc, CameraView cam, LightSet lights,
+__global__ void __launch_bounds__(kTraceThreads, RT_SAMPLE_MIN_BLOCKS) k_render_float(SC sc, CameraView cam, LightSet lights,
                                                           MaterialTable table, float *__restrict__ fimg,
                                                           Counters *ctr)
 {
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
 // (rt_render_materials without mirror or refracted rays): a separate kernel
 // so that the single-material one keeps its code and parameter block.
 template <bool COUNT, class SC>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_table(SC sc, CameraView cam, LightSet lights,
+__global__ void __launch_bounds__(kTraceThreads, RT_FRAME_MIN_BLOCKS) k_render_table(SC sc, CameraView cam, LightSet lights,
                                                           MaterialView mat, uint8_t *__restrict__ rgb,
                                                           int32_t *__restrict__ ids, Counters *ctr,
                                                           MaterialTable table)
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
 // which recomputes it from samples shaded with the exact power in a compact
 // second pass, so that no warp waits on one lane's exact re-shade.
 template <bool COUNT, class SC>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa(SC sc, CameraView cam,
+__global__ void __launch_bounds__(kTraceThreads, RT_SAMPLE_MIN_BLOCKS) k_render_aa(SC sc, CameraView cam,
                                                              LightSet lights, MaterialView mat, int32_t aa_x,
                                                              int32_t aa_y, int32_t out_x, int32_t out_y,
                                                              uint8_t *__restrict__ rgb, int32_t *__restrict__ redo,
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
 // bit, while the warp's lanes trace one sample each instead of looping
 // over a pixel's samples.
 template <bool COUNT, class SC>
-__global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa_lanes(SC sc, CameraView cam,
+__global__ void __launch_bounds__(kTraceThreads, RT_SAMPLE_MIN_BLOCKS) k_render_aa_lanes(SC sc, CameraView cam,
                                                              LightSet lights, MaterialView mat, int32_t aa_x,
                                                              int32_t aa_y, int32_t out_x, int32_t out_y,
                                                              uint8_t *__restrict__ rgb, int32_t *__restrict__ redo,
