@@ -581,10 +581,13 @@ rt_status rt_bvh_stats_get(const rt_scene *s, rt_bvh_stats *out)
 
 }  // extern "C"
 
-// Host rays up to which a query is staged through the context's pinned
-// buffer (768 KB): beyond, the bulk copies cost less than the link's latency
-// per ray.
+// Host rays up to which a query is staged through the context's pinned buffer
+// (768 KB): beyond, the bulk copies cost less than the link's latency per ray.
+// Closest hits bring 16 bytes a ray back, any hits one: 20k sphere, 12288 closest
+// 42..61 us against 43..68, 16384 51..73 against 44..69; 16384 any 34..52
+// against 43..55.
 constexpr int32_t kFewHostRays = 16384;
+constexpr int32_t kFewHostClosest = 12288;
 
 template <bool ANY>
 static rt_status trace_common(rt_scene *s, const rt_ray *rays, int32_t n, void *out, const char *name)
@@ -598,10 +601,12 @@ static rt_status trace_common(rt_scene *s, const rt_ray *rays, int32_t n, void *
     const size_t out_bytes = ANY ? (size_t)n : (size_t)n * sizeof(rt_hit);
     const bool rays_dev = is_device_ptr(rays), out_dev = is_device_ptr(out);
     const SceneView sv = scene_view(s);
-    if (n <= (rays_dev && out_dev ? few_ray_warps(ctx->sm_count) * 32 : kFewHostRays)) {
+    uint32_t *word = &ctx->h_counters->status;   // pinned: the kernels write it on errors only
+    *word = 0;
+    if (n <= (rays_dev && out_dev ? few_ray_warps(ctx->sm_count) * 32 : ANY ? kFewHostRays : kFewHostClosest)) {
         // one launch and one wait: host rays and results go through pinned
         // memory that the kernel reads and writes in place, the status word
-        // too.  (300 host rays: 85 -> 44 us a call; copies, counter clear and
+        // too.  (300 host rays: 78 -> 37 us a call; copies, counter clear and
         // counter read-back were most of it.)
         if (!ctx->h_rays && !(rays_dev && out_dev) &&
             cudaMallocHost(&ctx->h_rays, (size_t)kFewHostRays * (sizeof(rt_ray) + sizeof(rt_hit))) != cudaSuccess) {
@@ -616,8 +621,6 @@ static rt_status trace_common(rt_scene *s, const rt_ray *rays, int32_t n, void *
                 in = (const rt_ray *)ctx->h_rays;
             }
             if (!out_dev) res = (rt_ray *)ctx->h_rays + kFewHostRays;
-            uint32_t *word = &ctx->h_counters->status;
-            *word = 0;
             launch_trace_few<ANY>(sv, in, n, res, word, ctx->sm_count, ctx->stream);
             RT_CUDA(cudaGetLastError(), "trace launch");
             RT_CUDA(cudaStreamSynchronize(ctx->stream), "stream synchronize");
@@ -634,19 +637,18 @@ static rt_status trace_common(rt_scene *s, const rt_ray *rays, int32_t n, void *
         RT_CUDA(ctx->stage_b.reserve(out_bytes), "staging allocation");
         d_out = ctx->stage_b.ptr;
     }
-    RT_CUDA(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), ctx->stream), "counter clear");
-    if (ANY)
-        launch_trace_any(sv, (const rt_ray *)d_rays, n, (uint8_t *)d_out, ctx->d_counters, ctx->sm_count, ctx->stream);
-    else
-        launch_trace_closest(sv, (const rt_ray *)d_rays, n, (rt_hit *)d_out, ctx->d_counters, ctx->sm_count,
-                             ctx->stream);
+    int *work = (int *)ctx->d_counters;   // its first words
+    if (ANY) {
+        launch_trace_any(sv, (const rt_ray *)d_rays, n, (uint8_t *)d_out, work, word, ctx->sm_count, ctx->stream);
+    } else {
+        RT_CUDA(cudaMemsetAsync(work, 0, sizeof(int), ctx->stream), "counter clear");
+        launch_trace_closest(sv, (const rt_ray *)d_rays, n, (rt_hit *)d_out, work, word, ctx->sm_count, ctx->stream);
+    }
     RT_CUDA(cudaGetLastError(), "trace launch");
     if (!out_dev)
         RT_CUDA(cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, ctx->stream), "device-to-host copy");
-    Counters c;
-    st = read_counters(ctx, &c);
-    if (st != RT_OK) return st;
-    return status_to_error(c.status);
+    RT_CUDA(cudaStreamSynchronize(ctx->stream), "stream synchronize");
+    return status_to_error(*word);
 }
 
 extern "C" {

@@ -90,8 +90,10 @@ struct LightSet {
 // of kTruncGuard).
 bool fast_pow_ok(const rt_light *lights, int32_t n, const rt_material &m);
 
-void launch_trace_closest(const SceneView &sc, const rt_ray *rays, int32_t n, rt_hit *hits, Counters *ctr, int sm_count,
-                          cudaStream_t st);
+// work: a device word, cleared by the caller; status (OR of device status
+// bits, zeroed by the caller) may be pinned host memory.
+void launch_trace_closest(const SceneView &sc, const rt_ray *rays, int32_t n, rt_hit *hits, int *work, uint32_t *status,
+                          int sm_count, cudaStream_t st);
 // Up to few_ray_warps * 32 rays in one pass without a work queue: fewer rays
 // to a warp while warps are idle.  rays, out (rt_hit or uint8_t) and status
 // (OR of device status bits, zeroed by the caller) may be pinned host memory.
@@ -99,8 +101,9 @@ inline int32_t few_ray_warps(int sm_count) { return sm_count * 32; }
 template <bool ANY>
 void launch_trace_few(const SceneView &sc, const rt_ray *rays, int32_t n, void *out, uint32_t *status, int sm_count,
                       cudaStream_t st);
-void launch_trace_any(const SceneView &sc, const rt_ray *rays, int32_t n, uint8_t *occ, Counters *ctr, int sm_count,
-                      cudaStream_t st);
+// work: two device words, in any state; status as above.
+void launch_trace_any(const SceneView &sc, const rt_ray *rays, int32_t n, uint8_t *occ, int *work, uint32_t *status,
+                      int sm_count, cudaStream_t st);
 void launch_render(const SceneView &sc, const CameraView &cam, const LightSet &lights, const MaterialView &mat,
                    uint8_t *rgb, int32_t *ids, Counters *ctr, int sm_count, cudaStream_t st, bool count = false);
 // Float frame (3 floats per pixel, exact) of a frame without secondary rays.

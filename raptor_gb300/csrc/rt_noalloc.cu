@@ -122,7 +122,7 @@ extern "C" rt_status rt_trace_closest_noalloc(rt_scene *s, const rt_ray *rays, i
     st = cuda_check(cudaMemcpyAsync(d_rays, rays, (size_t)n * sizeof(rt_ray), cudaMemcpyDefault, stream),
                     "rt_trace_closest_noalloc: ray copy");
     if (st != RT_OK) return st;
-    launch_trace_closest(scene_view(s), d_rays, n, d_hits, d_ctr, ctx->sm_count, stream);
+    launch_trace_closest(scene_view(s), d_rays, n, d_hits, &d_ctr->work, &d_ctr->status, ctx->sm_count, stream);
     st = cuda_check(cudaGetLastError(), "rt_trace_closest_noalloc: trace launch");
     if (st != RT_OK) return st;
     st = cuda_check(cudaMemcpyAsync(hits, d_hits, (size_t)n * sizeof(rt_hit), cudaMemcpyDefault, stream),

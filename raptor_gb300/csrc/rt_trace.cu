@@ -14,11 +14,11 @@ namespace {
 template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_closest(SC sc, const rt_ray *__restrict__ rays,
                                                                  int32_t n, rt_hit *__restrict__ hits,
-                                                                 Counters *ctr)
+                                                                 int *work, uint32_t *out_status)
 {
     uint32_t status = 0;
     for (;;) {
-        const int base = warp_claim(&ctr->work, 32);
+        const int base = warp_claim(work, 32);
         if (base >= n) break;
         const int i = base + (threadIdx.x & 31);
         if (i < n) {
@@ -30,58 +30,85 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_c
             reinterpret_cast<float4 *>(hits)[i] = make_float4(__int_as_float(h.id), h.t, h.u, h.v);
         }
     }
-    if (status) atomicOr(&ctr->status, status);
+    if (status) atomicOr_system(out_status, status);
 }
 
-// Do the rays of a list (at least 32) start all over the scene?  Most of
-// kRayGroups groups of 32, spread over the list, have rays that start further
-// than a 32nd of the scene from their first.
-constexpr int kRayGroups = 8;
-__device__ __forceinline__ bool rays_scattered(const SceneView &sc, const rt_ray *__restrict__ rays, int n)
+// Waits for the kernels before this one on the stream, where it may be
+// launched while they end.
+__device__ __forceinline__ void earlier_kernels() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Before a large any-hit query (at least 32 rays), in place of its counters'
+// clear: does k_trace_any_list take it?  *use is set where the rays start all
+// over the scene -- most of kRayGroups groups of 32, spread over the list, have
+// rays that start further than a 32nd of the scene from their first -- and
+// kGoingRays or more of them (one in 64) are not through after kLookSteps
+// nodes.  Of fewer than that a warp of 32 rarely has one that the others wait
+// for: 2M parallel rays from scattered points against a sphere on a large ground
+// (one in 700 comes near it) take 69 us in k_trace_any, 83 in the list's
+// kernel; of rays in all directions one in 16 does, 195 and 145.  One block: every
+// warp of the list's kernel looking by itself cost queries that stay with
+// k_trace_any 5 us; with both kernels launched early this and the kernel that
+// finds nothing to do cost less than the counters' read-back did (2M camera rays
+// on the sphere 106 us then, 109 with every warp looking, now 99).
+constexpr int kRayGroups = 8, kLookSteps = 2, kGoingRays = kRayGroups * 32 / 64;
+template <class SC>
+__global__ void __launch_bounds__(32 * kRayGroups) k_look_any(SC sc, const rt_ray *__restrict__ rays, int32_t n, int *use,
+                                                              int *work)
 {
     const uint32_t e = __float_as_uint(__ldg(reinterpret_cast<const float4 *>(sc.nodes + sc.root)).w);
     // the root's grid is 255 units wide
     const float3 near_ = make_float3(8.0f * __uint_as_float((e & 0xffu) << 23),
                                      8.0f * __uint_as_float(((e >> 8) & 0xffu) << 23),
                                      8.0f * __uint_as_float(((e >> 16) & 0xffu) << 23));
-    int scattered = 0;
-#pragma unroll
-    for (int k = 0; k < kRayGroups; ++k) {
-        const int at = (int)((int64_t)(n - 32) * k / (kRayGroups - 1)) + (int)(threadIdx.x & 31u);
-        const float4 r0 = __ldg(reinterpret_cast<const float4 *>(rays + at));
-        const float dx = r0.x - __shfl_sync(0xffffffffu, r0.x, 0), dy = r0.y - __shfl_sync(0xffffffffu, r0.y, 0),
-                    dz = r0.z - __shfl_sync(0xffffffffu, r0.z, 0);
-        scattered += !__all_sync(0xffffffffu, (int)(fabsf(dx) < near_.x) & (int)(fabsf(dy) < near_.y) &
-                                                  (int)(fabsf(dz) < near_.z));
+    const int group = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31u);
+    const float4 *rp = reinterpret_cast<const float4 *>(rays + ((int64_t)(n - 32) * group / (kRayGroups - 1) + lane));
+    const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
+    const float dx = r0.x - __shfl_sync(0xffffffffu, r0.x, 0), dy = r0.y - __shfl_sync(0xffffffffu, r0.y, 0),
+                dz = r0.z - __shfl_sync(0xffffffffu, r0.z, 0);
+    const bool together = __all_sync(0xffffffffu, (int)(fabsf(dx) < near_.x) & (int)(fabsf(dy) < near_.y) &
+                                                      (int)(fabsf(dz) < near_.z));
+    bool list = 2 * __syncthreads_count(lane == 0 && !together) > kRayGroups;
+    if (list) {
+        uint2 stack[kStackSize];
+        Trav T;
+        trav_begin(T, sc, make_float3(r0.x, r0.y, r0.z), make_float3(r1.x, r1.y, r1.z), r0.w, true);
+        uint32_t status = 0u;   // the query's own kernels tell
+        bool going = true;
+        for (int k = 0; k < kLookSteps && going; ++k)
+            going = !trav_step<false, SC::kWatertight>(T, stack, sc, true, status, nullptr);
+        list = __syncthreads_count(going) >= kGoingRays;
     }
-    return 2 * scattered > kRayGroups;
+    if (threadIdx.x == 0) {
+        *use = list;
+        *work = 0;
+    }
 }
 
 // Any-hit rays in no order.  A warp of 32 of them lasts as long as its longest
 // while the others wait (6.3 lanes an instruction for 2M rays against a 2M
 // triangle terrain); here a lane takes the warp's next ray when eight lanes are
 // idle.  Launched before k_trace_any, which finds the rays claimed or, where
-// the rays are not scattered, all of them left.  2M rays: terrain 760 -> 590 us,
+// k_look_any says so, all of them left.  2M rays: terrain 760 -> 590 us,
 // instances 1085 -> 888, 20k sphere 183 -> 147; parallel ones from scattered
-// points 318 -> 233, 652 -> 434, but 82 -> 97 us against the lone sphere, whose
-// rays end after a few nodes.  Rays of neighbouring lanes that start together
+// points 318 -> 233, 652 -> 434.  Rays of neighbouring lanes that start together
 // lose (camera rays 390 -> 490 us, one point's hemisphere of rays as before), as
 // do closest hits (1358 -> 1440): their lanes no longer meet nodes and triangles
 // at the same time.  Below kListRays to a lane of the grid a warp has too few rays
-// to choose from (500k: 229 -> 210 us, 200k: 122 -> 130).  The look at the rays
-// costs 5 us of a query that stays with k_trace_any.
+// to choose from (500k: 229 -> 210 us, 200k: 122 -> 130).
 constexpr int kListRays = 4;
 template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_any_list(
-    SC sc, const rt_ray *__restrict__ rays, int32_t n, uint8_t *__restrict__ occluded, Counters *ctr)
+    SC sc, const rt_ray *__restrict__ rays, int32_t n, uint8_t *__restrict__ occluded, const int *use,
+    int *work, uint32_t *out_status)
 {
-    if (!rays_scattered(sc, rays, n)) return;
+    earlier_kernels();
+    if (!__ldcg(use)) return;
     int at = 0, end = 0;
     const uint32_t status = traverse_list<true>(
         sc,
         [&](int want, int &base) {
             if (at >= end) {
-                at = warp_claim(&ctr->work, 32);
+                at = warp_claim(work, 32);
                 end = min(at + 32, n);
             }
             base = at;
@@ -98,16 +125,17 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_a
             tmax = r0.w;
         },
         [&](int k, const Trav &T) { occluded[k] = T.occluded ? 1 : 0; });
-    if (status) atomicOr(&ctr->status, status);
+    if (status) atomicOr_system(out_status, status);
 }
 
 template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_any(SC sc, const rt_ray *__restrict__ rays, int32_t n,
-                                                             uint8_t *__restrict__ occluded, Counters *ctr)
+                                                             uint8_t *__restrict__ occluded, int *work, uint32_t *out_status)
 {
+    earlier_kernels();
     uint32_t status = 0;
     for (;;) {
-        const int base = warp_claim(&ctr->work, 32);
+        const int base = warp_claim(work, 32);
         if (base >= n) break;
         const int i = base + (threadIdx.x & 31);
         if (i < n) {
@@ -119,7 +147,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_trace_a
             occluded[i] = occ ? 1 : 0;
         }
     }
-    if (status) atomicOr(&ctr->status, status);
+    if (status) atomicOr_system(out_status, status);
 }
 
 // Few rays: `per` of them (a power of two) to a warp of its own block.  A
@@ -636,14 +664,14 @@ static int blocks_per_sm(K kernel)
     return per_sm;
 }
 
-void launch_trace_closest(const SceneView &sc, const rt_ray *rays, int32_t n, rt_hit *hits, Counters *ctr, int sm_count,
-                          cudaStream_t st)
+void launch_trace_closest(const SceneView &sc, const rt_ray *rays, int32_t n, rt_hit *hits, int *work, uint32_t *status,
+                          int sm_count, cudaStream_t st)
 {
     with_scene(sc, [&](const auto &view) {
         using SC = std::decay_t<decltype(view)>;
         static const int per_sm = blocks_per_sm(k_trace_closest<SC>);
         const int grid = per_sm * sm_count;
-        k_trace_closest<SC><<<grid, kTraceThreads, 0, st>>>(view, rays, n, hits, ctr);
+        k_trace_closest<SC><<<grid, kTraceThreads, 0, st>>>(view, rays, n, hits, work, status);
     });
 }
 
@@ -661,16 +689,30 @@ void launch_trace_few(const SceneView &sc, const rt_ray *rays, int32_t n, void *
 template void launch_trace_few<false>(const SceneView &, const rt_ray *, int32_t, void *, uint32_t *, int, cudaStream_t);
 template void launch_trace_few<true>(const SceneView &, const rt_ray *, int32_t, void *, uint32_t *, int, cudaStream_t);
 
-void launch_trace_any(const SceneView &sc, const rt_ray *rays, int32_t n, uint8_t *occ, Counters *ctr, int sm_count,
-                      cudaStream_t st)
+void launch_trace_any(const SceneView &sc, const rt_ray *rays, int32_t n, uint8_t *occ, int *work, uint32_t *status,
+                      int sm_count, cudaStream_t st)
 {
     with_scene(sc, [&](const auto &view) {
         using SC = std::decay_t<decltype(view)>;
         static const int per_sm = blocks_per_sm(k_trace_any<SC>);
         const int grid = per_sm * sm_count;
-        if (view.nnodes > 0 && n >= kListRays * grid * kTraceThreads)
-            k_trace_any_list<SC><<<grid, kTraceThreads, 0, st>>>(view, rays, n, occ, ctr);
-        k_trace_any<SC><<<grid, kTraceThreads, 0, st>>>(view, rays, n, occ, ctr);
+        cudaLaunchAttribute early;   // launched while the kernel before ends (earlier_kernels)
+        early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        early.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(kTraceThreads);
+        cfg.stream = st;
+        cfg.attrs = &early;
+        if (view.nnodes > 0 && n >= kListRays * grid * kTraceThreads) {
+            const int *use = work + 1;
+            k_look_any<SC><<<1, 32 * kRayGroups, 0, st>>>(view, rays, n, work + 1, work);
+            cfg.numAttrs = 1;
+            cudaLaunchKernelEx(&cfg, k_trace_any_list<SC>, view, rays, n, occ, use, work, status);
+        } else {
+            cudaMemsetAsync(work, 0, sizeof(int), st);
+        }
+        cudaLaunchKernelEx(&cfg, k_trace_any<SC>, view, rays, n, occ, work, status);
     });
 }
 
