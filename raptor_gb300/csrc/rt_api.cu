@@ -161,7 +161,7 @@ SceneView scene_view(const rt_scene *s)
 {
     SceneView v;
     v.nodes = s->d_nodes;
-    v.any_nodes = s->any_ready ? (const WideNode *)s->any.ptr : s->d_nodes;
+    v.any_nodes = s->d_any ? s->d_any : s->d_nodes;
     v.tris = s->d_tris;
     v.shade = s->d_shade;
     v.idx = s->d_idx;
@@ -358,8 +358,8 @@ static void scene_free_geometry(rt_scene *s)
     cudaFree(s->d_nodes); s->d_nodes = nullptr;
     cudaFree(s->d_tris); s->d_tris = nullptr;
     s->temp.release();
-    s->any.release();
-    s->any_ready = s->passing = false;
+    s->d_any = nullptr;
+    s->passing = false;
     s->built = false;
     s->nnodes = s->tri_slots = s->depth = 0;
 }
@@ -443,28 +443,13 @@ static int32_t builder_of(int b)
     return b == RT_BUILDER_LBVH ? kBuilderLbvh : b == RT_BUILDER_HPLOC ? kBuilderHploc : kBuilderPloc;
 }
 
-// The any-hit rays' nodes of a scene that has triangles they pass, after its
-// hierarchy was built (mark) or refitted; without memory for them the rays
-// take the scene's own nodes.
-static void make_any_nodes(rt_scene *s, int32_t nnodes, bool mark)
-{
-    if (!s->passing || nnodes < 1) return;
-    const size_t n = (size_t)nnodes;
-    if (mark && s->any.reserve(n * (sizeof(WideNode) + 2 * sizeof(int32_t))) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    build_any_nodes(s->d_nodes, nnodes, s->d_tris, (WideNode *)s->any.ptr,
-                    (int32_t *)((WideNode *)s->any.ptr + n), mark, s->ctx->stream);
-    s->any_ready = true;
-}
-
 rt_status rt_bvh_build(rt_scene *s, float *build_ms)
 {
     if (!s) return fail(RT_ERR_INVALID_ARG, "rt_bvh_build: NULL scene");
     rt_context *ctx = s->ctx;
     DeviceGuard g(ctx->device);
-    s->built = s->any_ready = false;
+    s->built = false;
+    s->d_any = nullptr;
     s->refit = RefitArrays();
     if (build_ms) *build_ms = 0.f;
     if (s->ntris == 0) {
@@ -475,7 +460,7 @@ rt_status rt_bvh_build(rt_scene *s, float *build_ms)
     const size_t nt = (size_t)s->ntris;
     if (!s->d_nodes) RT_CUDA(cudaMalloc(&s->d_nodes, (nt + 1) * sizeof(WideNode)), "node allocation");
     if (!s->d_tris) RT_CUDA(cudaMalloc(&s->d_tris, nt * sizeof(PackedTri)), "triangle allocation");
-    const size_t tb = build_temp_bytes(s->ntris);
+    const size_t tb = build_temp_bytes(s->ntris, s->passing);
     RT_CUDA(s->temp.reserve(tb), "build scratch allocation");
     BuildInputs in;
     in.ntris = s->ntris;
@@ -490,6 +475,7 @@ rt_status rt_bvh_build(rt_scene *s, float *build_ms)
     in.host_scratch = ctx->h_scratch;
     in.builder = builder_of(ctx->builder);
     in.morton_bits = ctx->morton_bits;
+    in.passing = s->passing;
     RT_CUDA(cudaEventRecord(ctx->ev0, ctx->stream), "event record");
     const BuildResult R = build_wide_bvh(in, s->temp.ptr, s->temp.cap, ctx->stream);
     if (R.status != 0) {
@@ -498,7 +484,6 @@ rt_status rt_bvh_build(rt_scene *s, float *build_ms)
         if (R.status == RT_ERR_STACK_OVERFLOW) return fail(RT_ERR_STACK_OVERFLOW, "bvh build: tree deeper than the traversal stack");
         return fail(R.status, "bvh build failed");
     }
-    make_any_nodes(s, R.nodes, true);
     RT_CUDA(cudaEventRecord(ctx->ev1, ctx->stream), "event record");
     RT_CUDA(cudaEventSynchronize(ctx->ev1), "event synchronize");
     RT_CUDA(cudaGetLastError(), "bvh build kernels");
@@ -508,6 +493,7 @@ rt_status rt_bvh_build(rt_scene *s, float *build_ms)
     s->tri_slots = R.tri_slots;
     s->depth = R.depth;
     s->refit = R.refit;
+    s->d_any = R.any_nodes;
     s->built = true;
     return RT_OK;
 }
@@ -529,14 +515,13 @@ rt_status rt_scene_refit_vertices(rt_scene *s, const float *verts, int32_t nvert
     }
     s->built = false;
     RT_CUDA(cudaEventRecord(ctx->ev0, ctx->stream), "event record");
-    const int32_t st = refit_wide_bvh(s->refit, s->d_verts, s->d_idx, s->d_shade, s->d_nodes, s->d_tris,
-                                      ctx->h_scratch, ctx->stream);
+    const int32_t st = refit_wide_bvh(s->refit, s->d_verts, s->d_idx, s->d_shade, s->d_nodes, s->d_any,
+                                      s->d_tris, ctx->h_scratch, ctx->stream);
     if (st != 0) {
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "refit");
         return fail(st, "rt_scene_refit_vertices: refit failed");
     }
-    if (s->any_ready) make_any_nodes(s, s->nnodes, false);
     RT_CUDA(cudaEventRecord(ctx->ev1, ctx->stream), "event record");
     RT_CUDA(cudaEventSynchronize(ctx->ev1), "event synchronize");
     if (refit_ms) cudaEventElapsedTime(refit_ms, ctx->ev0, ctx->ev1);

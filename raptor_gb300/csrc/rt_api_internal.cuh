@@ -76,8 +76,7 @@ struct rt_scene {
     int32_t nnodes = 0, tri_slots = 0, depth = 0;
     bool built = false;
     bool passing = false;                 // some triangles stop no any-hit ray (light, transparent)
-    rtc::DevBuf any;                      // their scenes: the any-hit rays' nodes, then two ints per node
-    bool any_ready = false;
+    rtc::WideNode *d_any = nullptr;       // their scenes' nodes for any-hit rays, behind d_nodes' (nullptr: d_nodes)
     rtc::DevBuf temp;
     rtc::RefitArrays refit;   // the last build's tree, for rt_scene_refit_vertices
 };

@@ -415,9 +415,11 @@ static_assert(kBuildWords <= 64, "the words are read back into BuildInputs::host
 // bounds per segment, a single segment's triangle range.  One launch for what
 // took three clears and three copies of a few bytes from pageable memory
 // (with one copy back instead of three: 50k triangles 0.379 -> 0.367 ms).
+// links (nullable): of the root, which has no parent.
 __global__ void k_build_init(int32_t *__restrict__ words, int *__restrict__ cbounds, int32_t *__restrict__ seg_first,
-                             int32_t n, int32_t nseg)
+                             int32_t n, int32_t nseg, int2 *__restrict__ links)
 {
+    if (links && threadIdx.x == 0) links[0] = make_int2(-1, 0);
     for (int i = threadIdx.x; i < kBuildWords; i += blockDim.x) words[i] = i == 0 ? nseg : 0;
     for (int i = threadIdx.x; i < 6 * nseg; i += blockDim.x) cbounds[i] = i % 6 < 3 ? 0x7fffffff : (int)0x80000000;
     if (nseg == 1 && threadIdx.x < 2) seg_first[threadIdx.x] = threadIdx.x ? n : 0;
@@ -1194,6 +1196,8 @@ __device__ __forceinline__ int grid_exponent(float extent)
     return min(max(e, 1), 253);
 }
 
+constexpr uint32_t kPassing = RT_TRI_LIGHT | RT_TRI_TRANSPARENT;
+
 struct BuildArgs {
     int32_t n;
     const int32_t *left, *right;
@@ -1213,6 +1217,8 @@ struct BuildArgs {
     const int2 *tasks_in;         // (binary ref, wide node index)
     int2 *tasks_out;
     int32_t max_nodes;
+    int2 *links;                  // per wide node: its parent; a bit per leaf slot with a triangle that stops any-hit
+                                  // rays, and kAnyMark (nullptr: not asked for)
 };
 
 // Wide nodes and triangle slots allocated together: counters[0] and
@@ -1260,8 +1266,10 @@ __device__ __forceinline__ bool leaf_refs(const BuildArgs &A, int32_t ref, int32
 // The packed triangles of leaves lv[0 .. nlv) at tris[at ..]: the caller's
 // ids, then their indices and flags, then the vertices, each step's loads
 // issued together.
-__device__ __forceinline__ void emit_leaf_tris(const BuildArgs &A, const int32_t *lv, int nlv, int32_t at)
+// Returns whether one of them stops any-hit rays.
+__device__ __forceinline__ bool emit_leaf_tris(const BuildArgs &A, const int32_t *lv, int nlv, int32_t at)
 {
+    bool stops = false;
     int32_t id[kMaxLeafTris];
     int3 t[kMaxLeafTris];
     uint32_t fl[kMaxLeafTris];
@@ -1273,6 +1281,7 @@ __device__ __forceinline__ void emit_leaf_tris(const BuildArgs &A, const int32_t
         if (j < nlv) {
             t[j] = A.idx[id[j]];
             fl[j] = A.flags ? A.flags[id[j]] : 0u;
+            stops |= (fl[j] & kPassing) == 0u;
         }
 #pragma unroll
     for (int j = 0; j < kMaxLeafTris; ++j)
@@ -1284,6 +1293,7 @@ __device__ __forceinline__ void emit_leaf_tris(const BuildArgs &A, const int32_t
             P.w2 = make_float4(v[3 * t[j].z + 2], __int_as_float(id[j]), __uint_as_float(fl[j]), 0.f);
             A.tris[at + j] = P;
         }
+    return stops;
 }
 
 // The children of wide node `node` by the surface-area decisions: its 8
@@ -1463,6 +1473,7 @@ __device__ __forceinline__ void collapse_task(const BuildArgs &A, const int2 tas
             W.meta[s] = 0x80;
             const int slot = atomicAdd(A.next_count, 1);
             A.tasks_out[slot] = make_int2(ch[k], child_base + int_k);
+            if (A.links) A.links[child_base + int_k] = make_int2(wide, 0);
             ++int_k;
         } else {
             const int c = cnt[k];
@@ -1470,7 +1481,7 @@ __device__ __forceinline__ void collapse_task(const BuildArgs &A, const int2 tas
             int32_t lv[kMaxLeafTris];
             int nlv = 0;
             if (!leaf_refs(A, ch[k], lv, nlv) || nlv != c) { atomicExch(&A.counters[3], 1); return; }
-            emit_leaf_tris(A, lv, nlv, tri_base + tri_off);
+            if (emit_leaf_tris(A, lv, nlv, tri_base + tri_off) && A.links) atomicOr(&A.links[wide].y, 1 << s);
             tri_off += c;
         }
     }
@@ -1716,6 +1727,7 @@ __device__ __forceinline__ void collapse_task_group(const BuildArgs &A, const in
     if (internal) {
         const int rank = __popc(imask & ((1u << myslot) - 1u));
         A.tasks_out[next + rank] = make_int2(ref, child_base + rank);
+        if (A.links) A.links[child_base + rank] = make_int2(task.y, 0);
     } else if (active) {
         int32_t lv[kMaxLeafTris];
         int nlv = 0;
@@ -1723,7 +1735,8 @@ __device__ __forceinline__ void collapse_task_group(const BuildArgs &A, const in
             atomicExch(&A.counters[3], 1);
             return;
         }
-        emit_leaf_tris(A, lv, nlv, tri_base + tri_off);
+        if (emit_leaf_tris(A, lv, nlv, tri_base + tri_off) && A.links)
+            atomicOr(&A.links[task.y].y, 1 << myslot);
     }
 }
 
@@ -1783,9 +1796,67 @@ __global__ void k_collapse_level(BuildArgs A)
         collapse_task(A, A.tasks_in[ti]);
 }
 
+// Any-hit rays in scenes with triangles that stop none of them spend most of
+// their node tests on such triangles: a ray that leaves a glass sphere meets
+// the sphere's own nodes first.  They take a copy of the nodes in which
+// children with nothing else below are empty; it costs no instruction in the
+// traversal (another node pointer), and its nodes lie behind the scene's own in
+// their array, which has room for a node a triangle.  512x512 glass frames: ray
+// trees 649 -> 436 us, diffuse sets 18.65 -> 12.04 ms.  The collapse, which reads
+// the triangles' flags, notes the leaf slots that stop rays and the parents; two
+// short launches are left to a build, a refit writes the copy beside the nodes.
+// (Three launches that looked for both and one after a refit, in a buffer of
+// their own: 41k triangles built in 417 us, refitted in 115; now 402 and 102,
+// 413 and 101 without any of it.)
+
+// Do any of n triangles stop no any-hit ray?
+__global__ void k_find_passing(const uint32_t *__restrict__ flags, int32_t n, int32_t *__restrict__ out)
+{
+    uint32_t f = 0u;
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) f |= flags[i];
+    if (__any_sync(0xffffffffu, (f & kPassing) != 0u) && (threadIdx.x & 31u) == 0u) *out = 1;
+}
+
+// A node with such a leaf marks itself and all above it, up to the first that is
+// marked already.
+constexpr int32_t kAnyMark = 1 << 8;
+__global__ void k_any_marks(int2 *__restrict__ links, int32_t n)
+{
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    int32_t at = i < n && (links[i].y & 0xff) != 0 ? i : -1;
+    for (int step = 0; at >= 0 && step <= kMaxDepth && !(atomicOr(&links[at].y, kAnyMark) & kAnyMark); ++step)
+        at = links[at].x;
+}
+
+__global__ void __launch_bounds__(128) k_any_nodes(const WideNode *__restrict__ nodes, int32_t n,
+                                                   const int2 *__restrict__ links, WideNode *__restrict__ out)
+{
+    const int32_t i = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 3);
+    const int lane = threadIdx.x & 7;   // a slot, and a 16-byte word of the node
+    bool keep = false;
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
+    if (i < n) {
+        if (lane < 5) w = reinterpret_cast<const uint4 *>(nodes + i)[lane];
+        const uint32_t imask = nodes[i].imask;
+        if ((imask >> lane) & 1u) {
+            const int32_t child = (int32_t)nodes[i].child_base + __popc(imask & ((1u << lane) - 1u));
+            keep = child < n && (links[child].y & kAnyMark) != 0;
+        } else {
+            keep = (links[i].y >> lane) & 1;
+        }
+    }
+    const uint32_t kept = (__ballot_sync(0xffffffffu, keep) >> (threadIdx.x & 24u)) & 0xffu;
+    if (i >= n || lane >= 5) return;
+    if (lane == 1) {   // the meta bytes: 0 where nothing is kept
+        w.z &= (((kept & 15u) * 0x00204081u) & 0x01010101u) * 0xffu;
+        w.w &= (((kept >> 4) * 0x00204081u) & 0x01010101u) * 0xffu;
+    }
+    reinterpret_cast<uint4 *>(out + i)[lane] = w;
+}
+
 }  // namespace
 
-size_t build_temp_bytes(int32_t n)
+size_t build_temp_bytes(int32_t n, bool passing)
 {
     size_t cub_bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, (const uint64_t *)nullptr, (uint64_t *)nullptr,
@@ -1807,7 +1878,8 @@ size_t build_temp_bytes(int32_t n)
     b += (nn / kPlocBlock + 2) * sizeof(int2) + kStWords * sizeof(int32_t);
     b += 16 * sizeof(int32_t) + 2 * nn * sizeof(int2);   // counters, root tasks
     b += (6 + 1) * (size_t)kMaxSegments * sizeof(int) + 1024;
-    b += cub_bytes + 16 * 256;
+    if (passing) b += (nn + 1) * sizeof(int2);   // the wide nodes' links
+    b += cub_bytes + 17 * 256;
     return b;
 }
 
@@ -1875,6 +1947,7 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
     if (ploc) pstate = counters + kStateWord;
     int *cbounds = (int *)carve(p, 6 * (size_t)nseg * sizeof(int));
     int32_t *seg_first = (int32_t *)carve(p, ((size_t)nseg + 1) * sizeof(int32_t));
+    int2 *links = in.passing ? (int2 *)carve(p, (nn + 1) * sizeof(int2)) : nullptr;
     size_t cub_bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, keys, keys2, vals, vals2, (int)nn, 0, 64, st);
     void *cub_temp = carve(p, cub_bytes);
@@ -1882,7 +1955,7 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
 
     // segment offsets (sorted positions of each segment = its triangle range)
     int32_t *h_cnt = in.host_scratch;   // pinned
-    k_build_init<<<1, 256, 0, st>>>(counters, cbounds, seg_first, n, nseg);
+    k_build_init<<<1, 256, 0, st>>>(counters, cbounds, seg_first, n, nseg, links);
     if (nseg > 1)
         cudaMemcpyAsync(seg_first, in.seg_first, ((size_t)nseg + 1) * sizeof(int32_t), cudaMemcpyDefault, st);
     int sb = 0;
@@ -1970,6 +2043,7 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
     A.verts = in.verts; A.idx = in.idx; A.flags = in.flags;
     A.nodes = in.nodes; A.tris = in.tris; A.counters = counters;
     A.max_nodes = in.max_nodes;
+    A.links = links;
     int depth = 0;
     // levels back to back in groups of kCollapseGroup (a level past the last
     // one finds no tasks), one read-back per group: most trees end within
@@ -2015,6 +2089,11 @@ BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes,
     K.blo = blo; K.bhi = bhi; K.llo = llo; K.lhi = lhi; K.ilo = ilo; K.ihi = ihi; K.flags = rflags;
     K.slot_ref = slot_ref; K.err = counters + 3;
     K.ntris = n; K.nnodes = R.nodes; K.tri_slots = R.tri_slots;
+    if (links && R.nodes <= in.max_nodes - R.nodes) {
+        R.any_nodes = in.nodes + R.nodes;
+        k_any_marks<<<(R.nodes + 127) / 128, 128, 0, st>>>(links, R.nodes);
+        k_any_nodes<<<(R.nodes + 15) / 16, 128, 0, st>>>(in.nodes, R.nodes, links, R.any_nodes);
+    }
     return R;
 }
 
@@ -2041,8 +2120,10 @@ __global__ void k_refit_tris(const float *__restrict__ verts, const int3 *__rest
 }
 
 // Refit, per wide node: new quantisation frame from its children's refitted
-// boxes, every occupied slot re-quantised; links and triangle groups kept.
-__global__ void k_requant(WideNode *__restrict__ nodes, int32_t nnodes, const int32_t *__restrict__ slot_ref,
+// boxes, every occupied slot re-quantised; links and triangle groups kept.  any
+// (nullable): the any-hit rays' copy, which keeps its own meta bytes.
+__global__ void k_requant(WideNode *__restrict__ nodes, int32_t nnodes, WideNode *__restrict__ any,
+                          const int32_t *__restrict__ slot_ref,
                           const float4 *__restrict__ llo, const float4 *__restrict__ lhi,
                           const float4 *__restrict__ ilo, const float4 *__restrict__ ihi)
 {
@@ -2079,6 +2160,10 @@ __global__ void k_requant(WideNode *__restrict__ nodes, int32_t nnodes, const in
         W.qz[s] = quant_planes(lo[s].z, hi[s].z, pz, iz);
     }
     nodes[w] = W;
+    if (any) {
+        *reinterpret_cast<uint2 *>(W.meta) = *reinterpret_cast<const uint2 *>(any[w].meta);
+        any[w] = W;
+    }
 }
 
 // Refit, per packed triangle (leaf order): the new vertices, id and flags kept.
@@ -2097,99 +2182,14 @@ __global__ void k_repack(PackedTri *__restrict__ tris, int32_t nslots, const flo
 
 }  // namespace
 
-namespace {
-
-constexpr uint32_t kPassing = RT_TRI_LIGHT | RT_TRI_TRANSPARENT;
-
-// Any-hit rays in scenes with triangles that stop none of them spend most of
-// their node tests on such triangles: a ray that leaves a glass sphere meets
-// the sphere's own nodes first.  They take a copy of the nodes in which
-// children with nothing else below are empty; it costs no instruction in the
-// traversal (another node pointer), 88 bytes a node and three short kernels a
-// build, only in scenes that have such triangles.  512x512 glass frames: ray
-// trees 649 -> 436 us, diffuse sets 18.65 -> 12.04 ms.
-
-// Do any of n triangles stop no any-hit ray?
-__global__ void k_find_passing(const uint32_t *__restrict__ flags, int32_t n, int32_t *__restrict__ out)
-{
-    uint32_t f = 0u;
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) f |= flags[i];
-    if (__any_sync(0xffffffffu, (f & kPassing) != 0u) && (threadIdx.x & 31u) == 0u) *out = 1;
-}
-
-__device__ __forceinline__ bool leaf_stops(const WideNode &N, int s, const PackedTri *__restrict__ tris)
-{
-    const PackedTri *t = tris + N.tri_base + (N.meta[s] & 31u);
-    for (int k = 0; k < (N.meta[s] >> 5); ++k)
-        if ((__float_as_uint(t[k].w2.z) & kPassing) == 0u) return true;
-    return false;
-}
-
-__global__ void k_any_parents(const WideNode *__restrict__ nodes, int32_t n, int32_t *__restrict__ parent,
-                              int32_t *__restrict__ stops)
-{
-    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int32_t first = (int32_t)nodes[i].child_base, kids = __popc(nodes[i].imask);
-    for (int32_t c = first; c < first + kids; ++c)
-        if (c < n) parent[c] = i;
-    if (i == 0) parent[0] = -1;
-    stops[i] = 0;
-}
-
-// A node with a triangle that stops rays marks itself and the nodes above it,
-// up to the first that is marked already.
-__global__ void k_any_marks(const WideNode *__restrict__ nodes, int32_t n, const PackedTri *__restrict__ tris,
-                            const int32_t *__restrict__ parent, int32_t *__restrict__ stops)
-{
-    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const WideNode N = nodes[i];
-    bool stop = false;
-    for (int s = 0; s < 8 && !stop; ++s) stop = N.meta[s] != 0 && N.meta[s] != 0x80u && leaf_stops(N, s, tris);
-    int32_t at = stop ? i : -1;
-    for (int step = 0; at >= 0 && step < kRefitMaxDepth && atomicExch(stops + at, 1) == 0; ++step) at = parent[at];
-}
-
-__global__ void k_any_nodes(const WideNode *__restrict__ nodes, int32_t n, const PackedTri *__restrict__ tris,
-                            const int32_t *__restrict__ stops, WideNode *__restrict__ out)
-{
-    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    WideNode N = nodes[i];
-    int32_t child = (int32_t)N.child_base;
-    for (int s = 0; s < 8; ++s) {
-        if ((N.imask >> s) & 1u) {
-            if (child >= n || !stops[child]) N.meta[s] = 0;
-            ++child;
-        } else if (N.meta[s] != 0 && !leaf_stops(N, s, tris)) {
-            N.meta[s] = 0;
-        }
-    }
-    out[i] = N;
-}
-
-}  // namespace
-
 void find_passing(const uint32_t *flags, int32_t n, int32_t *out, cudaStream_t st)
 {
     cudaMemsetAsync(out, 0, sizeof(int32_t), st);
     if (n > 0) k_find_passing<<<std::min((n + 255) / 256, 1024), 256, 0, st>>>(flags, n, out);
 }
 
-void build_any_nodes(const WideNode *nodes, int32_t n, const PackedTri *tris, WideNode *any_nodes, int32_t *scratch,
-                     bool mark, cudaStream_t st)
-{
-    const int g = (n + 127) / 128;
-    if (mark) {
-        k_any_parents<<<g, 128, 0, st>>>(nodes, n, scratch, scratch + n);
-        k_any_marks<<<g, 128, 0, st>>>(nodes, n, tris, scratch, scratch + n);
-    }
-    k_any_nodes<<<g, 128, 0, st>>>(nodes, n, tris, scratch + n, any_nodes);
-}
-
 int32_t refit_wide_bvh(const RefitArrays &K, const float *verts, const int3 *idx, ShadeTri *shade, WideNode *nodes,
-                       PackedTri *tris, int32_t *host_scratch, cudaStream_t st)
+                       WideNode *any_nodes, PackedTri *tris, int32_t *host_scratch, cudaStream_t st)
 {
     if (!K.valid) return -4;
     const int threads = 256;
@@ -2201,7 +2201,7 @@ int32_t refit_wide_bvh(const RefitArrays &K, const float *verts, const int3 *idx
     cudaMemsetAsync(K.flags, 0, (size_t)n * sizeof(int32_t), st);
     k_refit<<<g, threads, 0, st>>>(n, K.left, K.right, K.parent, K.leaf_parent, K.llo, K.lhi, K.ilo, K.ihi, K.flags,
                                    nullptr, nullptr, nullptr, K.err);
-    k_requant<<<(K.nnodes + 127) / 128, 128, 0, st>>>(nodes, K.nnodes, K.slot_ref, K.llo, K.lhi, K.ilo, K.ihi);
+    k_requant<<<(K.nnodes + 127) / 128, 128, 0, st>>>(nodes, K.nnodes, any_nodes, K.slot_ref, K.llo, K.lhi, K.ilo, K.ihi);
     k_repack<<<(K.tri_slots + 255) / 256, 256, 0, st>>>(tris, K.tri_slots, verts, idx);
     cudaMemcpyAsync(host_scratch, K.err, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return -2;

@@ -27,6 +27,10 @@ struct BuildInputs {
     int32_t nseg = 1;
     const int32_t *seg_of_tri = nullptr;
     const int32_t *seg_first = nullptr;
+    // a single scene has triangles that stop no any-hit ray (light and
+    // transparent ones): the build also makes a copy of the nodes for those
+    // rays, without the children that hold nothing else
+    bool passing = false;
 };
 
 // Device arrays a build leaves in its scratch so that the same tree can be
@@ -49,30 +53,26 @@ struct BuildResult {
     int32_t nodes = 0;
     int32_t tri_slots = 0;
     int32_t depth = 0;
+    WideNode *any_nodes = nullptr;   // the any-hit rays' copy, behind the nodes (nullptr: none, they take the nodes)
     RefitArrays refit;
 };
 
 // Device scratch needed by build_wide_bvh for n triangles.
-size_t build_temp_bytes(int32_t n);
+size_t build_temp_bytes(int32_t n, bool passing = false);
 
 // Build on stream st; synchronises st once at the end (and, for PLOC,
 // once per kPlocGroup clustering iterations).
 BuildResult build_wide_bvh(const BuildInputs &in, void *temp, size_t temp_bytes, cudaStream_t st);
 
-// Refit the tree of a previous build (arrays K, still in its scratch) to
-// moved vertices: shading records, boxes bottom-up, every wide node
-// re-quantised, packed triangles rewritten; topology kept.  0 or an
-// rt_status code.  Synchronises st once.
-// The any-hit rays' copy of a scene's nodes (any_nodes), for scenes with
-// triangles that stop none of them (light and transparent ones): children
-// with nothing else below are left out.  mark: n nodes' marks are made again
-// (a new hierarchy), else kept (a refit).  scratch: 2 n ints.
-void build_any_nodes(const WideNode *nodes, int32_t n, const PackedTri *tris, WideNode *any_nodes, int32_t *scratch,
-                     bool mark, cudaStream_t st);
 // Sets *out to 1 where one of n triangles' flags is a light's or transparent.
 void find_passing(const uint32_t *flags, int32_t n, int32_t *out, cudaStream_t st);
 
+// Refit the tree of a previous build (arrays K, still in its scratch) to
+// moved vertices: shading records, boxes bottom-up, every wide node
+// re-quantised (in the any-hit rays' copy, any_nodes, too, where the build made
+// one), packed triangles rewritten; topology kept.  0 or an rt_status code.
+// Synchronises st once.
 int32_t refit_wide_bvh(const RefitArrays &K, const float *verts, const int3 *idx, ShadeTri *shade, WideNode *nodes,
-                       PackedTri *tris, int32_t *host_scratch, cudaStream_t st);
+                       WideNode *any_nodes, PackedTri *tris, int32_t *host_scratch, cudaStream_t st);
 
 }  // namespace rtc
