@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(256, RT_RENDER_MIN_BLOCKS / 2) k_render_batche
                 if (__ldg(&jobs[mid].items_begin) <= item0) lo = mid; else hi = mid - 1;
             }
             const BatchJob &J = jobs[lo];
-            const SC &sc = static_cast<const SC &>(J.sc);
+            const SC &sc = J.sc;
             int x, y;
             tile_pixel<TW>(item0 - J.items_begin + (threadIdx.x & 31), J.tiles_x, x, y);
             const bool live = (x < J.cam.xres) && (y < J.cam.yres);
@@ -260,7 +260,7 @@ rt_status make_graph(rt_batch *b)
         return set_cuda_error(e, "graph capture streams");
     }
     // every job's scene carries the intersector set when the jobs were
-    with_scene(b->h_jobs.empty() ? SceneView{} : b->h_jobs[0].sc, [&](const auto &view) {
+    with_scene(b->h_jobs.empty() ? SceneView{} : static_cast<const SceneView &>(b->h_jobs[0].sc), [&](const auto &view) {
         using SC = std::decay_t<decltype(view)>;
         const int grid = batch_grid<SC>(b);
         e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);

@@ -33,7 +33,7 @@ FrameJob single_job(const SceneView &sc, const CameraView &cam, const MaterialVi
 {
     FrameJob J;
     memset(&J, 0, sizeof(J));
-    J.sc = sc;
+    static_cast<SceneView &>(J.sc) = sc;
     J.cam = cam;
     J.mat = mat;
     J.rgb = rgb;

@@ -24,7 +24,7 @@ constexpr int kWaveBatch = 16;
 // One frame of work: a scene, a camera, lights or AO, outputs, and the range
 // of work items (32-pixel tiles) it owns in the queue.
 struct FrameJob {
-    SceneView sc;
+    WatertightView sc;         // a kernel takes it as its scene type, this or SceneView
     CameraView cam;
     MaterialView mat;
     LightView lights[RT_MAX_LIGHTS];
