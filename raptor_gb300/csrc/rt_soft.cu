@@ -184,7 +184,7 @@ struct SoftState {
     // (colour, material; first item, set sizes), the items (its sets' rays),
     // their subtrees' colours, the item count
     DevBuf root_c, root_sets, items, item_c, nitems;
-    DevBuf node_sets, node_hits, node_over;   // the nodes' children, hit nodes, nodes walked whole
+    DevBuf nodes, node_sets, node_hits, node_over;   // nodes below them, their children, hit nodes, nodes walked whole
     int64_t item_cap = 0;
     // The stream's words on the device: the window a frame reads from and one
     // for the words that follow the frame's slice, where the next frame of an
@@ -230,6 +230,7 @@ void soft_release(rt_context *ctx)
     S.items.release();
     S.item_c.release();
     S.nitems.release();
+    S.nodes.release();
     S.node_sets.release();
     S.node_hits.release();
     S.node_over.release();
@@ -1238,9 +1239,15 @@ __global__ void __launch_bounds__(kTraceThreads, RT_DIST_MIN_BLOCKS) k_dist_root
 
 // The items of a frame: nr of the reflection sets from entry 0, nt of the
 // refraction sets from entry cap, walked as [0, nr) rounded up to a warp and
-// then [0, nt).  Entries 2 cap .. 2 cap + pool hold the nodes below them.
+// then [0, nt).  Entries 2 cap .. 2 cap + pool are the nodes below them.
 struct DistLists {
     int32_t nr, nt, cap, pool;
+    DistItem *items, *nodes;
+
+    __device__ __forceinline__ DistItem *item(int slot) const
+    {
+        return slot < 2 * cap ? items + slot : nodes + (slot - 2 * cap);
+    }
 
     __host__ __device__ __forceinline__ int count() const { return ((nr + 31) & ~31) + nt; }
     __device__ __forceinline__ int slot(int v) const   // -1: none
@@ -1295,7 +1302,7 @@ constexpr float kDistNoNode = -1.0f;   // the power of an entry without a node
 template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_DIST_NODE_MIN_BLOCKS) k_dist_node(
     SC sc, CameraView cam, LightSet lights, MaterialTable table, DistLights dl, DistParams dp,
-    const float *__restrict__ lut, DistItem *__restrict__ items, DistLists lists, int v0, int v1, int level, int last,
+    const float *__restrict__ lut, DistLists lists, int v0, int v1, int level, int last,
     int4 *__restrict__ sets, float4 *__restrict__ item_c, DistHit *__restrict__ hits, int32_t *__restrict__ over,
     DistCounts *dc, Counters *ctr)
 {
@@ -1317,7 +1324,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_DIST_NODE_MIN_BLOCKS) k_dist
         bool on = slot >= 0;
         uint32_t pix = 0;
         if (on) {
-            const DistItem it = items[slot];
+            const DistItem it = *lists.item(slot);
             f.o = make_float3(it.o_magn.x, it.o_magn.y, it.o_magn.z);
             f.magn = it.o_magn.w;
             f.d = make_float3(it.d_level.x, it.d_level.y, it.d_level.z);
@@ -1384,11 +1391,11 @@ __global__ void __launch_bounds__(kTraceThreads, RT_DIST_NODE_MIN_BLOCKS) k_dist
                     it.o_magn = make_float4(C.o.x, C.o.y, C.o.z, C.magn);
                     it.d_level = make_float4(C.d.x, C.d.y, C.d.z, __int_as_float(C.level));
                     it.node = make_ulonglong2(C.node, (unsigned long long)pix);
-                    items[pool0 + (size_t)child + j] = it;
+                    lists.nodes[child + j] = it;
                 }
             } else {
                 for (int64_t j = child; j < lists.pool; ++j)
-                    items[pool0 + (size_t)j].o_magn = make_float4(0.f, 0.f, 0.f, kDistNoNode);
+                    lists.nodes[j].o_magn = make_float4(0.f, 0.f, 0.f, kDistNoNode);
                 over[atomicAdd(&dc->over, 1)] = slot;
             }
         }
@@ -1423,8 +1430,8 @@ __global__ void __launch_bounds__(kTraceThreads, RT_DIST_NODE_MIN_BLOCKS) k_dist
 template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_DIST_LIGHTS_MIN_BLOCKS) k_dist_lights(
     SC sc, LightSet lights, MaterialTable table, DistLights dl, DistParams dp, const int4 *__restrict__ area,
-    const float *__restrict__ verts, const float *__restrict__ lut, const DistItem *__restrict__ items,
-    const DistHit *__restrict__ hits, float4 *__restrict__ item_c, DistCounts *dc, Counters *ctr)
+    const float *__restrict__ verts, const float *__restrict__ lut, DistLists lists, const DistHit *__restrict__ hits,
+    float4 *__restrict__ item_c, DistCounts *dc, Counters *ctr)
 {
     struct Hit {
         uint64_t node;
@@ -1440,7 +1447,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_DIST_LIGHTS_MIN_BLOCKS) k_di
         const bool on = base + (int)lane < n;
         const DistHit H = hits[on ? base + (int)lane : base];
         const int slot = __float_as_int(H.start_slot.w);
-        const DistItem it = items[slot];
+        const DistItem it = *lists.item(slot);
         const float3 start = make_float3(H.start_slot.x, H.start_slot.y, H.start_slot.z);
         const float3 kd = make_float3(H.kd_mat.x, H.kd_mat.y, H.kd_mat.z);
         const float3 sn = make_float3(H.sn.x, H.sn.y, H.sn.z);
@@ -1528,8 +1535,8 @@ __global__ void k_dist_gather(MaterialTable table, DistLists lists, int v0, int 
 template <class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_DIST_SUB_MIN_BLOCKS) k_dist_sub(
     SC sc, CameraView cam, LightSet lights, MaterialTable table, DistLights dl, DistParams dp,
-    const int4 *__restrict__ area, const float *__restrict__ verts, const float *__restrict__ lut,
-    const DistItem *__restrict__ items, DistLists lists, const int32_t *__restrict__ list,
+    const int4 *__restrict__ area, const float *__restrict__ verts, const float *__restrict__ lut, DistLists lists,
+    const int32_t *__restrict__ list,
     const int32_t *__restrict__ nlist, int32_t *work, float4 *__restrict__ item_c, Counters *ctr)
 {
     DistFrame F[kDistDepth];
@@ -1543,7 +1550,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_DIST_SUB_MIN_BLOCKS) k_dist_
         const int i = list ? (v < n ? list[v] : -1) : lists.slot(v);
         uint32_t nsec = 0, drawn = 0;
         if (i >= 0) {
-            const DistItem it = items[i];
+            const DistItem it = *lists.item(i);
             F[0].o = make_float3(it.o_magn.x, it.o_magn.y, it.o_magn.z);
             F[0].magn = it.o_magn.w;
             F[0].d = make_float3(it.d_level.x, it.d_level.y, it.d_level.z);
@@ -2207,8 +2214,12 @@ rt_status stream_finish(SoftState &S)
 }
 
 // The subtrees of a frame's items (on the device already): a piece of at most
-// kDistPiece items at a time, level by level, the nodes below them in a pool
-// of up to kDistPoolPerItem for each.
+// kDistPiece items at a time, level by level, the nodes below them in a pool of
+// one for each item and one for each ray of a set at an item, at most
+// kDistPoolPerItem (frames of the glass scene make 0.92 an item with sets of 1 or
+// 4 rays, 3.7 with 16): 132 bytes a node, the items' colours and sets and a
+// piece's hits beside them.  They take at most half of the device's free memory;
+// without room for all of them the items are walked whole.
 constexpr int32_t kDistPiece = 1 << 22;
 constexpr int32_t kDistPoolPerItem = 4;
 
@@ -2218,17 +2229,34 @@ rt_status trace_items(SoftState &S, rt_scene *s, const CameraView &cv, const Lig
 {
     const int32_t n = lists.count(), piece = std::min(n, kDistPiece);
     DistCounts *dc = (DistCounts *)((int32_t *)S.nitems.ptr + 2);
-    DistItem *items = (DistItem *)S.items.ptr;
-    float4 *item_c = (float4 *)S.item_c.ptr;
-    const size_t entries = 2 * (size_t)lists.cap + (size_t)lists.pool;
-    const size_t nodes = (size_t)piece + (size_t)lists.pool;   // of a piece, at most
+    lists.items = (DistItem *)S.items.ptr;
+    constexpr size_t kNode = sizeof(DistItem) + sizeof(float4) + sizeof(int4) + sizeof(DistHit) + sizeof(int32_t);
+    const int64_t per_item = std::min(1 + std::max(dp.diffuse >> 2, 1), kDistPoolPerItem);
+    int64_t pool = levels < 2 ? 0 : std::min(per_item * piece, ((int64_t)1 << 31) - 1 - 2 * (int64_t)lists.cap);
+    const size_t held = S.nodes.cap + S.item_c.cap + S.node_sets.cap + S.node_hits.cap + S.node_over.cap;
+    if ((size_t)pool * kNode > held) {   // more than these buffers were ever asked for, maybe
+        size_t free_b = 0, all_b = 0;
+        if (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess) free_b = 0;
+        pool = std::min(pool, (int64_t)((free_b + held) / 2 / (kNode + kNode / 4)));
+    }
+    lists.pool = (int32_t)pool;
+    const size_t entries = 2 * (size_t)lists.cap + (size_t)pool;
+    const size_t nodes = (size_t)piece + (size_t)pool;   // of a piece, at most
     const int4 *area = (const int4 *)S.area.ptr;
     const float *lut = (const float *)S.lut.ptr;
-    // without room for the lists the items are walked whole
-    const bool walk = S.node_sets.reserve(entries * sizeof(int4)) != cudaSuccess ||
+    const bool walk = S.nodes.reserve((size_t)pool * sizeof(DistItem)) != cudaSuccess ||
+                      S.item_c.reserve(entries * sizeof(float4)) != cudaSuccess ||
+                      S.node_sets.reserve(entries * sizeof(int4)) != cudaSuccess ||
                       S.node_hits.reserve(nodes * sizeof(DistHit)) != cudaSuccess ||
                       S.node_over.reserve(nodes * sizeof(int32_t)) != cudaSuccess;
-    if (walk) cudaGetLastError();
+    if (walk) {
+        cudaGetLastError();
+        for (DevBuf *b : {&S.nodes, &S.item_c, &S.node_sets, &S.node_hits, &S.node_over}) b->release();
+        lists.pool = 0;
+        RT_CUDA_S(S.item_c.reserve(2 * (size_t)lists.cap * sizeof(float4)), "item colour allocation");
+    }
+    lists.nodes = (DistItem *)S.nodes.ptr;
+    float4 *item_c = (float4 *)S.item_c.ptr;
     int4 *sets = (int4 *)S.node_sets.ptr;
     DistHit *hits = (DistHit *)S.node_hits.ptr;
     int32_t *over = (int32_t *)S.node_over.ptr;
@@ -2240,13 +2268,13 @@ rt_status trace_items(SoftState &S, rt_scene *s, const CameraView &cv, const Lig
             if (!walk) {
                 for (int k = 0; k < levels; ++k)
                     k_dist_node<SC><<<node_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
-                        view, cv, ls, mt, dl, dp, lut, items, lists, v0, v1, k, k == levels - 1, sets, item_c, hits,
-                        over, dc, ctx->d_counters);
+                        view, cv, ls, mt, dl, dp, lut, lists, v0, v1, k, k == levels - 1, sets, item_c, hits, over,
+                        dc, ctx->d_counters);
                 k_dist_lights<SC><<<light_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
-                    view, ls, mt, dl, dp, area, s->d_verts, lut, items, hits, item_c, dc, ctx->d_counters);
+                    view, ls, mt, dl, dp, area, s->d_verts, lut, lists, hits, item_c, dc, ctx->d_counters);
             }
             k_dist_sub<SC><<<sub_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
-                view, cv, ls, mt, dl, dp, area, s->d_verts, lut, items, lists, walk ? nullptr : over, &dc->over,
+                view, cv, ls, mt, dl, dp, area, s->d_verts, lut, lists, walk ? nullptr : over, &dc->over,
                 &dc->work_over, item_c, ctx->d_counters);
             if (!walk)
                 for (int k = levels - 1; k-- > 0;)
@@ -2455,19 +2483,9 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
         RT_CUDA_S(S.nitems.reserve(2 * sizeof(int32_t) + sizeof(DistCounts)), "item counter allocation");
         // items per list (reflection sets, refraction sets)
         int64_t cap = std::min((int64_t)npix * per_pixel / 2, std::max(S.item_cap, (int64_t)npix * 2));
-        int64_t pool = 0;
         int32_t n[2] = {0, 0};
         for (int attempt = 0; attempt < 2; ++attempt) {
-            // room for the nodes below the items where it can be had
-            pool = std::min({kDistPoolPerItem * 2 * cap, (int64_t)kDistPoolPerItem * kDistPiece,
-                             ((int64_t)1 << 31) - 1 - 2 * cap});
-            if (S.items.reserve((2 * (size_t)cap + (size_t)pool) * sizeof(DistItem)) != cudaSuccess ||
-                S.item_c.reserve((2 * (size_t)cap + (size_t)pool) * sizeof(float4)) != cudaSuccess) {
-                cudaGetLastError();
-                pool = 0;
-                RT_CUDA_S(S.items.reserve(2 * (size_t)cap * sizeof(DistItem)), "item allocation");
-                RT_CUDA_S(S.item_c.reserve(2 * (size_t)cap * sizeof(float4)), "item colour allocation");
-            }
+            RT_CUDA_S(S.items.reserve(2 * (size_t)cap * sizeof(DistItem)), "item allocation");
             RT_CUDA_S(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), st), "counter clear");
             RT_CUDA_S(cudaMemsetAsync(S.nitems.ptr, 0, 2 * sizeof(int32_t), st), "item counter clear");
             with_scene(sv, [&](const auto &view) {
@@ -2489,7 +2507,7 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
         }
         S.item_cap = cap;
         if (n[0] + n[1] > 0) {
-            const rt_status wst = trace_items(S, s, cv, ls, mt, dl, dp, sv, DistLists{n[0], n[1], (int32_t)cap, (int32_t)pool},
+            const rt_status wst = trace_items(S, s, cv, ls, mt, dl, dp, sv, DistLists{n[0], n[1], (int32_t)cap, 0, nullptr, nullptr},
                                               std::max(tb.depth, 1), ctx, st);
             if (wst != RT_OK) return wst;
         }
