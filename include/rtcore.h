@@ -511,10 +511,8 @@ typedef struct rt_light_shape {
  * image) are nullable, not both, host or device memory.  Runs two passes
  * with one host round trip between them: the camera rays, then the frame's
  * slice of the random stream (generated on the device as far as earlier
- * frames have not) and the shading.  Beside the kernels of a frame that starts
- * where the last one ended the generator runs on a stream of the context's,
- * for this frame and the next; it ends with the frame, nothing runs on after
- * the call. */
+ * frames have not) and the shading.  A context that has drawn 12.5 million
+ * numbers keeps 62 MB on the device that let many SMs generate the rest. */
 rt_status rt_render_soft_shadows(rt_scene *scene, const rt_camera *camera, const rt_light *lights, int32_t nlights,
                                  const rt_light_shape *shapes, const rt_material *materials, int32_t nmaterials,
                                  int32_t samples, int64_t stream_offset, uint8_t *rgb_out, float *rgb_f32,

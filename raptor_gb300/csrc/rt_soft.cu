@@ -15,9 +15,9 @@
 // is therefore fixed by how many pixels before it hit something, so a frame
 // is rendered in two passes: the camera rays first (hit records kept, one
 // flag per pixel), an exclusive scan of the flags (each hit draws the same
-// count), the frame's slice of the stream generated on the device (k_ref_stream:
-// one block walks the generator's states in order), then the shading pass,
-// every pixel reading its own slice.
+// count), the frame's slice of the stream generated on the device (k_ref_jump,
+// k_ref_stream: blocks walk the generator's states from points a jump apart), then
+// the shading pass, every pixel reading its own slice.
 // The cosine table the offsets go through (common/common.h:171-209) is
 // built on the host the same way and kept on the device.
 #include <algorithm>
@@ -61,24 +61,16 @@ __device__ __forceinline__ uint32_t mt_twist(uint32_t a, uint32_t b)
     return (y >> 1) ^ ((uint32_t)((int32_t)(b << 31) >> 31) & 0x9908b0dfu);
 }
 
-// `refills` refills of `state`, one after another; but for kSkip the words
-// after each go to out, else they are positions that are skipped.  kAhead: the
-// words of a next frame, until *stop is set (looked at every kStopEvery
-// refills, its load a look old so that nobody waits for it); *done: how many
-// were made.  A chain of refills no two of which can overlap, so what counts is
-// the latency of one.
-// A new word i needs old words i and i + 1 and word i + 397, which for
-// i >= 227 is the new word i - 227: thread t takes words t, t + 227 and
-// t + 454, so those chains stay inside a thread and a refill is one exchange
-// of the old words through shared memory (two buffers, one barrier).
-// Measured 106 ns a refill with output, 85 without (138 and 110 with
-// branches around the idle threads' work; 177 on four warps of two words per
-// third; a host core takes 350).
+// Refills follow one another, so what counts is the latency of one.  A new word
+// i needs old words i and i + 1 and word i + 397, which for i >= 227 is the new
+// word i - 227: thread t takes words t, t + 227 and t + 454, so those chains stay
+// inside a thread and a refill is one exchange of the old words through shared
+// memory (two buffers, one barrier).  130 ns a refill with output, 85 without (138
+// and 110 with branches around the idle threads' work; 177 on four warps of two
+// words per third; a host core takes 350).
 constexpr int kMtThreads = 256;
 constexpr int kMtThird = kMtWords - 1 - 2 * 227;   // words 454..622
 constexpr int kMtBuffer = 1024;                    // idle threads read past the words
-constexpr int kStopEvery = 32;
-enum StreamMode : int { kSkip, kWords, kAhead };
 template <bool OUT>
 __device__ __forceinline__ void mt_refill(uint32_t *w, int t, int t3, bool on, bool third, uint32_t &a, uint32_t &b,
                                           uint32_t &c, uint32_t *dst)
@@ -104,45 +96,138 @@ __device__ __forceinline__ void mt_refill(uint32_t *w, int t, int t3, bool on, b
     }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kMtThreads) k_ref_stream(uint32_t *__restrict__ state, int32_t refills,
-                                                           uint32_t *__restrict__ out, const volatile int32_t *stop,
-                                                           int32_t *done)
+// `refills` refills of a state whose words are a (t), b (t + 227), c (t + 454)
+// and `last`; OUT: the words after each go to out.
+template <bool OUT>
+__device__ __forceinline__ void mt_refills(uint32_t *words, int32_t refills, uint32_t &a, uint32_t &b, uint32_t &c,
+                                           uint32_t last, uint32_t *out)
 {
-    constexpr bool OUT = MODE != kSkip;
-    extern __shared__ uint32_t mt_words[];   // two buffers (and what keeps other blocks off the SM)
-    __shared__ int32_t s_stop;
     const int t = threadIdx.x;
     const bool on = t < 227, third = t < kMtThird;
     const int t3 = third ? t : kMtThird - 1;
-    uint32_t a = state[on ? t : 0], b = state[on ? t + 227 : 0], c = state[t3 + 454];
-    const uint32_t last = state[kMtWords - 1];
-    for (int i = t; i < 2 * kMtBuffer; i += kMtThreads) mt_words[i] = 0u;
+    for (int i = t; i < 2 * kMtBuffer; i += kMtThreads) words[i] = 0u;
     __syncthreads();
-    if (t < 2) mt_words[t * kMtBuffer + kMtWords - 1] = last;
+    if (t < 2) words[t * kMtBuffer + kMtWords - 1] = last;
     uint32_t *dst = out;
-    int32_t r = 0, seen = 0;
+    int32_t r = 0;
     for (; r + 1 < refills; r += 2) {
-        const bool look = MODE == kAhead && r % kStopEvery == 0;
-        if (look && t == kMtThreads - 1) {
-            s_stop = seen;
-            seen = *stop;
-        }
-        mt_refill<OUT>(mt_words, t, t3, on, third, a, b, c, dst);
+        mt_refill<OUT>(words, t, t3, on, third, a, b, c, dst);
         if (OUT) dst += kMtWords;
-        mt_refill<OUT>(mt_words + kMtBuffer, t, t3, on, third, a, b, c, dst);
+        mt_refill<OUT>(words + kMtBuffer, t, t3, on, third, a, b, c, dst);
         if (OUT) dst += kMtWords;
-        if (look && s_stop) refills = r + 2;   // written before the pair's barriers
     }
-    if (r < refills) mt_refill<OUT>(mt_words, t, t3, on, third, a, b, c, dst);
+    if (r < refills) mt_refill<OUT>(words, t, t3, on, third, a, b, c, dst);
     if (OUT)
         for (int32_t i = t; i < refills; i += kMtThreads) out[(size_t)i * kMtWords + kMtWords - 1] = last;
+}
+
+// `total` refills, `each` of them to a block, block k from state starts + k * kMtWords
+// on; the words after every one to out (OUT), the state after the last to end.
+template <bool OUT>
+__global__ void __launch_bounds__(kMtThreads) k_ref_stream(const uint32_t *starts, int64_t total, int32_t each,
+                                                           uint32_t *__restrict__ out, uint32_t *end)
+{
+    __shared__ uint32_t words[2 * kMtBuffer];
+    const int t = threadIdx.x;
+    const bool on = t < 227, third = t < kMtThird;
+    const uint32_t *state = starts + (size_t)blockIdx.x * kMtWords;
+    const int64_t first = (int64_t)blockIdx.x * each;
+    uint32_t a = state[on ? t : 0], b = state[on ? t + 227 : 0], c = state[third ? t + 454 : kMtWords - 2];
+    const uint32_t last = state[kMtWords - 1];
+    mt_refills<OUT>(words, (int32_t)min((int64_t)each, total - first), a, b, c, last,
+                    OUT ? out + (size_t)first * kMtWords : nullptr);
+    if (first + each < total) return;
     if (on) {
-        state[t] = a;
-        state[t + 227] = b;
+        end[t] = a;
+        end[t + 227] = b;
     }
-    if (third) state[t + 454] = c;
-    if (MODE == kAhead && t == 0) *done = refills;
+    if (third) end[t + 454] = c;
+    if (t == 0) end[kMtWords - 1] = last;
+}
+
+// A refill is linear over GF(2) in the state's bits (the twist is, and word 623
+// stays), so kJump refills are one bit matrix.  Its column j, the state that
+// kJump refills make of bit j alone, is walked by block j.
+// With it the states kJump refills apart follow one another by one product each
+// (k_ref_jump, 4 us) and a block walks the refills after each (k_ref_stream): 52,000
+// refills, a 900p frame's of 16 samples, take 0.47 ms where one block takes 6.8, and
+// 3,400 of a 320x200 frame 85 us for 440.  50 MB and 3 ms, made once a context has
+// walked as long (kJumpWorth).  Jumps of 1024: 0.32 ms, 150 us, 6 ms to make; of 256
+// 0.85 ms, 85 us.
+constexpr int kJump = 512;
+constexpr int kMtBits = kMtWords * 32;
+__global__ void __launch_bounds__(kMtThreads) k_ref_matrix(uint32_t *__restrict__ columns)
+{
+    __shared__ uint32_t words[2 * kMtBuffer];
+    const int t = threadIdx.x, j = blockIdx.x;
+    const uint32_t bit = 1u << (j & 31);
+    const int w = j >> 5;
+    uint32_t a = w == t ? bit : 0u, b = w == t + 227 ? bit : 0u, c = w == t + 454 ? bit : 0u;
+    const uint32_t last = w == kMtWords - 1 ? bit : 0u;
+    mt_refills<false>(words, kJump, a, b, c, last, nullptr);
+    uint32_t *col = columns + (size_t)j * kMtWords;
+    if (t < 227) {
+        col[t] = a;
+        col[t + 227] = b;
+    }
+    if (t < kMtThird) col[t + 454] = c;
+    if (t == 0) col[kMtWords - 1] = last;
+}
+
+// One jump, its state's words shared out over kJumpBlocks blocks, four each: a
+// block puts its words of the state together -- from `state`, or from the parts
+// that the blocks of the jump before made of theirs -- and stores them in `at`;
+// then (product) its part of the next state is the sum of the columns of their
+// set bits.  What counts is the latency of a jump, so all of a block's columns
+// (half of 128, 16 bytes a thread) are in flight at once; together the blocks
+// read half of the matrix, out of the L2, and a launch is ready while the one
+// before ends: 4 us a jump (10 without any of it in the caches).
+constexpr int kJumpBlocks = kMtWords / 4;
+constexpr int kJumpLanes = 160;                    // a group's threads: one for four words of a column
+constexpr int kJumpThreads = 4 * kJumpLanes;       // four groups, for a word's bits each
+__global__ void __launch_bounds__(kJumpThreads) k_ref_jump(const uint4 *__restrict__ columns, const uint4 *state,
+                                                           const uint4 *parts, uint4 *next, uint4 *at, bool product)
+{
+    __shared__ uint4 s_part[kJumpThreads / 32];
+    __shared__ uint32_t s_word[4];
+    __shared__ uint4 s_sum[3][kJumpBlocks];
+    const auto add = [](uint4 p, uint4 q) { return make_uint4(p.x ^ q.x, p.y ^ q.y, p.z ^ q.z, p.w ^ q.w); };
+    const int t = threadIdx.x, b = blockIdx.x;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint4 mine = make_uint4(0u, 0u, 0u, 0u);
+    if (state) {
+        if (t == 0) mine = state[b];
+    } else if (t < kJumpBlocks) {
+        mine = __ldcg(parts + (size_t)t * kJumpBlocks + b);
+    }
+    for (int o = 16; o > 0; o >>= 1)
+        mine = add(mine, make_uint4(__shfl_xor_sync(0xffffffffu, mine.x, o), __shfl_xor_sync(0xffffffffu, mine.y, o),
+                                    __shfl_xor_sync(0xffffffffu, mine.z, o), __shfl_xor_sync(0xffffffffu, mine.w, o)));
+    if ((t & 31) == 0) s_part[t >> 5] = mine;
+    __syncthreads();
+    if (t == 0) {
+        for (int w = 1; w < kJumpLanes / 32; ++w) mine = add(mine, s_part[w]);
+        at[b] = mine;
+        s_word[0] = mine.x;
+        s_word[1] = mine.y;
+        s_word[2] = mine.z;
+        s_word[3] = mine.w;
+    }
+    __syncthreads();
+    if (!product) return;
+    const int group = t / kJumpLanes, lane = t % kJumpLanes;
+    const uint32_t bits = s_word[group];
+    uint4 sum = make_uint4(0u, 0u, 0u, 0u);
+    if (lane < kJumpBlocks) {
+        const uint4 *col = columns + (size_t)(128 * b + 32 * group) * kJumpBlocks + lane;
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if ((bits >> j) & 1u) sum = add(sum, __ldg(col + (size_t)j * kJumpBlocks));
+        if (group > 0) s_sum[group - 1][lane] = sum;
+    }
+    __syncthreads();
+    if (group == 0 && lane < kJumpBlocks)
+        next[(size_t)b * kJumpBlocks + lane] = add(add(sum, s_sum[0][lane]), add(s_sum[1][lane], s_sum[2][lane]));
 }
 
 // The rays light::find_rays makes for a triangle-defined light of ntris
@@ -186,25 +271,19 @@ struct SoftState {
     DevBuf root_c, root_sets, items, item_c, nitems;
     DevBuf nodes, node_sets, node_hits, node_over;   // nodes below them, their children, hit nodes, nodes walked whole
     int64_t item_cap = 0;
-    // The stream's words on the device: the window a frame reads from and one
-    // for the words that follow the frame's slice, where the next frame of an
-    // animation starts.  refills counts what the generator's state has behind
-    // it (-1: to be seeded).  Nothing of this is in flight between calls.
+    // The stream's words on the device, in two windows: words that a window has
+    // no more room behind go on in the other.  refills counts what the
+    // generator's state has behind it (-1: to be seeded).
     struct Window {
         DevBuf words;
         int64_t first = 0, count = 0;      // refills [first, first + count)
     } win[2];
     int cur = 0;                           // the window the last frame read
-    int64_t end = -1;                      // the number the last frame ended before
-    int64_t last = 0;                      // the refills its numbers took
-    DevBuf rng;                            // the generator's state, the seeded one, the word that stops it
+    DevBuf rng;                            // the generator's state, then the seeded one
     int64_t refills = -1;
-    size_t gen_smem = 0;
-    cudaStream_t gen = nullptr;            // reads ahead on a stream of its own
-    cudaEvent_t ready = nullptr;           // what it starts from is written
-    int32_t *done = nullptr;               // pinned (a word of the context's scratch): the refills it made
-    Window *ahead = nullptr;               // it is running, into this window, from ahead_from on
-    int64_t ahead_from = 0;
+    DevBuf jump;                           // the jump's matrix, the states of a row of jumps, their parts
+    bool jump_ready = false;
+    int64_t walked = 0;                    // refills walked one after another
     int device = 0;
 };
 
@@ -212,10 +291,9 @@ void soft_release(rt_context *ctx)
 {
     if (!ctx->soft) return;
     SoftState &S = *ctx->soft;
-    if (S.gen) cudaStreamDestroy(S.gen);
-    if (S.ready) cudaEventDestroy(S.ready);
     for (SoftState::Window &w : S.win) w.words.release();
     S.rng.release();
+    S.jump.release();
     S.lut.release();
     S.hits.release();
     S.flags.release();
@@ -1636,20 +1714,6 @@ struct SGuard {
 rt_status check_shapes(const rt_scene *s, const rt_light *lights, int32_t nlights, const rt_light_shape *shapes,
                        const char *who);
 rt_status stream_window(SoftState &S, int64_t offset, int64_t total, cudaStream_t st, const uint32_t **rnd);
-rt_status stream_begin(SoftState &S, int64_t offset, cudaStream_t st);
-rt_status stream_stop(SoftState &S, cudaStream_t st);
-rt_status stream_finish(SoftState &S);
-
-// Ends what the generator does beside a frame that ends early.
-struct StreamEnd {
-    SoftState &S;
-    cudaStream_t st;
-    ~StreamEnd()
-    {
-        stream_stop(S, st);
-        stream_finish(S);
-    }
-};
 
 template <class SC>
 int soft_blocks_per_sm()
@@ -1700,7 +1764,6 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
         ctx->soft = new (std::nothrow) SoftState();
         if (!ctx->soft) return sfail(RT_ERR_OUT_OF_MEMORY, "rt_render_soft_shadows: state allocation");
         ctx->soft->device = ctx->device;
-        ctx->soft->done = ctx->h_scratch + 2;
     }
     SoftState &S = *ctx->soft;
     cudaStream_t st = ctx->stream;
@@ -1766,9 +1829,6 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
 
     RT_CUDA_S(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), st), "counter clear");
     RT_CUDA_S(cudaEventRecord(ctx->ev0, st), "event record");
-    StreamEnd end_stream{S, st};
-    rt_status sst = stream_begin(S, stream_offset, st);
-    if (sst != RT_OK) return sst;
     with_scene(sv, [&](const auto &view) {
         using SC = std::decay_t<decltype(view)>;
         k_soft_primary<SC><<<soft_blocks_per_sm<SC>() * ctx->sm_count, kTraceThreads, 0, st>>>(
@@ -1778,8 +1838,6 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
     cub::DeviceScan::ExclusiveSum(S.scan_temp.ptr, scan_bytes, (const int32_t *)S.flags.ptr, (int32_t *)S.prefix.ptr,
                                   (int)npix, st);
     RT_CUDA_S(cudaGetLastError(), "scan launch");
-    sst = stream_stop(S, st);
-    if (sst != RT_OK) return sst;
     // the frame's count of numbers: per_hit for every hit pixel
     int32_t *h = ctx->h_scratch;
     RT_CUDA_S(cudaMemcpyAsync(h, (const int32_t *)S.prefix.ptr + (npix - 1), sizeof(int32_t), cudaMemcpyDeviceToHost, st),
@@ -1792,8 +1850,8 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
     const int64_t total = nhits * per_hit;
     // the frame's slice of the reference's stream
     const uint32_t *rnd = nullptr;
-    sst = stream_window(S, stream_offset, total, st, &rnd);
-    if (sst != RT_OK) return sst;
+    const rt_status wst = stream_window(S, stream_offset, total, st, &rnd);
+    if (wst != RT_OK) return wst;
 
     // outputs: device pointers as given, host ones staged
     const bool rgb_host = rgb_out && !is_device_ptr(rgb_out);
@@ -1818,16 +1876,12 @@ extern "C" rt_status rt_render_soft_shadows(rt_scene *s, const rt_camera *camera
     });
     RT_CUDA_S(cudaGetLastError(), "shade launch");
     RT_CUDA_S(cudaEventRecord(ctx->ev1, st), "event record");
-    sst = stream_stop(S, st);
-    if (sst != RT_OK) return sst;
     if (rgb_host) RT_CUDA_S(cudaMemcpyAsync(rgb_out, d_rgb, npix * 3, cudaMemcpyDeviceToHost, st), "rgb copy");
     if (f_host)
         RT_CUDA_S(cudaMemcpyAsync(rgb_f32, d_f, npix * 3 * sizeof(float), cudaMemcpyDeviceToHost, st), "image copy");
     Counters c;
     RT_CUDA_S(cudaMemcpyAsync(&c, ctx->d_counters, sizeof(Counters), cudaMemcpyDeviceToHost, st), "counter read");
     RT_CUDA_S(cudaStreamSynchronize(st), "synchronize");
-    sst = stream_finish(S);
-    if (sst != RT_OK) return sst;
     if (stats) {
         stats->primary_rays = (int64_t)c.primary;
         stats->secondary_rays = (int64_t)c.secondary;
@@ -1999,20 +2053,11 @@ rt_status check_shapes(const rt_scene *s, const rt_light *lights, int32_t nlight
 rt_status stream_setup(SoftState &S)
 {
     if (S.rng.ptr) return RT_OK;
-    // the generator's block takes all the shared memory a block can have, so
-    // that no render block shares its SM and lengthens its chain of refills
-    int most = 0;
-    RT_CUDA_S(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, S.device), "shared memory size");
-    S.gen_smem = (size_t)most - 128;   // less what the kernel itself has
-    for (const auto kernel : {k_ref_stream<kSkip>, k_ref_stream<kWords>, k_ref_stream<kAhead>})
-        RT_CUDA_S(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.gen_smem),
-                  "shared memory size");
     // the seeded state (common/common.cc:35-50)
-    uint32_t mt[2 * kMtWords + 1];
+    uint32_t mt[2 * kMtWords];
     mt[0] = 5489u;
     for (int i = 1; i < kMtWords; ++i) mt[i] = 1812433253u * (mt[i - 1] ^ (mt[i - 1] >> 30)) + (uint32_t)i;
     std::memcpy(mt + kMtWords, mt, kMtWords * sizeof(uint32_t));
-    mt[2 * kMtWords] = 0;
     RT_CUDA_S(S.rng.reserve(sizeof(mt)), "generator allocation");
     const cudaError_t e = cudaMemcpy(S.rng.ptr, mt, sizeof(mt), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) S.rng.release();
@@ -2054,21 +2099,82 @@ rt_status window_start(SoftState &S, SoftState::Window &w, int64_t r0, int64_t r
     return RT_OK;
 }
 
+// The jump's matrix, once the context has walked (or is about to) as many refills
+// as it costs; without memory for it the refills are walked.
+constexpr int64_t kJumpWorth = 20000;
+constexpr int kJumpRow = 256;   // jumps whose states are kept at a time
+constexpr size_t kMatrixWords = (size_t)kMtBits * kMtWords, kPartWords = (size_t)kJumpBlocks * kMtWords;
+void jump_setup(SoftState &S, int64_t refills, cudaStream_t st)
+{
+    if (S.jump_ready || S.walked + refills < kJumpWorth) return;
+    if (S.jump.reserve((kMatrixWords + (size_t)(kJumpRow + 1) * kMtWords + 2 * kPartWords) * sizeof(uint32_t)) !=
+        cudaSuccess) {
+        cudaGetLastError();
+        S.walked = 0;   // tried again after as many
+        return;
+    }
+    k_ref_matrix<<<kMtBits, kMtThreads, 0, st>>>((uint32_t *)S.jump.ptr);
+    S.jump_ready = true;
+}
+
+// Jumps from the generator's state: state k, k jumps on, to states + k * kMtWords,
+// k = 0 .. n - 1.
+rt_status jump_states(SoftState &S, uint32_t *states, int n, cudaStream_t st)
+{
+    const uint4 *columns = (const uint4 *)S.jump.ptr;
+    uint32_t *parts = (uint32_t *)S.jump.ptr + kMatrixWords + (size_t)(kJumpRow + 1) * kMtWords;
+    cudaLaunchAttribute early;   // launched while the jump before ends
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kJumpBlocks);
+    cfg.blockDim = dim3(kJumpThreads);
+    cfg.stream = st;
+    cfg.attrs = &early;
+    for (int k = 0; k < n; ++k) {
+        const uint4 *state = k == 0 ? (const uint4 *)S.rng.ptr : nullptr;
+        const uint4 *from = (const uint4 *)(parts + ((k + 1) & 1) * kPartWords);
+        uint4 *to = (uint4 *)(parts + (k & 1) * kPartWords), *at = (uint4 *)(states + (size_t)k * kMtWords);
+        cfg.numAttrs = k > 0 ? 1 : 0;
+        RT_CUDA_S(cudaLaunchKernelEx(&cfg, k_ref_jump, columns, state, from, to, at, k + 1 < n), "jump launch");
+    }
+    return RT_OK;
+}
+
 // The generator up to refill r1, its words to the end of w (null: skipped).
-// Launches of at most kMtLaunch refills, a few milliseconds each.
-constexpr int64_t kMtLaunch = 65536;
+// Walks are launched at most kMtLaunch refills at a time, a few milliseconds
+// each; slices from kJumpLeast on take jumps (a jump costs 4 us, a block's walk of
+// kJump refills 60).
+constexpr int64_t kMtLaunch = 65536, kJumpLeast = kJump + kJump / 2;
 rt_status generate(SoftState &S, SoftState::Window *w, int64_t r1, cudaStream_t st)
 {
     uint32_t *state = (uint32_t *)S.rng.ptr;
     int64_t pos = S.refills;
     S.refills = -1;   // whatever fails below, the next frame starts from the seed
+    if (r1 - pos >= kJumpLeast) jump_setup(S, r1 - pos, st);
+    uint32_t *states = (uint32_t *)S.jump.ptr + kMatrixWords;
     while (pos < r1) {
-        const int64_t n = std::min(r1 - pos, kMtLaunch);
-        if (w) {
-            k_ref_stream<kWords><<<1, kMtThreads, S.gen_smem, st>>>(
-                state, (int32_t)n, (uint32_t *)w->words.ptr + (pos - w->first) * kMtWords, nullptr, nullptr);
+        uint32_t *out = w ? (uint32_t *)w->words.ptr + (pos - w->first) * kMtWords : nullptr;
+        int64_t n = r1 - pos;
+        if (!S.jump_ready || n < kJumpLeast) {
+            n = std::min(n, kMtLaunch);
+            S.walked += n;
+            if (w) k_ref_stream<true><<<1, kMtThreads, 0, st>>>(state, n, (int32_t)n, out, state);
+            else k_ref_stream<false><<<1, kMtThreads, 0, st>>>(state, n, (int32_t)n, nullptr, state);
+        } else if (w) {
+            n = std::min(n, (int64_t)kJumpRow * kJump);
+            const int blocks = (int)((n + kJump - 1) / kJump);
+            const rt_status rc = jump_states(S, states, blocks, st);
+            if (rc != RT_OK) return rc;
+            k_ref_stream<true><<<blocks, kMtThreads, 0, st>>>(states, n, kJump, out, state);
         } else {
-            k_ref_stream<kSkip><<<1, kMtThreads, S.gen_smem, st>>>(state, (int32_t)n, nullptr, nullptr, nullptr);
+            const int jumps = (int)std::min(n / kJump, (int64_t)kJumpRow);
+            n = (int64_t)jumps * kJump;
+            const rt_status rc = jump_states(S, states, jumps + 1, st);
+            if (rc != RT_OK) return rc;
+            RT_CUDA_S(cudaMemcpyAsync(state, states + (size_t)jumps * kMtWords, kMtWords * sizeof(uint32_t),
+                                      cudaMemcpyDeviceToDevice, st),
+                      "generator state");
         }
         pos += n;
     }
@@ -2078,85 +2184,17 @@ rt_status generate(SoftState &S, SoftState::Window *w, int64_t r1, cudaStream_t 
     return RT_OK;
 }
 
-// The generator beside the frame's kernels on a stream of its own: from its
-// position on into w, up to refill `to` or until stream_stop.
-rt_status run_ahead(SoftState &S, SoftState::Window &w, int64_t to, cudaStream_t st)
-{
-    const int64_t room = (int64_t)(w.words.cap / refill_bytes(1)) - w.count;
-    const int64_t n = std::min({to - S.refills, room, (int64_t)1 << 24});
-    if (n <= 0) return RT_OK;
-    if (!S.gen) RT_CUDA_S(cudaStreamCreateWithFlags(&S.gen, cudaStreamNonBlocking), "stream create");
-    if (!S.ready) RT_CUDA_S(cudaEventCreateWithFlags(&S.ready, cudaEventDisableTiming), "event creation");
-    uint32_t *state = (uint32_t *)S.rng.ptr;
-    int32_t *stop = (int32_t *)(state + 2 * kMtWords);
-    RT_CUDA_S(cudaMemsetAsync(stop, 0, sizeof(int32_t), st), "generator start");
-    RT_CUDA_S(cudaEventRecord(S.ready, st), "event record");
-    RT_CUDA_S(cudaStreamWaitEvent(S.gen, S.ready, 0), "stream wait");
-    S.ahead = &w;
-    S.ahead_from = S.refills;
-    S.refills = -1;
-    *S.done = -1;
-    k_ref_stream<kAhead><<<1, kMtThreads, S.gen_smem, S.gen>>>(
-        state, (int32_t)n, (uint32_t *)w.words.ptr + (S.ahead_from - w.first) * kMtWords, stop, S.done);
-    RT_CUDA_S(cudaGetLastError(), "generator launch");
-    return RT_OK;
-}
-
-// Frames that start where the last one ended, as an animation's do, have the
-// generator run beside all of their kernels: beside the camera rays for their
-// own numbers, as many as the last frame drew (stream_begin), and beside the
-// shading for the next frame's, a quarter more than this one drew (read_ahead);
-// each ends with those kernels (stream_stop, stream_finish), so that the call
-// leaves nothing running.  A 900p terrain frame of 16 samples (52,000 refills):
-// 7.25 ms, the generator's chain; 9.1 where it starts anywhere else.
-// Frames that drew little (kAheadRefills) don't: two launches and a wait take
-// about 15 us, a refill 0.1.
-constexpr int64_t kAheadRefills = 512;
-rt_status stream_begin(SoftState &S, int64_t offset, cudaStream_t st)
-{
-    if (offset != S.end || S.last < kAheadRefills) return RT_OK;
-    const int64_t r0 = offset / kMtWords;
-    for (SoftState::Window &w : S.win)
-        if (window_leads(S, w, r0)) return run_ahead(S, w, r0 + S.last, st);
-    return RT_OK;
-}
-
-rt_status read_ahead(SoftState &S, int64_t next, int64_t total, cudaStream_t st)
-{
-    const int64_t n0 = next / kMtWords, n2 = (next + total + total / 4 + kMtWords - 1) / kMtWords;
-    SoftState::Window &cur = S.win[S.cur], &w = S.win[S.cur ^ 1];
-    if (!window_leads(S, w, n0)) {
-        if (!window_leads(S, cur, n0) || S.refills >= n2) return RT_OK;
-        // without room for it the next frame generates all of its own numbers
-        const size_t bytes = refill_bytes(n2 - n0);
-        if (bytes > w.words.cap) {
-            size_t free_b = 0, all_b = 0;
-            w.count = 0;
-            if (cudaMemGetInfo(&free_b, &all_b) != cudaSuccess || 2 * bytes >= free_b ||
-                w.words.reserve(bytes) != cudaSuccess) {
-                cudaGetLastError();
-                return RT_OK;
-            }
-        }
-        const rt_status rc = window_start(S, w, n0, n2 - n0, &cur, st);
-        if (rc != RT_OK) return rc;
-    }
-    return run_ahead(S, w, n2, st);
-}
-
 // The frame's numbers [offset, offset + total) of the reference's stream as
 // words on the device (ref_number), kept while later frames fall inside their
 // window; *rnd points at number offset.  Of frames that each start where the
 // one before ended, only the first can start from the seed: one of the windows
-// always leads from the last one's end on.  The caller has called stream_stop
-// after the kernels before, calls it after its last kernel and stream_finish once
-// `st` is through.
+// always leads from the last one's end on.
 rt_status stream_window(SoftState &S, int64_t offset, int64_t total, cudaStream_t st, const uint32_t **rnd)
 {
     *rnd = nullptr;
-    rt_status rc = stream_finish(S);
-    if (rc == RT_OK && total > 0) rc = stream_setup(S);
-    if (rc != RT_OK || total <= 0) return rc;
+    if (total <= 0) return RT_OK;
+    rt_status rc = stream_setup(S);
+    if (rc != RT_OK) return rc;
     const int64_t r0 = offset / kMtWords, r1 = (offset + total + kMtWords - 1) / kMtWords;
     const int a = S.cur, b = S.cur ^ 1;
     int use = window_holds(S.win[a], r0, r1) ? a : window_holds(S.win[b], r0, r1) ? b : -1;
@@ -2185,31 +2223,6 @@ rt_status stream_window(SoftState &S, int64_t offset, int64_t total, cudaStream_
     }
     S.cur = use;
     *rnd = (const uint32_t *)S.win[use].words.ptr + (offset - S.win[use].first * kMtWords);
-    const bool follows = offset == S.end;
-    S.end = offset + total;
-    S.last = r1 - r0;
-    return follows && r1 - r0 >= kAheadRefills ? read_ahead(S, S.end, total, st) : RT_OK;
-}
-
-// After the kernels on `st` that the generator runs beside: it ends.
-rt_status stream_stop(SoftState &S, cudaStream_t st)
-{
-    if (S.ahead)
-        RT_CUDA_S(cudaMemsetAsync((uint32_t *)S.rng.ptr + 2 * kMtWords, 1, sizeof(int32_t), st), "generator stop");
-    return RT_OK;
-}
-
-// Waits for its end and takes what it made.
-rt_status stream_finish(SoftState &S)
-{
-    if (!S.ahead) return RT_OK;
-    SoftState::Window &w = *S.ahead;
-    S.ahead = nullptr;
-    RT_CUDA_S(cudaStreamSynchronize(S.gen), "synchronize");
-    if (*S.done >= 0) {
-        w.count += *S.done;
-        S.refills = S.ahead_from + *S.done;
-    }
     return RT_OK;
 }
 
@@ -2350,7 +2363,6 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
         ctx->soft = new (std::nothrow) SoftState();
         if (!ctx->soft) return sfail(RT_ERR_OUT_OF_MEMORY, "rt_render_distributed: state allocation");
         ctx->soft->device = ctx->device;
-        ctx->soft->done = ctx->h_scratch + 2;
     }
     SoftState &S = *ctx->soft;
     cudaStream_t st = ctx->stream;
@@ -2423,13 +2435,9 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
     RT_CUDA_S(cudaMemsetAsync(ctx->d_counters, 0, sizeof(Counters), st), "counter clear");
     RT_CUDA_S(cudaEventRecord(ctx->ev0, st), "event record");
     const uint32_t *rnd = nullptr;
-    StreamEnd end_stream{S, st};
-    rt_status sst = RT_OK;
     int64_t total = 0;
     if (smp.stream == RT_STREAM_REFERENCE) {
         // counting pass, scan, the frame's slice of the stream
-        sst = stream_begin(S, smp.stream_offset, st);
-        if (sst != RT_OK) return sst;
         RT_CUDA_S(S.counts.reserve(npix * sizeof(int64_t)), "count allocation");
         RT_CUDA_S(S.prefix64.reserve(npix * sizeof(int64_t)), "prefix allocation");
         size_t scan_bytes = 0;
@@ -2446,8 +2454,6 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
         cub::DeviceScan::ExclusiveSum(S.scan64_temp.ptr, scan_bytes, (const int64_t *)S.counts.ptr,
                                       (int64_t *)S.prefix64.ptr, (int)npix, st);
         RT_CUDA_S(cudaGetLastError(), "scan launch");
-        sst = stream_stop(S, st);
-        if (sst != RT_OK) return sst;
         int64_t last[2];
         RT_CUDA_S(cudaMemcpyAsync(&last[0], (const int64_t *)S.prefix64.ptr + (npix - 1), sizeof(int64_t),
                                   cudaMemcpyDeviceToHost, st),
@@ -2457,8 +2463,8 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
                   "count read");
         RT_CUDA_S(cudaStreamSynchronize(st), "synchronize");
         total = last[0] + last[1];
-        sst = stream_window(S, smp.stream_offset, total, st, &rnd);
-        if (sst != RT_OK) return sst;
+        const rt_status wst = stream_window(S, smp.stream_offset, total, st, &rnd);
+        if (wst != RT_OK) return wst;
         RT_CUDA_S(cudaMemsetAsync(&ctx->d_counters->work, 0, sizeof(int), st), "work counter clear");
     }
     const bool rgb_host = rgb_out && !is_device_ptr(rgb_out);
@@ -2524,16 +2530,12 @@ extern "C" rt_status rt_render_distributed(rt_scene *s, const rt_camera *camera,
     }
     RT_CUDA_S(cudaGetLastError(), "shade launch");
     RT_CUDA_S(cudaEventRecord(ctx->ev1, st), "event record");
-    sst = stream_stop(S, st);
-    if (sst != RT_OK) return sst;
     if (rgb_host) RT_CUDA_S(cudaMemcpyAsync(rgb_out, d_rgb, npix * 3, cudaMemcpyDeviceToHost, st), "rgb copy");
     if (f_host)
         RT_CUDA_S(cudaMemcpyAsync(rgb_f32, d_f, npix * 3 * sizeof(float), cudaMemcpyDeviceToHost, st), "image copy");
     Counters c;
     RT_CUDA_S(cudaMemcpyAsync(&c, ctx->d_counters, sizeof(Counters), cudaMemcpyDeviceToHost, st), "counter read");
     RT_CUDA_S(cudaStreamSynchronize(st), "synchronize");
-    sst = stream_finish(S);
-    if (sst != RT_OK) return sst;
     if (stats) {
         stats->primary_rays = (int64_t)c.primary;
         stats->secondary_rays = (int64_t)c.secondary;
