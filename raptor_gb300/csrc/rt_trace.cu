@@ -542,16 +542,23 @@ __global__ void __launch_bounds__(kTraceThreads, RT_SAMPLE_MIN_BLOCKS) k_render_
 }
 
 // The queued pixels of k_render_aa, one per thread, every sample shaded
-// with the exact specular power.  They lie all over the frame: rays one by
-// one (in step 1283x717 instances with 2x2 samples took 3.82 ms, now 3.55).
-template <class SC>
+// with the exact specular power (and whole backgrounds, which cost little).  They
+// lie all over the frame: rays one by one, but in step up to kFixPixels to an SM,
+// where the latency of a warp is what counts.  Launched for both; the other finds
+// nothing to do.  2x2 samples, in step / one by one: 513x517 sphere (842 queued an
+// SM) 660 / 697 us, terrain (712) 702 / 760, instances (1745) 1462 / 1453; 1283x717
+// (2864, 3132, 6052) 1047 / 1010, 1405 / 1358, 3825 / 3558.
+constexpr int kFixPixels = 1280;
+template <bool STEP, class SC>
 __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_aa_fix(SC sc, CameraView cam,
                                                                  LightSet lights, MaterialView mat, int32_t aa_x,
                                                                  int32_t aa_y, int32_t out_x,
                                                                  uint8_t *__restrict__ rgb,
-                                                                 const int32_t *__restrict__ redo, Counters *ctr)
+                                                                 const int32_t *__restrict__ redo, int32_t few,
+                                                                 Counters *ctr)
 {
     const int32_t n = min(ctr->redo, out_x * (cam.yres / aa_y));
+    if ((n <= few) != STEP) return;
     const float nsamples = (float)(aa_x * aa_y);
     uint32_t status = 0;
     const int lane = threadIdx.x & 31;
@@ -562,7 +569,7 @@ __global__ void __launch_bounds__(kTraceThreads, RT_RENDER_MIN_BLOCKS) k_render_
         float3 sum = make_float3(0.f, 0.f, 0.f);
         for (int ax = 0; ax < aa_x; ++ax)
             for (int ay = 0; ay < aa_y; ++ay) {
-                const PixelOut po = shade_pixel_lights<false, false, false>(sc, cam, lights.l, lights.n, mat,
+                const PixelOut po = shade_pixel_lights<false, false, STEP>(sc, cam, lights.l, lights.n, mat,
                                                                             x * aa_x + ax, y * aa_y + ay, status,
                                                                             nullptr, false, nullptr, live);
                 sum = xadd3(sum, po.c);
@@ -802,8 +809,13 @@ void launch_render_aa(const SceneView &sc, const CameraView &cam, const LightSet
         else
             k_render_aa<false, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, aa_x, aa_y, out_x, out_y, rgb, redo,
                                                                 ctr);
-        if (lights.fast_pow)
-            k_render_aa_fix<SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, aa_x, aa_y, out_x, rgb, redo, ctr);
+        if (lights.fast_pow) {
+            const int32_t few = kFixPixels * sm_count;
+            k_render_aa_fix<true, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, aa_x, aa_y, out_x, rgb,
+                                                                      redo, few, ctr);
+            k_render_aa_fix<false, SC><<<grid, kTraceThreads, 0, st>>>(view, cam, lights, mat, aa_x, aa_y, out_x, rgb,
+                                                                       redo, few, ctr);
+        }
     });
 }
 
